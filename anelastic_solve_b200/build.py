@@ -38,6 +38,7 @@ SOURCES = {
     "mg_col64.cu": ["-fmad=false"],
     "tune.cu": [],
     "mg_coarse.cu": ["-fmad=true"],
+    "mg_spectral.cu": ["-fmad=true"],
 }
 
 

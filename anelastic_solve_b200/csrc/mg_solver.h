@@ -7,6 +7,7 @@
 #include "mg_coarse.h"
 #include "mg_col.h"
 #include "mg_launch.h"
+#include "mg_spectral.h"
 
 namespace anel {
 
@@ -94,6 +95,18 @@ class MGSolver {
   DirectHost dirfine_;
   int build_direct(int l, DirectHost& D);
   void choose_direct_level();
+  // FP64 direct solve of the fine level (mg_spectral.cuh): the mixed solve's
+  // correction where x and y are periodic and uniform and the extents are
+  // transformable; V-cycles take over if two corrections do not reach the
+  // tolerance (an incompatible right-hand side, a tolerance below FP64's
+  // reach)
+  bool spec_want_ = false;
+  SpecHost spec_;
+  double* d_bspec_ = nullptr;  // spectral work space of a batch
+  int build_spec();
+  void solve_spec(int n, const SpecDev& D, const DevLevel<double>& F, cudaStream_t s);
+  int solve_vcycle(double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);
+  int spec_report(const SpecState& st, double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);
   ColLevel C32(int l) const;
   int64_t fp32_elems(int l) const;
   // nb = 0: this solver's own FP32 levels; nb >= 1: the first nb members of

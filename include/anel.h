@@ -113,8 +113,10 @@ typedef struct {
   double resid;        /* ||f - A phi||_2 / ||f||_2 (fine operator) after the solve */
   double ms;           /* device time of the solve (CUDA events) */
   int64_t launches;    /* kernels of this library launched by the solve */
-  int32_t fine_sweeps; /* finest-level smoother launches timed (profiling on) */
-  int32_t reserved;
+  int32_t fine_sweeps; /* finest-level smoother launches timed (profiling on);
+                        * direct solves: launches of the z-system pass */
+  int32_t reserved;    /* 1: solved by the direct fine-level solve alone (iter
+                        * then counts its corrections) */
   double fine_sweep_ms;/* their summed device time (CUDA events, profiling on) */
 } anel_mg_report;
 
