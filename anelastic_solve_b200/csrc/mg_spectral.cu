@@ -359,24 +359,25 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
   }
 }
 
-// |f - A phi|: a thread takes 8 planes of one (i, j), the z neighbours kept
-// in registers; grid (ceil(nx/32), ceil(ny/8), ceil(nz/8) * members).
-constexpr int kCheckK = 8;
+// |f - A phi|: a thread takes K planes of one (i, j), the z neighbours kept
+// in registers; grid (ceil(nx*ny/256), ceil(nz/K) * members).  K = 8, or 2
+// on the grids that 8 planes leave with less than two blocks per SM.
+template <int K>
 __global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int nzb) {
-  const int b = blockIdx.z / nzb;
+  const int b = blockIdx.y / nzb;
   if (!D.st[b].act) return;
   const double* __restrict__ phi = D.mt ? D.mt[b].phi : D.phi;
   const double* __restrict__ rhs = D.mt ? D.mt[b].rhs : D.rhs;
-  const int i = 2 + blockIdx.x * 32 + (threadIdx.x & 31);
-  const int j = 2 + blockIdx.y * 8 + (threadIdx.x >> 5);
-  const int zb = blockIdx.z - b * nzb;
-  const int k0 = 2 + zb * kCheckK;
+  const int col = blockIdx.x * 256 + threadIdx.x;
+  const int zb = blockIdx.y - b * nzb;
+  const int k0 = 2 + zb * K;
   double rr = 0.0, ff = 0.0;
-  if (i <= D.nx + 1 && j <= D.ny + 1) {
+  if (col < D.nx * D.ny) {
+    const int j = 2 + col / D.nx, i = 2 + col - (j - 2) * D.nx;
     int64_t c = cidx(i, j, k0, D.X, D.XY);
     double pm = phi[c - D.XY], pc = phi[c];
 #pragma unroll
-    for (int q = 0; q < kCheckK; ++q) {
+    for (int q = 0; q < K; ++q) {
       const int k = k0 + q;
       if (k <= D.nz + 1) {
         const double pp = phi[c + D.XY], f = rhs[c];
@@ -395,8 +396,7 @@ __global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int nzb) {
       }
     }
   }
-  spec_norm_finish(D, b, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * zb), gridDim.x * gridDim.y * nzb, rr, ff,
-                   true);
+  spec_norm_finish(D, b, blockIdx.x + gridDim.x * zb, gridDim.x * nzb, rr, ff, true);
 }
 
 // ------------------------------------------------------------------ host
@@ -443,7 +443,10 @@ bool spec_supported(int nx, int ny, int nz) {
   return plan_radices(nx, r) && plan_radices(ny, r) && nz >= 2 && nz <= kSpecMaxNz;
 }
 
-static int check_blocks(const SpecDev& D) { return ((D.nx + 31) / 32) * ((D.ny + 7) / 8) * ((D.nz + kCheckK - 1) / kCheckK); }
+constexpr int kFillBlocks = 2 * 148;
+static int check_cols(const SpecDev& D) { return (D.nx * D.ny + 255) / 256; }
+static int check_planes(const SpecDev& D) { return check_cols(D) * ((D.nz + 7) / 8) < kFillBlocks ? 2 : 8; }
+static int check_zblocks(const SpecDev& D) { return (D.nz + check_planes(D) - 1) / check_planes(D); }
 static size_t x_smem(const SpecDev& D) { return (size_t)2 * D.pairs * spec_row(D.nx) * sizeof(double2); }
 // columns per block of the y passes: eight fill a 128-byte line; fewer
 // where the two buffers of a longer transform would not fit
@@ -491,8 +494,11 @@ int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const 
   D.scale = 1.0 / ((double)nx * ny);
   D.coef = coef;
   segment(nz, &D.S, &D.M);
-  // row pairs per block: about 256 butterflies of radix 8
+  // row pairs per block: about 256 butterflies of radix 8, fewer (down to a
+  // warp's) where that leaves the GPU with less than two blocks per SM
   D.pairs = std::max(1, std::min(ny / 2, 2048 / nx));
+  while (D.pairs * nx > 256 && D.pairs > 1 && (int64_t)nz * ((ny / 2 + D.pairs - 1) / D.pairs) < kFillBlocks)
+    D.pairs = (D.pairs + 1) / 2;
   const double pi = 3.14159265358979323846;
   // tables: twiddles of x and y, eigenvalues, z coefficients
   std::vector<double> tab;
@@ -593,7 +599,7 @@ int spec_reserve(SpecHost& H, int n) {
   H.d_count = nullptr;
   H.cap = 0;
   const int64_t fwd = (int64_t)((D.ny / 2 + D.pairs - 1) / D.pairs) * D.nz;
-  D.pstride = 2 * std::max<int64_t>(fwd, check_blocks(D));
+  D.pstride = 2 * std::max<int64_t>(fwd, (int64_t)check_cols(D) * check_zblocks(D));
   ANEL_CUDA_TRY(cudaMalloc(&H.d_part, (size_t)n * D.pstride * sizeof(double)));
   ANEL_CUDA_TRY(cudaMalloc(&H.d_st, (size_t)n * sizeof(SpecState)));
   ANEL_CUDA_TRY(cudaMalloc(&H.d_count, (size_t)n * sizeof(unsigned)));
@@ -619,10 +625,10 @@ void spec_free(SpecHost& H) {
 
 static int x_threads(const SpecDev& D) {
   const int t = (D.pairs * D.nx / 8 + 31) / 32 * 32;
-  return std::max(64, std::min(256, t));
+  return std::max(32, std::min(256, t));
 }
 static int y_threads(const SpecDev& D) {
-  return std::max(64, std::min(256, (y_cols(D) * D.ny / 8 + 31) / 32 * 32));
+  return std::max(32, std::min(256, (y_cols(D) * D.ny / 8 + 31) / 32 * 32));
 }
 
 void launch_spec_forward(const SpecDev& D, int nm, bool test, cudaStream_t s) {
@@ -653,9 +659,10 @@ void launch_spec_update(const SpecDev& D, int nm, cudaStream_t s) {
 }
 
 void launch_spec_check(const SpecDev& D, int nm, cudaStream_t s) {
-  const int nzb = (D.nz + kCheckK - 1) / kCheckK;
-  const dim3 g((unsigned)((D.nx + 31) / 32), (unsigned)((D.ny + 7) / 8), (unsigned)(nzb * nm));
-  k_spec_check<<<g, 256, 0, s>>>(D, nzb);
+  const int nzb = check_zblocks(D);
+  const dim3 g((unsigned)check_cols(D), (unsigned)(nzb * nm));
+  if (check_planes(D) == 8) k_spec_check<8><<<g, 256, 0, s>>>(D, nzb);
+  else k_spec_check<2><<<g, 256, 0, s>>>(D, nzb);
   count_launch();
 }
 

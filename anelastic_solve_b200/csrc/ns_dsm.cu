@@ -363,15 +363,13 @@ int NSSolver::dyn_ratio(double* num, double* den, double* out, cudaStream_t s) {
   double* pd = pn + Z;
   const dim3 g = interior_grid(D_);
   const ZRule cf = zrule(NV_CFLUC);
-  launch_ghost_field(D_, num, cf, s);
-  launch_ghost_field(D_, den, cf, s);
+  launch_ghost_fields2(D_, num, den, cf, s);
   launch_plane_avg(D_, num, dxc, dyc, dyn_area_, dyn_part_, pn, s);
   launch_plane_avg(D_, den, dxc, dyc, dyn_area_, dyn_part_, pd, s);
   k_dyn_bcast<<<g, 128, 0, s>>>(D_, pn, 1, num);
   k_dyn_bcast<<<g, 128, 0, s>>>(D_, pd, 0, den);
   count_launch(2);
-  launch_ghost_field(D_, num, cf, s);
-  launch_ghost_field(D_, den, cf, s);
+  launch_ghost_fields2(D_, num, den, cf, s);
   k_dyn_ratio<<<g, 128, 0, s>>>(D_, num, den, out);
   count_launch();
   launch_ghost_field(D_, out, cf, s);

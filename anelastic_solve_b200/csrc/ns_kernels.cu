@@ -6,9 +6,20 @@
 namespace anel {
 
 static constexpr double R12 = 1.0 / 2.0;  // ratios::r_1_2 (modules.F90:203)
-// planes of one (i, j) per thread in the one-cell kernels (SGS, Psource,
-// Pgrad): the z-neighbours a thread reads next are the ones it just read
-static constexpr int kCellK = 8;
+// The one-cell kernels (SGS, Psource, Pgrad) give a thread up to kCellK
+// planes of one (i, j): the z-neighbours it reads next are the ones it just
+// read.  Where that makes fewer than kFillBlocks blocks (two per SM) it
+// takes fewer planes: 64x32x64 has 128 blocks at 8 planes, and its threads'
+// serial planes cost 12-15 us in kernels of 1 MB.  The columns are laid out
+// flat (kCellCols per block), so a short row leaves no lanes idle.
+static constexpr int kCellK = 8, kCellCols = 128;
+static constexpr int64_t kFillBlocks = 2 * 148;
+#define CELL_COLUMN()                                              \
+  const int col_ = blockIdx.x * kCellCols + threadIdx.x;           \
+  if (col_ >= D.nx * D.ny) return;                                 \
+  const int j = 2 + col_ / D.nx, i = 2 + col_ - (j - 2) * D.nx;    \
+  const int k0 = 2 + blockIdx.y * per;                             \
+  const int kend = min(k0 + per, D.nz + 2)  /* exclusive */
 
 // --------------------------------------------------------------- RHS
 // The right-hand-side functions read their fields through an accessor A_:
@@ -261,8 +272,9 @@ __device__ __forceinline__ double rhs_scalar(const NSDev& D, const Acc& A_, int 
 // first = substep with a1 = 0 after zero_temps: q is known to be zero,
 // so it is not read (0*0 + x == 0 + x).
 //
-// Tiled: a block owns 32 (i) x 8 (j) columns and marches kRT_K planes in
-// z.  u, v, w and rho are staged in shared memory plane by plane (the
+// Tiled: a block owns 32 (i) x 8 (j) columns and marches `per` planes in z
+// (kRT_K = 32, fewer on grids that would not fill the GPU: 64x32x64 has 16
+// tiles of 32 planes, 59 us; 4 planes still repay the two halo planes).  u, v, w and rho are staged in shared memory plane by plane (the
 // tile plus a one-cell halo), four planes per field in a ring: the
 // functions read planes k-1, k, k+1 while the block brings plane k+2 in
 // with asynchronous copies, so every field value is read from global memory once
@@ -306,14 +318,15 @@ struct TileAcc {
 constexpr size_t rhs_smem_bytes(bool les) { return (size_t)(les ? 6 : 4) * 4 * kRT_PL * sizeof(double); }
 
 template <bool kFirst, bool kU, bool kL>
-__global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(NSDev D, double a1, double a2, double dt) {
+__global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(NSDev D, double a1, double a2, double dt,
+                                                                       int per) {
   extern __shared__ double sm[];
   constexpr int NF = kL ? 6 : 4;
   const int t = threadIdx.x;
   const int tx = t & 31, ty = t >> 5;
-  const int i0 = 2 + blockIdx.x * kRT_I, j0 = 2 + blockIdx.y * kRT_J, k0 = 2 + blockIdx.z * kRT_K;
+  const int i0 = 2 + blockIdx.x * kRT_I, j0 = 2 + blockIdx.y * kRT_J, k0 = 2 + blockIdx.z * per;
   const int i = i0 + tx, j = j0 + ty;
-  const int kend = min(k0 + kRT_K, D.nz + 2);  // exclusive
+  const int kend = min(k0 + per, D.nz + 2);  // exclusive
   const double* fld[6] = {D.u, D.v, D.w, D.rho, D.nuT, D.kT};
   // plane element e of the tile (halo included) -> global offset, or -1
   int64_t off[kRT_PER];
@@ -424,45 +437,29 @@ __device__ __forceinline__ void zghost_column(const NSDev& D, const ZRule& R, do
 }
 
 // Periodic images in x and y (BC.F90:55-63 with TB = 3 in x and y) of up
-// to three fields, after their interior columns are final (z ghosts
+// to five fields, after their interior columns are final (z ghosts
 // included): one thread per (ghost column of the ring, k).  Every copy
 // reads an interior column, so the order of the copies does not matter:
 //   (1, j) <- (nx+1, j), (nx+2, j) <- (2, j)      j = 2..ny+1
 //   (i, 1) <- (i, ny+1), (i, ny+2) <- (i, 2)      i = 2..nx+1
 //   corners from the diagonally opposite interior column.
-struct Fields3 {
-  double* a[3];
+struct ImageFields {
+  double* a[5];
   int n;
 };
 
-__global__ void k_images(NSDev D, Fields3 F) {
-  const int nx = D.nx, ny = D.ny;
-  const int ring = 2 * ny + 2 * nx + 4;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ring) return;
-  const int k = 1 + blockIdx.y;
-  int di, dj, si, sj;
+// ghost column t of the ring and the interior column it copies
+__device__ __forceinline__ void ring_column(int t, int nx, int ny, int& di, int& dj, int& si, int& sj) {
   if (t < 2 * ny) {
     const int j = 2 + (t % ny);
     dj = sj = j;
-    if (t < ny) {
-      di = 1;
-      si = nx + 1;
-    } else {
-      di = nx + 2;
-      si = 2;
-    }
+    di = t < ny ? 1 : nx + 2;
+    si = t < ny ? nx + 1 : 2;
   } else if (t < 2 * ny + 2 * nx) {
     const int u = t - 2 * ny;
-    const int i = 2 + (u % nx);
-    di = si = i;
-    if (u < nx) {
-      dj = 1;
-      sj = ny + 1;
-    } else {
-      dj = ny + 2;
-      sj = 2;
-    }
+    di = si = 2 + (u % nx);
+    dj = u < nx ? 1 : ny + 2;
+    sj = u < nx ? ny + 1 : 2;
   } else {
     const int c = t - 2 * ny - 2 * nx;
     di = (c & 1) ? nx + 2 : 1;
@@ -470,17 +467,63 @@ __global__ void k_images(NSDev D, Fields3 F) {
     dj = (c & 2) ? ny + 2 : 1;
     sj = (c & 2) ? 2 : ny + 1;
   }
+}
+
+__global__ void k_images(NSDev D, ImageFields F) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2 * D.ny + 2 * D.nx + 4) return;
+  const int k = 1 + blockIdx.y;
+  int di, dj, si, sj;
+  ring_column(t, D.nx, D.ny, di, dj, si, sj);
   const int64_t dst = NS_IX(di, dj, k), src = NS_IX(si, sj, k);
   for (int f = 0; f < F.n; ++f) F.a[f][dst] = F.a[f][src];
 }
 
-// Generic z-ghost pass of one field: one thread per interior column (the
-// periodic images follow in k_images).
-__global__ void k_ghost_field(NSDev D, double* a, ZRule R) {
-  const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  if (i > D.nx + 1) return;
-  zghost_column(D, R, a, NS_IX(i, j, 1));
+// The ghost pass of up to three fields in one launch (blockIdx.y: field).
+// The first nba blocks take one interior column per thread: the z walls
+// (zghost_column), then the column's four end rows 1, 2, nz+1, nz+2 -- the
+// only ones a z rule writes -- to its periodic images.  The other blocks
+// copy rows 3..nz of the ring's columns as k_images does; no row is both
+// read and written.  A launch costs 4 us on a 192x96x96 field whatever it
+// does: one instead of two for each of the dynamic models' ~240 ghost
+// passes.
+struct GhostFields {
+  double* a[3];
+  ZRule R[3];
+};
+
+__global__ void __launch_bounds__(128) k_ghost_images(NSDev D, GhostFields F, int nba) {
+  double* a = F.a[blockIdx.y];
+  const int nx = D.nx, ny = D.ny, nz = D.nz;
+  if ((int)blockIdx.x < nba) {
+    const int c = blockIdx.x * 128 + threadIdx.x;
+    if (c >= nx * ny) return;
+    const int j = 2 + c / nx, i = 2 + c % nx;
+    const int64_t base = NS_IX(i, j, 1);
+    zghost_column(D, F.R[blockIdx.y], a, base);
+    // image columns: x and y shifts by a period (0: none)
+    const int di = i == 2 ? nx : (i == nx + 1 ? -nx : 0);
+    const int dj = j == 2 ? ny : (j == ny + 1 ? -ny : 0);
+    if (di == 0 && dj == 0) return;
+    const int64_t ox = di, oy = (int64_t)dj * D.X;
+    const int rows[4] = {1, 2, nz + 1, nz + 2};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t o = base + D.XY * (rows[q] - 1);
+      const double v = a[o];
+      if (di) a[o + ox] = v;
+      if (dj) a[o + oy] = v;
+      if (di && dj) a[o + ox + oy] = v;
+    }
+  } else {
+    const int ring = 2 * ny + 2 * nx + 4;
+    const int64_t t = (int64_t)(blockIdx.x - nba) * 128 + threadIdx.x;
+    const int k = 3 + (int)(t / ring);
+    if (k > nz) return;
+    int di, dj, si, sj;
+    ring_column((int)(t % ring), nx, ny, di, dj, si, sj);
+    a[NS_IX(di, dj, k)] = a[NS_IX(si, sj, k)];
+  }
 }
 
 // ------------------------------------------------------- CN (z implicit)
@@ -502,13 +545,12 @@ struct CNFac {
 constexpr int kCNU = 8;
 constexpr int kCNThreads = 256;
 
-// U rows per batch, TPB threads (columns) per block: the launch variants
-// the autotuner chooses from (launch_cn); the arithmetic does not depend
-// on them.
-template <int kVar, int U = kCNU, int TPB = kCNThreads>
-__global__ void __launch_bounds__(TPB) k_cn_column(NSDev D, double* __restrict__ fld,
-                                                          const double* __restrict__ q, CNFac F,
-                                                          double a3, double rkdt, ZRule R) {
+// U rows per batch: with the columns per block, the launch variants the
+// autotuner chooses from (launch_cn); the arithmetic does not depend on
+// them.
+template <int kVar, int U>
+__device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ fld, const double* __restrict__ q,
+                                          const CNFac& F, double a3, double rkdt, const ZRule& R) {
   extern __shared__ double cn_sm[];
   const int n = D.nz + 2;
   const int S = n + 1;
@@ -602,6 +644,31 @@ __global__ void __launch_bounds__(TPB) k_cn_column(NSDev D, double* __restrict__
   zghost_column(D, R, fld, base);
 }
 
+// The column solves of all variables in one launch (blockIdx.z: job): they
+// read and write nothing of one another's.  On its own a variable's launch
+// lasts one column's serial chain (25 us at 64 rows) with most SMs idle on
+// the small grids: 64x32x64 has 8 blocks of 256 columns per variable.
+struct CNJob {
+  double* fld;
+  const double* q;
+  const double* kT;  // LES: eddy coefficient and eliminated-diagonal scratch
+  double* b;
+  CNFac F;
+  ZRule R;
+  int var;
+};
+struct CNJobs {
+  CNJob j[5];
+  int n;
+};
+
+template <int U, int TPB>
+__global__ void __launch_bounds__(TPB) k_cn_column(NSDev D, CNJobs J, double a3, double rkdt) {
+  const CNJob& c = J.j[blockIdx.z];
+  if (c.var == 3) cn_column<3, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R);
+  else cn_column<1, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R);
+}
+
 // LES form of var_advance_CN_PL (NSsolver.F90:3054-3465 with Vmodel =
 // SSM): every row adds the eddy terms of the column's kT to the DNS
 // coefficients, so the tridiagonal system differs per column and is
@@ -677,12 +744,11 @@ __device__ __forceinline__ double les_sup(const double* s_c, const double* s_re,
     return s_c[k - 1] - rkdt * t2 * s_re[k - 1] * s_rc[k];
 }
 
-template <int kVar, bool kU, int U = kCNU, int TPB = kCNThreads>
-__global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, double* __restrict__ fld,
-                                                              const double* __restrict__ q, CNFac F,
-                                                              double a3, double rkdt, ZRule R,
-                                                              const double* __restrict__ kT,
-                                                              double* __restrict__ bb) {
+template <int kVar, bool kU, int U>
+__device__ __forceinline__ void cn_column_les(const NSDev& D, double* __restrict__ fld,
+                                              const double* __restrict__ q, const CNFac& F, double a3, double rkdt,
+                                              const ZRule& R, const double* __restrict__ kT,
+                                              double* __restrict__ bb) {
   extern __shared__ double cn_sm[];
   const int n = D.nz + 2;
   const int S = n + 1;
@@ -828,16 +894,24 @@ __global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, double* __restri
   zghost_column(D, R, fld, base);
 }
 
+template <bool kU, int U, int TPB>
+__global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, CNJobs J, double a3, double rkdt) {
+  const CNJob& c = J.j[blockIdx.z];
+  switch (c.var) {
+    case 1: cn_column_les<1, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
+    case 2: cn_column_les<2, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
+    case 3: cn_column_les<3, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
+    case 5: cn_column_les<5, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
+    default: cn_column_les<8, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
+  }
+}
+
 // ------------------------------------------------------------------ SGS
 // SGSdiff (straincal.F90:339-414) with straincal's strain magnitude
 // (:48-73) on the interior: nuT = -(Csgs + 0) delg^2 |S| + 0 and the same
 // with CTsgs (kappaT) and CSsgs (nappaT); x**2.d0 is x*x.
-__global__ void __launch_bounds__(128) k_sgs(NSDev D) {
-  const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  const int k0 = 2 + blockIdx.z * kCellK;
-  if (i > D.nx + 1) return;
-  const int kend = min(k0 + kCellK, D.nz + 2);  // exclusive
+__global__ void __launch_bounds__(kCellCols) k_sgs(NSDev D, int per) {
+  CELL_COLUMN();
   for (int k = k0; k < kend; ++k) {
     const double modS = strain_mag(D, D.u, D.v, D.w, i, j, k);
     const double dg2 = D.delg2[k - 1];
@@ -875,12 +949,8 @@ __global__ void k_clip(NSDev D, double* a, double vmin, double vmax) {
 // ------------------------------------------------------------ Psource
 // NSsolver.F90:2167-2223 (its ghost pass is not needed: the multigrid
 // reads the interior of the right-hand side only).
-__global__ void k_psource(NSDev D, double rdt) {
-  const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  const int k0 = 2 + blockIdx.z * kCellK;
-  if (i > D.nx + 1) return;
-  const int kend = min(k0 + kCellK, D.nz + 2);  // exclusive
+__global__ void __launch_bounds__(kCellCols) k_psource(NSDev D, double rdt, int per) {
+  CELL_COLUMN();
   for (int k = k0; k < kend; ++k) {
     const double rk = D.rz[k - 1];
     const double H = 0.5;
@@ -895,18 +965,14 @@ __global__ void k_psource(NSDev D, double rdt) {
 
 // ------------------------------------------------------ Pgrad + ghosts
 // Pgrad (NSsolver.F90:2023-2085): one thread per interior cell (the update
-// of a cell reads p only), then ghost(u,'u'), ghost(v,'v'), ghost(w,'w')
-// (NSsolver.F90:572-574) by columns.
+// of a cell reads p only); ghost(u,'u'), ghost(v,'v'), ghost(w,'w')
+// (NSsolver.F90:572-574) follow in one k_ghost_images.
 // hist (may be null): the interior of p is also copied there (the history
 // of the pressure initial guess).  kU: r is 1 on every plane, so the
 // divisions by r are left out (x / 1.0 == x exactly in IEEE arithmetic).
 template <bool kU>
-__global__ void __launch_bounds__(128) k_pgrad(NSDev D, double dt, double* __restrict__ hist) {
-  const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  const int k0 = 2 + blockIdx.z * kCellK;
-  if (i > D.nx + 1) return;
-  const int kend = min(k0 + kCellK, D.nz + 2);  // exclusive
+__global__ void __launch_bounds__(kCellCols) k_pgrad(NSDev D, double dt, double* __restrict__ hist, int per) {
+  CELL_COLUMN();
   const int kend_w = D.nz + 1 - D.ew;
   const double* __restrict__ p = D.p;
   for (int k = k0; k < kend; ++k) {
@@ -923,16 +989,6 @@ __global__ void __launch_bounds__(128) k_pgrad(NSDev D, double dt, double* __res
       FA(D.w, i, j, k) = FA(D.w, i, j, k) - (pt - pr) * MT(D.rdze, k) * dt;
     }
   }
-}
-
-__global__ void k_pgrad_ghost(NSDev D, ZRule Ru, ZRule Rv, ZRule Rw) {
-  const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = 2 + blockIdx.y;
-  if (i > D.nx + 1) return;
-  const int64_t base = NS_IX(i, j, 1);
-  zghost_column(D, Ru, D.u, base);
-  zghost_column(D, Rv, D.v, base);
-  zghost_column(D, Rw, D.w, base);
 }
 
 // -------------------------------------------------------------- calcdt
@@ -1044,120 +1100,139 @@ __global__ void __launch_bounds__(128) k_divergence(NSDev D, unsigned long long*
 }
 
 // ------------------------------------------------------------ launchers
-static void launch_images(const NSDev& D, double* a0, double* a1, double* a2, cudaStream_t s) {
-  Fields3 F{{a0, a1, a2}, a2 ? 3 : (a1 ? 2 : 1)};
+static void launch_images(const NSDev& D, const ImageFields& F, cudaStream_t s) {
   const int ring = 2 * D.ny + 2 * D.nx + 4;
   k_images<<<dim3((unsigned)((ring + 127) / 128), (unsigned)D.Z, 1u), 128, 0, s>>>(D, F);
+  count_launch();
+}
+
+static void launch_ghost_images(const NSDev& D, const GhostFields& F, int n, cudaStream_t s) {
+  const int nba = (D.nx * D.ny + 127) / 128;
+  const int64_t copies = D.nz > 2 ? (int64_t)(2 * D.ny + 2 * D.nx + 4) * (D.nz - 2) : 0;
+  k_ghost_images<<<dim3((unsigned)(nba + (copies + 127) / 128), (unsigned)n), 128, 0, s>>>(D, F, nba);
   count_launch();
 }
 
 static dim3 cell_grid(const NSDev& D, int tx) {
   return dim3((unsigned)((D.nx + tx - 1) / tx), (unsigned)D.ny, (unsigned)D.nz);
 }
-// kernels whose thread does kCellK planes of one (i, j)
-static dim3 cell_grid_k(const NSDev& D, int tx) {
-  return dim3((unsigned)((D.nx + tx - 1) / tx), (unsigned)D.ny, (unsigned)((D.nz + kCellK - 1) / kCellK));
+// planes per z-block of a kernel with `cols` blocks of columns: `most`,
+// halved down to `least` while the blocks do not fill the GPU
+static int fill_planes(const NSDev& D, int64_t cols, int most, int least) {
+  int per = most;
+  while (per > least && cols * ((D.nz + per - 1) / per) < kFillBlocks) per /= 2;
+  return per;
+}
+// kernels whose thread takes *per planes of one (i, j)
+static dim3 cell_grid_k(const NSDev& D, int* per) {
+  const int64_t cols = ((int64_t)D.nx * D.ny + kCellCols - 1) / kCellCols;
+  *per = fill_planes(D, cols, kCellK, 1);
+  return dim3((unsigned)cols, (unsigned)((D.nz + *per - 1) / *per), 1u);
 }
 static dim3 col_grid(const NSDev& D, int tx) {
   return dim3((unsigned)((D.nx + tx - 1) / tx), (unsigned)D.ny, 1u);
 }
 
 template <bool kFirst, bool kU, bool kL>
-static void rhs_launch(const NSDev& D, dim3 g, double a1, double a2, double dt, cudaStream_t s) {
+static void rhs_launch(const NSDev& D, dim3 g, int per, double a1, double a2, double dt, cudaStream_t s) {
   const size_t sm = rhs_smem_bytes(kL);
   if (kL) set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL>, (int)sm);
-  k_rhs_accum<kFirst, kU, kL><<<g, kRT_I * kRT_J, sm, s>>>(D, a1, a2, dt);
+  k_rhs_accum<kFirst, kU, kL><<<g, kRT_I * kRT_J, sm, s>>>(D, a1, a2, dt, per);
 }
 
 void launch_rhs_accum(const NSDev& D, double a1, double a2, double dt, bool first, cudaStream_t s) {
-  const dim3 g((unsigned)((D.nx + kRT_I - 1) / kRT_I), (unsigned)((D.ny + kRT_J - 1) / kRT_J),
-               (unsigned)((D.nz + kRT_K - 1) / kRT_K));
+  dim3 g((unsigned)((D.nx + kRT_I - 1) / kRT_I), (unsigned)((D.ny + kRT_J - 1) / kRT_J));
+  const int per = fill_planes(D, (int64_t)g.x * g.y, kRT_K, 4);
+  g.z = (unsigned)((D.nz + per - 1) / per);
   const bool les = D.nuT && D.kT;
   const int sel = (first ? 4 : 0) + (D.unit_r ? 2 : 0) + (les ? 1 : 0);
   switch (sel) {
-    case 0: rhs_launch<false, false, false>(D, g, a1, a2, dt, s); break;
-    case 1: rhs_launch<false, false, true>(D, g, a1, a2, dt, s); break;
-    case 2: rhs_launch<false, true, false>(D, g, a1, a2, dt, s); break;
-    case 3: rhs_launch<false, true, true>(D, g, a1, a2, dt, s); break;
-    case 4: rhs_launch<true, false, false>(D, g, a1, a2, dt, s); break;
-    case 5: rhs_launch<true, false, true>(D, g, a1, a2, dt, s); break;
-    case 6: rhs_launch<true, true, false>(D, g, a1, a2, dt, s); break;
-    default: rhs_launch<true, true, true>(D, g, a1, a2, dt, s); break;
+    case 0: rhs_launch<false, false, false>(D, g, per, a1, a2, dt, s); break;
+    case 1: rhs_launch<false, false, true>(D, g, per, a1, a2, dt, s); break;
+    case 2: rhs_launch<false, true, false>(D, g, per, a1, a2, dt, s); break;
+    case 3: rhs_launch<false, true, true>(D, g, per, a1, a2, dt, s); break;
+    case 4: rhs_launch<true, false, false>(D, g, per, a1, a2, dt, s); break;
+    case 5: rhs_launch<true, false, true>(D, g, per, a1, a2, dt, s); break;
+    case 6: rhs_launch<true, true, false>(D, g, per, a1, a2, dt, s); break;
+    default: rhs_launch<true, true, true>(D, g, per, a1, a2, dt, s); break;
   }
   count_launch();
 }
 
-template <int kVar, int U, int TPB>
-static void cn_launch(const NSDev& D, double* fld, const double* q, const CNFac& f, double a3, double rkdt,
-                      const ZRule& R, cudaStream_t s) {
+static CNJobs cn_jobs(const CNSet* set, int n) {
+  CNJobs J{};
+  J.n = n;
+  for (int v = 0; v < n; ++v) {
+    const CNFacHost& F = set[v].F;
+    J.j[v] = CNJob{set[v].fld, set[v].q, set[v].kT, set[v].b,
+                   CNFac{F.ap, F.bp, F.c, F.t1, F.t2, F.rb, F.isbc, F.sub, F.diag}, set[v].R, set[v].var};
+  }
+  return J;
+}
+
+static void cn_images(const NSDev& D, const CNSet* set, int n, cudaStream_t s) {
+  ImageFields F{};
+  F.n = n;
+  for (int v = 0; v < n; ++v) F.a[v] = set[v].fld;
+  launch_images(D, F, s);
+}
+
+template <int U, int TPB>
+static void cn_launch(const NSDev& D, const CNJobs& J, double a3, double rkdt, cudaStream_t s) {
   const size_t sm = 9 * (size_t)(D.nz + 3) * sizeof(double);
-  set_smem_limit_once((const void*)k_cn_column<kVar, U, TPB>, 200 * 1024);
-  k_cn_column<kVar, U, TPB><<<col_grid(D, TPB), TPB, sm, s>>>(D, fld, q, f, a3, rkdt, R);
+  set_smem_limit_once((const void*)k_cn_column<U, TPB>, 200 * 1024);
+  dim3 g = col_grid(D, TPB);
+  g.z = (unsigned)J.n;
+  k_cn_column<U, TPB><<<g, TPB, sm, s>>>(D, J, a3, rkdt);
 }
 
-template <int kVar>
-static void cn_variant(const NSDev& D, double* fld, const double* q, const CNFac& f, double a3, double rkdt,
-                       const ZRule& R, int variant, cudaStream_t s) {
+void launch_cn(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s) {
+  const CNJobs J = cn_jobs(set, n);
   switch (variant) {
-    case 1: cn_launch<kVar, 16, 128>(D, fld, q, f, a3, rkdt, R, s); break;
-    case 2: cn_launch<kVar, 16, 256>(D, fld, q, f, a3, rkdt, R, s); break;
-    case 3: cn_launch<kVar, 32, 128>(D, fld, q, f, a3, rkdt, R, s); break;
-    default: cn_launch<kVar, kCNU, kCNThreads>(D, fld, q, f, a3, rkdt, R, s); break;
+    case 1: cn_launch<16, 128>(D, J, a3, rkdt, s); break;
+    case 2: cn_launch<16, 256>(D, J, a3, rkdt, s); break;
+    case 3: cn_launch<32, 128>(D, J, a3, rkdt, s); break;
+    case 4: cn_launch<16, 32>(D, J, a3, rkdt, s); break;
+    default: cn_launch<kCNU, kCNThreads>(D, J, a3, rkdt, s); break;
   }
-}
-
-void launch_cn(const NSDev& D, int var, double* fld, const double* q, const CNFacHost& F, double a3,
-               double rkdt, const ZRule& R, int variant, cudaStream_t s) {
-  CNFac f{F.ap, F.bp, F.c, F.t1, F.t2, F.rb, F.isbc, F.sub, F.diag};
-  if (var == 3) cn_variant<3>(D, fld, q, f, a3, rkdt, R, variant, s);
-  else cn_variant<1>(D, fld, q, f, a3, rkdt, R, variant, s);
   count_launch();
-  launch_images(D, fld, nullptr, nullptr, s);
+  cn_images(D, set, n, s);
 }
 
-template <int kVar, int U, int TPB>
-static void cn_les_launch(const NSDev& D, double* fld, const double* q, const CNFac& f, double a3, double rkdt,
-                          const ZRule& R, const double* kT, double* b, cudaStream_t s) {
+template <bool kU, int U, int TPB>
+static void cn_les_launch(const NSDev& D, const CNJobs& J, double a3, double rkdt, cudaStream_t s) {
   const size_t sm = 10 * (size_t)(D.nz + 3) * sizeof(double);
-  if (D.unit_r) {
-    set_smem_limit_once((const void*)k_cn_column_les<kVar, true, U, TPB>, 200 * 1024);
-    k_cn_column_les<kVar, true, U, TPB><<<col_grid(D, TPB), TPB, sm, s>>>(D, fld, q, f, a3, rkdt, R, kT, b);
-  } else {
-    set_smem_limit_once((const void*)k_cn_column_les<kVar, false, U, TPB>, 200 * 1024);
-    k_cn_column_les<kVar, false, U, TPB><<<col_grid(D, TPB), TPB, sm, s>>>(D, fld, q, f, a3, rkdt, R, kT, b);
-  }
+  set_smem_limit_once((const void*)k_cn_column_les<kU, U, TPB>, 200 * 1024);
+  dim3 g = col_grid(D, TPB);
+  g.z = (unsigned)J.n;
+  k_cn_column_les<kU, U, TPB><<<g, TPB, sm, s>>>(D, J, a3, rkdt);
 }
 
-template <int kVar>
-static void cn_les_variant(const NSDev& D, double* fld, const double* q, const CNFac& f, double a3, double rkdt,
-                           const ZRule& R, const double* kT, double* b, int variant, cudaStream_t s) {
+template <bool kU>
+static void cn_les_variant(const NSDev& D, const CNJobs& J, double a3, double rkdt, int variant, cudaStream_t s) {
   switch (variant) {
-    case 1: cn_les_launch<kVar, 4, 128>(D, fld, q, f, a3, rkdt, R, kT, b, s); break;
-    case 2: cn_les_launch<kVar, 8, 128>(D, fld, q, f, a3, rkdt, R, kT, b, s); break;
-    case 3: cn_les_launch<kVar, 16, 128>(D, fld, q, f, a3, rkdt, R, kT, b, s); break;
-    default: cn_les_launch<kVar, kCNU, kCNThreads>(D, fld, q, f, a3, rkdt, R, kT, b, s); break;
+    case 1: cn_les_launch<kU, 4, 128>(D, J, a3, rkdt, s); break;
+    case 2: cn_les_launch<kU, 8, 128>(D, J, a3, rkdt, s); break;
+    case 3: cn_les_launch<kU, 16, 128>(D, J, a3, rkdt, s); break;
+    case 4: cn_les_launch<kU, 8, 32>(D, J, a3, rkdt, s); break;
+    default: cn_les_launch<kU, kCNU, kCNThreads>(D, J, a3, rkdt, s); break;
   }
 }
 
-void launch_cn_les(const NSDev& D, int var, double* fld, const double* q, const CNFacHost& F, double a3,
-                   double rkdt, const ZRule& R, const double* kT, double* b, int variant, cudaStream_t s) {
-  CNFac f{F.ap, F.bp, F.c, F.t1, F.t2, F.rb, F.isbc, F.sub, F.diag};
-  switch (var) {
-    case 1: cn_les_variant<1>(D, fld, q, f, a3, rkdt, R, kT, b, variant, s); break;
-    case 2: cn_les_variant<2>(D, fld, q, f, a3, rkdt, R, kT, b, variant, s); break;
-    case 3: cn_les_variant<3>(D, fld, q, f, a3, rkdt, R, kT, b, variant, s); break;
-    case 5: cn_les_variant<5>(D, fld, q, f, a3, rkdt, R, kT, b, variant, s); break;
-    default: cn_les_variant<8>(D, fld, q, f, a3, rkdt, R, kT, b, variant, s); break;
-  }
+void launch_cn_les(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s) {
+  const CNJobs J = cn_jobs(set, n);
+  if (D.unit_r) cn_les_variant<true>(D, J, a3, rkdt, variant, s);
+  else cn_les_variant<false>(D, J, a3, rkdt, variant, s);
   count_launch();
-  launch_images(D, fld, nullptr, nullptr, s);
+  cn_images(D, set, n, s);
 }
 
 void launch_sgs(const NSDev& D, const ZRule& cfluc, cudaStream_t s) {
-  k_sgs<<<cell_grid_k(D, 128), 128, 0, s>>>(D);
-  for (double* a : {D.nuT, D.kT, D.nT}) k_ghost_field<<<col_grid(D, 64), 64, 0, s>>>(D, a, cfluc);
-  count_launch(4);
-  launch_images(D, D.nuT, D.kT, D.nT, s);
+  int per;
+  const dim3 g = cell_grid_k(D, &per);
+  k_sgs<<<g, kCellCols, 0, s>>>(D, per);
+  count_launch();
+  launch_ghost_images(D, GhostFields{{D.nuT, D.kT, D.nT}, {cfluc, cfluc, cfluc}}, 3, s);
 }
 
 // ------------------------------------------------------ plane statistics
@@ -1357,8 +1432,9 @@ void launch_clip(const NSDev& D, double* a, double vmin, double vmax, cudaStream
 }
 
 void launch_psource(const NSDev& D, double dt, cudaStream_t s) {
-  const int tx = 128;
-  k_psource<<<cell_grid_k(D, tx), tx, 0, s>>>(D, 1.0 / dt);
+  int per;
+  const dim3 g = cell_grid_k(D, &per);
+  k_psource<<<g, kCellCols, 0, s>>>(D, 1.0 / dt, per);
   count_launch();
 }
 
@@ -1369,20 +1445,22 @@ void launch_extrap(const NSDev& D, double* p, const double* h1, const double* h2
 
 void launch_pgrad(const NSDev& D, double dt, const ZRule& Ru, const ZRule& Rv, const ZRule& Rw,
                   cudaStream_t s, double* hist) {
+  int per;
+  const dim3 g = cell_grid_k(D, &per);
   if (D.unit_r)
-    k_pgrad<true><<<cell_grid_k(D, 128), 128, 0, s>>>(D, dt, hist);
+    k_pgrad<true><<<g, kCellCols, 0, s>>>(D, dt, hist, per);
   else
-    k_pgrad<false><<<cell_grid_k(D, 128), 128, 0, s>>>(D, dt, hist);
-  k_pgrad_ghost<<<col_grid(D, 64), 64, 0, s>>>(D, Ru, Rv, Rw);
-  count_launch(2);
-  launch_images(D, D.u, D.v, D.w, s);
+    k_pgrad<false><<<g, kCellCols, 0, s>>>(D, dt, hist, per);
+  count_launch();
+  launch_ghost_images(D, GhostFields{{D.u, D.v, D.w}, {Ru, Rv, Rw}}, 3, s);
 }
 
 void launch_ghost_field(const NSDev& D, double* a, const ZRule& R, cudaStream_t s) {
-  const int tx = 64;
-  k_ghost_field<<<col_grid(D, tx), tx, 0, s>>>(D, a, R);
-  count_launch();
-  launch_images(D, a, nullptr, nullptr, s);
+  launch_ghost_images(D, GhostFields{{a, nullptr, nullptr}, {R, R, R}}, 1, s);
+}
+
+void launch_ghost_fields2(const NSDev& D, double* a, double* b, const ZRule& R, cudaStream_t s) {
+  launch_ghost_images(D, GhostFields{{a, b, nullptr}, {R, R, R}}, 2, s);
 }
 
 void launch_cfl_max(const NSDev& D, unsigned long long* out, cudaStream_t s) {

@@ -16,22 +16,30 @@ struct CNFacHost {
 };
 
 void launch_rhs_accum(const NSDev& D, double a1, double a2, double dt, bool first, cudaStream_t s);
-// variant: rows per load batch and columns per block of the column solve
-// (0: 8 rows, 256; 1: 16, 128; 2: 16, 256; 3: 32, 128), chosen by the
-// autotuner; every variant computes the same bits
-constexpr int kCNVariants = 4;
-void launch_cn(const NSDev& D, int var, double* fld, const double* q, const CNFacHost& F, double a3,
-               double rkdt, const ZRule& R, int variant, cudaStream_t s);
-// var_advance_CN_PL with the eddy terms (Vmodel = SSM): per-column
-// elimination; b: G-sized scratch for the eliminated diagonal (the
+// One variable's column solve (var_advance_CN_PL): var 1 u, 2 v, 3 w, 5 rho,
+// 8 scal1; LES also its eddy coefficient kT (nuT for u, v, w, kappaT for
+// rho, nappaT for scal1) and scratch b of its own for the eliminated
+// diagonal (G values).
+struct CNSet {
+  int var;
+  double* fld;
+  const double* q;
+  CNFacHost F;
+  ZRule R;
+  const double* kT;
+  double* b;
+};
+// The column solves of n <= 5 variables in one launch, then the periodic
+// images of their fields.  variant: rows per load batch and columns per
+// block (0: 8 rows, 256; 1: 16, 128; 2: 16, 256; 3: 32, 128; 4: 16, 32),
+// chosen by the autotuner; every variant computes the same bits
+constexpr int kCNVariants = 5;
+void launch_cn(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s);
+// the same with the eddy terms (Vmodel = SSM): per-column elimination (the
 // super-diagonal is formed again from kT in the back substitution).
-// kT = nuT (u, v, w), kappaT (rho), nappaT (scal1).
-// variant: rows per load batch and columns per block (0: 8 rows, 256;
-// 1: 4, 128; 2: 8, 128; 3: 16, 128), chosen by the autotuner; every
-// variant computes the same bits
-constexpr int kCNLesVariants = 4;
-void launch_cn_les(const NSDev& D, int var, double* fld, const double* q, const CNFacHost& F, double a3,
-                   double rkdt, const ZRule& R, const double* kT, double* b, int variant, cudaStream_t s);
+// variant: 0: 8 rows, 256 columns; 1: 4, 128; 2: 8, 128; 3: 16, 128; 4: 8, 32
+constexpr int kCNLesVariants = 5;
+void launch_cn_les(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s);
 // SGSdiff (straincal.F90:339-414): modS, nuT, kappaT, nappaT on the
 // interior from the model profiles, then their ghosts ('cfluc').
 void launch_sgs(const NSDev& D, const ZRule& cfluc, cudaStream_t s);
@@ -47,6 +55,7 @@ void launch_pgrad(const NSDev& D, double dt, const ZRule& Ru, const ZRule& Rv, c
 // p = 2 h1 - h2 on the interior (the extrapolated pressure guess)
 void launch_extrap(const NSDev& D, double* p, const double* h1, const double* h2, cudaStream_t s);
 void launch_ghost_field(const NSDev& D, double* a, const ZRule& R, cudaStream_t s);
+void launch_ghost_fields2(const NSDev& D, double* a, double* b, const ZRule& R, cudaStream_t s);
 // clipVS (Routines.F90:301-380) of a cell-centred field's interior
 void launch_clip(const NSDev& D, double* a, double vmin, double vmax, cudaStream_t s);
 void launch_cfl_max(const NSDev& D, unsigned long long* out, cudaStream_t s);

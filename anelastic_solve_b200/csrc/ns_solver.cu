@@ -184,8 +184,10 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
     ANEL_CUDA_TRY(cudaMemset(d_les_, 0, 4 * (size_t)Z * sizeof(double)));
   }
   if (ns->vmodel != ANEL_MODEL_DNS) {
-    // per-column eliminated diagonal of the LES CN solve
-    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, G_ * sizeof(double)));
+    // per-column eliminated diagonal of the LES CN solve: one array per
+    // variable up to kCNSharedCells cells
+    cnb_n_ = (int64_t)nx_ * ny_ * nz_ <= kCNSharedCells ? 5 : 1;
+    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, cnb_n_ * G_ * sizeof(double)));
   }
   // metrics
   std::vector<double> met;
@@ -318,22 +320,48 @@ int NSSolver::tune_cn() {
     *out = v;
     return ANEL_OK;
   };
-  const ZRule R = zrule(NV_U);
   int st = pick("k_cn_column", kCNVariants, "ANEL_CN_VARIANT", [&](int q) {
-    launch_cn(D_, 1, D_.u, D_.qu, fac(0, 0), 1.0 / 3.0, 1e-3, R, q, stream_);
+    CNSet set[5];
+    launch_cn(D_, set, cn_set(0, set), 1.0 / 3.0, 1e-3, q, stream_);
   }, &cnvar_);
   if (st == ANEL_OK && D_.vles)
     st = pick("k_cn_column_les", kCNLesVariants, "ANEL_CN_LES_VARIANT", [&](int q) {
-      launch_cn_les(D_, 1, D_.u, D_.qu, fac(0, 0), 1.0 / 3.0, 1e-3, R, D_.nuT, d_cnb_, q, stream_);
+      cn_solve_les(0, 1.0 / 3.0, 1e-3, q, stream_);
     }, &cnlesvar_);
   if (st != ANEL_OK) return st;
   if (timed) {
     // back to the state of a fresh context
-    ANEL_CUDA_TRY(cudaMemsetAsync(D_.u, 0, G_ * sizeof(double), stream_));
+    for (double* f : {D_.u, D_.v, D_.w, D_.rho, D_.s})
+      ANEL_CUDA_TRY(cudaMemsetAsync(f, 0, G_ * sizeof(double), stream_));
     ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
     cn_rkdt_[0] = -1.0;
   }
   return ANEL_OK;
+}
+
+// The column solves of a sub-step: u, v, w, rho and scal1 where it is
+// advanced.  Returns their number.
+int NSSolver::cn_set(int slot, CNSet* set) const {
+  int n = 0;
+  set[n++] = CNSet{1, D_.u, D_.qu, fac(slot, 0), zrule(NV_U), D_.nuT, nullptr};
+  set[n++] = CNSet{2, D_.v, D_.qv, fac(slot, 1), zrule(NV_V), D_.nuT, nullptr};
+  set[n++] = CNSet{3, D_.w, D_.qw, fac(slot, 2), zrule(NV_W), D_.nuT, nullptr};
+  set[n++] = CNSet{5, D_.rho, D_.qr, fac(slot, 3), zrule(NV_RHO), D_.kT, nullptr};
+  if (prm_.scal1_on) set[n++] = CNSet{8, D_.s, D_.qs, fac(slot, 4), zrule(NV_SCAL1), D_.nT, nullptr};
+  return n;
+}
+
+// LES: as many variables per launch as there are scratch arrays for their
+// eliminated diagonals (five on grids that one variable does not fill the
+// GPU with, else one).
+void NSSolver::cn_solve_les(int slot, double a3, double dt_rk, int variant, cudaStream_t s) {
+  CNSet set[5];
+  const int n = cn_set(slot, set);
+  for (int v = 0; v < n; v += cnb_n_) {
+    const int m = n - v < cnb_n_ ? n - v : cnb_n_;
+    for (int q = 0; q < m; ++q) set[v + q].b = d_cnb_ + (size_t)q * G_;
+    launch_cn_les(D_, set + v, m, a3, dt_rk, variant, s);
+  }
 }
 
 int NSSolver::upload_profiles() {
@@ -575,23 +603,19 @@ int NSSolver::substep_pre(double a1, double a2, double a3, double dt_rk, double 
   }
   D_.g = gnow_;
   launch_rhs_accum(D_, a1, a2, dt, q_zero && a1 == 0.0, s);
-  const ZRule ru = zrule(NV_U), rv = zrule(NV_V), rw = zrule(NV_W);
   // var_advance_CN_PL: with Vmodel = SSM every variable gets the eddy
   // terms (the LES block is gated on Vmodel, NSsolver.F90:3160-3190)
-  auto cn = [&](int var, double* f, const double* q, int vi, const ZRule& R, const double* kT, cudaStream_t st) {
-    if (D_.vles) launch_cn_les(D_, var, f, q, fac(slot, vi), a3, dt_rk, R, kT, d_cnb_, cnlesvar_, st);
-    else launch_cn(D_, var, f, q, fac(slot, vi), a3, dt_rk, R, cnvar_, st);
-  };
-  cn(1, D_.u, D_.qu, 0, ru, D_.nuT, s);
-  cn(2, D_.v, D_.qv, 1, rv, D_.nuT, s);
-  cn(3, D_.w, D_.qw, 2, rw, D_.nuT, s);
+  if (D_.vles) {
+    cn_solve_les(slot, a3, dt_rk, cnlesvar_, s);
+  } else {
+    CNSet set[5];
+    launch_cn(D_, set, cn_set(slot, set), a3, dt_rk, cnvar_, s);
+  }
   launch_psource(D_, dt_rk, s);
   if (prm_.pguess && cur_sub_ >= 0 && nhist_[cur_sub_] >= 2) {
     const int q = cur_sub_;
     launch_extrap(D_, D_.p, hist_[q][last_[q]], hist_[q][last_[q] ^ 1], s);
   }
-  cn(5, D_.rho, D_.qr, 3, zrule(NV_RHO), D_.kT, s);
-  if (prm_.scal1_on) cn(8, D_.s, D_.qs, 4, zrule(NV_SCAL1), D_.nT, s);
   const size_t fb = G_ * sizeof(double);
   if (io_last_sub_ && io_out_) {
     // rho and scal1 are final: copy them out during the pressure solve

@@ -172,7 +172,11 @@ class NSSolver {
   double* d_prof_ = nullptr;        // rz bgz
   double* d_les_ = nullptr;         // LES profiles: Csgs CTsgs CSsgs delg^2 (nz+2 each)
   double* d_ic_ = nullptr;          // tanh(zc) and |zc| profiles of init_shear
-  double* d_cnb_ = nullptr;         // LES CN: eliminated diagonal per cell
+  double* d_cnb_ = nullptr;         // LES CN: eliminated diagonal per cell,
+  int cnb_n_ = 1;                   // for this many variables at once
+  static constexpr int64_t kCNSharedCells = 16 << 20;
+  int cn_set(int slot, CNSet* set) const;
+  void cn_solve_les(int slot, double a3, double dt_rk, int variant, cudaStream_t s);
   bool les_any_ = false;            // a subgrid model is on: nuT/kappaT/nappaT exist
   bool les_coeffs_done_ = false;
   double* d_cn_ = nullptr;          // CN factors: 3 slots x 5 vars x 9 arrays x (nz+2)
