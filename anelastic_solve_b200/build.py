@@ -39,6 +39,7 @@ SOURCES = {
     "tune.cu": [],
     "mg_coarse.cu": ["-fmad=true"],
     "mg_spectral.cu": ["-fmad=true"],
+    "mg_rb.cu": ["-fmad=false"],
 }
 
 

@@ -16,48 +16,6 @@ template void launch_prolong<double>(const DevLevel<double>&, const DevLevel<dou
                                      cudaStream_t);
 
 // ------------------------------------------------------------- reductions
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
-    v = w > v ? w : v;
-  }
-  return v;
-}
-
-// Non-negative doubles order like their bit patterns, so the maxima are
-// accumulated exactly (and order-independently) with integer atomicMax.
-__global__ void k_relmax_copy(DevLevel<double> L, const double* __restrict__ phin,
-                              double* __restrict__ phio, unsigned long long* out) {
-  unsigned long long m1 = 0, m2 = 0;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < L.G;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int i = 1 + (int)(t % L.X);
-    const int64_t r = t / L.X;
-    const int j = 1 + (int)(r % L.Y);
-    const int k = 1 + (int)(r / L.Y);
-    const double n = phin[t];
-    if (i >= 2 && i <= L.nx + 1 && j >= 2 && j <= L.ny + 1 && k >= 2 && k <= L.nz + 1) {
-      const unsigned long long a = __double_as_longlong(fabs(n));
-      const unsigned long long d = __double_as_longlong(fabs(n - phio[t]));
-      m1 = a > m1 ? a : m1;
-      m2 = d > m2 ? d : m2;
-    }
-    phio[t] = n;
-  }
-  m1 = warp_max_u64(m1);
-  m2 = warp_max_u64(m2);
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(out, m1);
-    atomicMax(out + 1, m2);
-  }
-}
-
-void launch_relmax_copy(const DevLevel<double>& L, const double* phin, double* phio,
-                        unsigned long long* out, cudaStream_t s) {
-  k_relmax_copy<<<gs_blocks(L.G), 256, 0, s>>>(L, phin, phio, out);
-  count_launch();
-}
-
 static constexpr int kNormThreads = 256;
 
 __device__ __forceinline__ double block_sum(double v, double* sh) {

@@ -42,12 +42,6 @@ void launch_restrict(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaS
 template <typename T>
 void launch_prolong(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaStream_t s);
 
-// max|phin|, max|phin - phio| over the interior (bit patterns of the two
-// non-negative maxima accumulated in out[0], out[1]), then phio <- phin on
-// the whole ghosted array (mg_residual.F90:60-105).
-void launch_relmax_copy(const DevLevel<double>& L, const double* phin, double* phio,
-                        unsigned long long* out, cudaStream_t s);
-
 // Deterministic sums over the interior of the FP64 fine level:
 //   part[b] = per-block partial of (f - A phi)^2 and f^2; then one block
 //   folds the partials in index order into out[0], out[1].

@@ -278,6 +278,10 @@ int MGSolver::init(const anel_grid_desc* g, const anel_mg_params* p, int device)
     spec_want_ = mixed && !off && (on || !col_ || p->tolmax < 1e-10) && b[4] == 0 && b[0] == 0 && b[1] != 0 &&
                  b[3] != 0 && spec_supported(nx_, ny_, nz_);
   }
+  if (!mixed && p->smoother == ANEL_SMOOTHER_RBPGS) {
+    const int rs = build_rb_shared();
+    if (rs != ANEL_OK) return rs;
+  }
   // default density r == 1
   std::vector<double> rz(geo_[ngrid_].Z, 1.0);
   int st = build_coefficients(rz);
@@ -372,6 +376,8 @@ MGSolver::~MGSolver() {
     cudaFree(d_img32_[l]);
     cudaFree(d_colfac_[l]);
   }
+  for (double* q : d_rbz_) cudaFree(q);
+  for (int2* q : d_rbtab_) cudaFree(q);
   direct_free(dir_);
   direct_free(dirfine_);
   spec_free(spec_);
@@ -1117,7 +1123,78 @@ int MGSolver::upload_coefficients() {
     }
   }
   op_hash_ = h;
+  if (prm_.precision != ANEL_PREC_MIXED && prm_.smoother == ANEL_SMOOTHER_RBPGS) return build_rb_levels();
   return spec_want_ ? build_spec() : ANEL_OK;
+}
+
+// The coarse levels the FP64 red-black cycle does in one block: from the
+// finest level below the fine one that fits (its boundary values are zero).
+int MGSolver::build_rb_shared() {
+  rbs_.lc = 0;
+  const int top = std::min(ngrid_ - 1, kRBSharedLevels);
+  for (int l = 1; l <= top; ++l) {
+    const LevelGeom& G = geo_[l];
+    rbs_.L[l] = L64(l);
+    rbs_.pre[l] = prm_.pre_relax[l - 1];
+    rbs_.post[l] = prm_.post_relax[l - 1];
+    rbs_.cd[l] = coarsen_dirs(l);
+    RBShared t = rbs_;
+    t.lc = l;
+    if ((int64_t)G.n[0] * G.n[1] * G.n[2] > kRBSharedCells || rb_shared_bytes(t) > kRBSharedBytes) break;
+    rbs_.lc = l;
+    const int64_t ngh = G.G - (int64_t)G.n[0] * G.n[1] * G.n[2];
+    ANEL_CUDA_TRY(cudaMalloc(&d_rbtab_[l], (size_t)ngh * sizeof(int2)));
+    launch_ghost_table(L32(l, true), d_rbtab_[l], stream_);
+    rbs_.gt[l] = d_rbtab_[l];
+  }
+  rb_shared_prepare();
+  ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
+  return check_launch("ghost tables");
+}
+
+// Self-ghosting half-sweeps: x and y periodic, even and with one
+// coefficient per direction, z walls; their z coefficients with the
+// diagonal summed in stencil_update's order.
+int MGSolver::build_rb_levels() {
+  const int* b = prm_.tbc;
+  for (int l = 1; l <= ngrid_; ++l) {
+    rb_ok_[l] = false;
+    const LevelGeom& G = geo_[l];
+    const LevelCoef& c = coef_[l];
+    if (l <= rbs_.lc || b[4] != 0 || b[0] != 0 || b[1] == 0 || b[3] == 0 || G.n[0] % 2 || G.n[1] % 2) continue;
+    const double a1 = c.cx1[G.s[0] - 1], a2 = c.cx2[G.s[0] - 1], a3 = c.cy3[G.s[1] - 1], a4 = c.cy4[G.s[1] - 1];
+    bool uni = true;
+    for (int i = G.s[0]; i <= G.e[0]; ++i) uni = uni && c.cx1[i - 1] == a1 && c.cx2[i - 1] == a2;
+    for (int j = G.s[1]; j <= G.e[1]; ++j) uni = uni && c.cy3[j - 1] == a3 && c.cy4[j - 1] == a4;
+    if (!uni) continue;
+    std::vector<double> z(3 * (size_t)G.Z);
+    for (int k = 1; k <= G.Z; ++k) {
+      z[k - 1] = c.cz5[k - 1];
+      z[G.Z + k - 1] = c.cz6[k - 1];
+      z[2 * G.Z + k - 1] = -(a1 + a2 + a3 + a4 + c.dz5[k - 1] + c.dz6[k - 1]);
+    }
+    if (!d_rbz_[l]) ANEL_CUDA_TRY(cudaMalloc(&d_rbz_[l], z.size() * sizeof(double)));
+    ANEL_CUDA_TRY(cudaMemcpy(d_rbz_[l], z.data(), z.size() * sizeof(double), cudaMemcpyHostToDevice));
+    RBLevel& R = rb_[l];
+    R.nx = G.n[0];
+    R.ny = G.n[1];
+    R.nz = G.n[2];
+    R.X = G.X;
+    R.XY = (int64_t)G.X * G.Y;
+    R.phi = d_phi64_[l];
+    R.src = d_src64_[l];
+    R.a1 = a1;
+    R.a2 = a2;
+    R.a3 = a3;
+    R.a4 = a4;
+    R.zc = d_rbz_[l];
+    R.n1 = rule_[l].type[1] == 1;
+    R.nZ = rule_[l].type[3] == 1;
+    R.add1 = rule_[l].val[1] * rule_[l].dist[1];
+    R.addZ = rule_[l].val[3] * rule_[l].dist[3];
+    rb_ok_[l] = true;
+  }
+  return ANEL_OK;
 }
 
 // The direct fine-level solve needs one coefficient per direction in x and
@@ -1276,28 +1353,30 @@ void MGSolver::relax64(int l, int iters, cudaStream_t s) {
       if (prof) prof_begin(s);
       if (zl) launch_zline(L, color, zf, zf + geo_[l].Z, s);
       else if (lj) launch_zline_lj(Lj, color, zf, zf + geo_[l].Z, s);
+      else if (rb_ok_[l]) launch_rb_march(rb_[l], color, s);
       else launch_rb_sweep(L, color, s);
       if (prof) prof_end(s);
-      launch_bdry(L, L.phi, s);
+      if (zl || lj || !rb_ok_[l] || any_ghosts_) launch_bdry(L, L.phi, s);
     }
   }
   if (iters == 0) launch_bdry(L, L.phi, s);
 }
 
-// mg_cycle.F90:186-325
+// mg_cycle.F90:186-325; levels 1..lc in one launch where lc > 0
 void MGSolver::cycle64(cudaStream_t s) {
-  const int ng = ngrid_;
+  const int ng = ngrid_, lc = rbs_.lc;
   const int* pre = prm_.pre_relax;
   const int* post = prm_.post_relax;
   relax64(ng, pre[ng - 1], s);
   launch_restrict(L64(ng), L64(ng - 1), coarsen_dirs(ng - 1), s);
-  for (int l = ng - 1; l >= 2; --l) {
+  for (int l = ng - 1; l >= 2 && l > lc; --l) {
     relax64(l, pre[l - 1], s);
     launch_restrict(L64(l), L64(l - 1), coarsen_dirs(l - 1), s);
   }
-  relax64(1, pre[0], s);
-  for (int l = 1; l <= ng - 1; ++l) {
-    relax64(l, post[l - 1], s);
+  if (lc > 0) launch_rb_shared(rbs_, s);
+  else relax64(1, pre[0], s);
+  for (int l = lc > 0 ? lc : 1; l <= ng - 1; ++l) {
+    if (l > lc) relax64(l, post[l - 1], s);
     const DevLevel<double> F = L64(l + 1);
     launch_prolong(F, L64(l), coarsen_dirs(l), s);
     launch_bdry(F, F.phi, s);
@@ -1642,7 +1721,7 @@ int MGSolver::solve_fp64(double* d_phi, const double* d_rhs, cudaStream_t s,
     true_resid(d_phi, d_rhs, s, &fn);
   }
   for (iter = 1; iter <= prm_.maxcy; ++iter) {
-    cycle64(s);
+    run_captured(s, [&]() { cycle64(s); });
     if (by_resid) {
       const double res = true_resid(W.phi, d_rhs, s, nullptr);
       relmax = res;
@@ -1653,7 +1732,7 @@ int MGSolver::solve_fp64(double* d_phi, const double* d_rhs, cudaStream_t s,
       }
     } else {
       ANEL_CUDA_TRY(cudaMemsetAsync(d_max_, 0, 2 * sizeof(unsigned long long), s));
-      launch_relmax_copy(W, W.phi, d_phi, d_max_, s);
+      launch_relmax_rows(W, W.phi, d_phi, d_max_, s);
       copy_words(d_max_, h_pin_, 2, s);
       ANEL_CUDA_TRY(cudaStreamSynchronize(s));
       const double v1 = h_pin_[0], v2 = h_pin_[1];  // bit patterns of the maxima
@@ -1691,13 +1770,15 @@ int MGSolver::solve_fp64(double* d_phi, const double* d_rhs, cudaStream_t s,
 // same order, so results are unchanged.  Profiling runs (events between
 // sweeps) and the legacy default stream stay uncaptured.
 void MGSolver::run_cycle32(cudaStream_t s) {
-  float* const e = d_phi32_[ngrid_];
-  const int64_t ne = fp32_elems(ngrid_);
-  auto cycle = [&]() {
-    cudaMemsetAsync(e, 0, ne * sizeof(float), s);
+  run_captured(s, [&]() {
+    cudaMemsetAsync(d_phi32_[ngrid_], 0, fp32_elems(ngrid_) * sizeof(float), s);
     if (col_) cycle_col(s);
     else cycle32(s);
-  };
+  });
+}
+
+template <class F>
+void MGSolver::run_captured(cudaStream_t s, F cycle) {
   const bool can = !prof_ && !g32_off_ && s != nullptr && s != cudaStreamLegacy &&
                    s != cudaStreamPerThread;
   if (!can || (++g32_calls_ < 2 && !g32x_)) {
@@ -2210,6 +2291,11 @@ int MGSolver::debug_pass(int which, double* d_phi, const double* d_src, cudaStre
   if (!s) s = stream_;
   const int ng = ngrid_;
   const DevLevel<double> W = L64(ng);
+  any_ghosts_ = true;
+  struct Reset {
+    bool& b;
+    ~Reset() { b = false; }
+  } reset{any_ghosts_};
   if (which == 1) {
     DevLevel<double> F = fine_view(d_phi, d_src);
     launch_bdry(F, d_phi, s);

@@ -7,6 +7,7 @@
 #include "mg_coarse.h"
 #include "mg_col.h"
 #include "mg_launch.h"
+#include "mg_rb.h"
 #include "mg_spectral.h"
 
 namespace anel {
@@ -67,6 +68,18 @@ class MGSolver {
   int upload_coefficients();
   void relax64(int l, int iters, cudaStream_t s);
   void cycle64(cudaStream_t s);
+  // FP64 red-black cycle (mg_rb.cu): levels whose half-sweeps write their
+  // own ghosts, and the coarse levels 1..rbs_.lc done by one block (0: none)
+  bool rb_ok_[ANEL_MAX_LEVELS + 1] = {};
+  bool any_ghosts_ = false;  // a debug pass: the caller's ghosts may be anything
+  RBLevel rb_[ANEL_MAX_LEVELS + 1];
+  double* d_rbz_[ANEL_MAX_LEVELS + 1] = {nullptr};
+  RBShared rbs_{};
+  int2* d_rbtab_[kRBSharedLevels + 1] = {nullptr};
+  int build_rb_shared();
+  int build_rb_levels();
+  template <class F>
+  void run_captured(cudaStream_t s, F cycle);
   void relax32(int l, int iters, cudaStream_t s);
   void cycle32(cudaStream_t s);
   // correction reset + FP32 V-cycle, replayed from a CUDA graph after the
