@@ -46,6 +46,18 @@ struct NSDev {
   int unit_r;  // r and densityBG are 1 on every plane (ghosts included)
 };
 
+// The members a launch works on (one, or up to kNSMany of an ensemble
+// cohort, all on one grid) and a value per member.
+constexpr int kNSMany = 16;
+template <int N>
+struct NSMany {
+  NSDev d[N];
+};
+template <int N>
+struct NSScal {
+  double v[N];
+};
+
 #define NS_IX(i, j, k) ((int64_t)((i) - 1) + (int64_t)D.X * ((j) - 1) + D.XY * ((k) - 1))
 #define FA(a, i, j, k) (a)[NS_IX(i, j, k)]
 #define MT(a, i) (a)[(i) - 1]

@@ -3,6 +3,8 @@
 // expressions evaluated left to right (citations per kernel).
 #include "ns_launch.h"
 
+#include <type_traits>
+
 namespace anel {
 
 static constexpr double R12 = 1.0 / 2.0;  // ratios::r_1_2 (modules.F90:203)
@@ -317,14 +319,18 @@ struct TileAcc {
 // shared-memory bytes of k_rhs_accum: four planes of 4 (6 with kL) fields
 constexpr size_t rhs_smem_bytes(bool les) { return (size_t)(les ? 6 : 4) * 4 * kRT_PL * sizeof(double); }
 
-template <bool kFirst, bool kU, bool kL>
-__global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(NSDev D, double a1, double a2, double dt,
-                                                                       int per) {
+template <bool kFirst, bool kU, bool kL, int N>
+__global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(const __grid_constant__ NSMany<N> P, double a1,
+                                                                double a2, const __grid_constant__ NSScal<N> dts,
+                                                                int per, int zb) {
   extern __shared__ double sm[];
+  const int m_ = N > 1 ? blockIdx.z / zb : 0;
+  const NSDev& D = P.d[m_];
+  const double dt = dts.v[m_];
   constexpr int NF = kL ? 6 : 4;
   const int t = threadIdx.x;
   const int tx = t & 31, ty = t >> 5;
-  const int i0 = 2 + blockIdx.x * kRT_I, j0 = 2 + blockIdx.y * kRT_J, k0 = 2 + blockIdx.z * per;
+  const int i0 = 2 + blockIdx.x * kRT_I, j0 = 2 + blockIdx.y * kRT_J, k0 = 2 + (blockIdx.z - m_ * zb) * per;
   const int i = i0 + tx, j = j0 + ty;
   const int kend = min(k0 + per, D.nz + 2);  // exclusive
   const double* fld[6] = {D.u, D.v, D.w, D.rho, D.nuT, D.kT};
@@ -437,15 +443,14 @@ __device__ __forceinline__ void zghost_column(const NSDev& D, const ZRule& R, do
 }
 
 // Periodic images in x and y (BC.F90:55-63 with TB = 3 in x and y) of up
-// to five fields, after their interior columns are final (z ghosts
+// to five fields of each member (blockIdx.z: field), after their interior columns are final (z ghosts
 // included): one thread per (ghost column of the ring, k).  Every copy
 // reads an interior column, so the order of the copies does not matter:
 //   (1, j) <- (nx+1, j), (nx+2, j) <- (2, j)      j = 2..ny+1
 //   (i, 1) <- (i, ny+1), (i, ny+2) <- (i, 2)      i = 2..nx+1
 //   corners from the diagonally opposite interior column.
 struct ImageFields {
-  double* a[5];
-  int n;
+  double* a[5 * kNSMany];
 };
 
 // ghost column t of the ring and the interior column it copies
@@ -476,10 +481,12 @@ __global__ void k_images(NSDev D, ImageFields F) {
   int di, dj, si, sj;
   ring_column(t, D.nx, D.ny, di, dj, si, sj);
   const int64_t dst = NS_IX(di, dj, k), src = NS_IX(si, sj, k);
-  for (int f = 0; f < F.n; ++f) F.a[f][dst] = F.a[f][src];
+  double* a = F.a[blockIdx.z];
+  a[dst] = a[src];
 }
 
-// The ghost pass of up to three fields in one launch (blockIdx.y: field).
+// The ghost pass of up to three fields (of each member) in one launch
+// (blockIdx.y: field).
 // The first nba blocks take one interior column per thread: the z walls
 // (zghost_column), then the column's four end rows 1, 2, nz+1, nz+2 -- the
 // only ones a z rule writes -- to its periodic images.  The other blocks
@@ -487,12 +494,18 @@ __global__ void k_images(NSDev D, ImageFields F) {
 // read and written.  A launch costs 4 us on a 192x96x96 field whatever it
 // does: one instead of two for each of the dynamic models' ~240 ghost
 // passes.
-struct GhostFields {
-  double* a[3];
+template <int N>
+struct GhostFields {  // n fields of each member; the rules are the members' common ones
+  double* a[3 * N];
   ZRule R[3];
+  int n;
 };
 
-__global__ void __launch_bounds__(128) k_ghost_images(NSDev D, GhostFields F, int nba) {
+template <int N>
+__global__ void __launch_bounds__(128) k_ghost_images(const __grid_constant__ NSMany<N> P,
+                                                      const __grid_constant__ GhostFields<N> F, int nba) {
+  const int m = N > 1 ? blockIdx.y / F.n : 0;
+  const NSDev& D = P.d[m];
   double* a = F.a[blockIdx.y];
   const int nx = D.nx, ny = D.ny, nz = D.nz;
   if ((int)blockIdx.x < nba) {
@@ -500,7 +513,7 @@ __global__ void __launch_bounds__(128) k_ghost_images(NSDev D, GhostFields F, in
     if (c >= nx * ny) return;
     const int j = 2 + c / nx, i = 2 + c % nx;
     const int64_t base = NS_IX(i, j, 1);
-    zghost_column(D, F.R[blockIdx.y], a, base);
+    zghost_column(D, F.R[blockIdx.y - m * F.n], a, base);
     // image columns: x and y shifts by a period (0: none)
     const int di = i == 2 ? nx : (i == nx + 1 ? -nx : 0);
     const int dj = j == 2 ? ny : (j == ny + 1 ? -ny : 0);
@@ -657,13 +670,19 @@ struct CNJob {
   ZRule R;
   int var;
 };
-struct CNJobs {
-  CNJob j[5];
+template <int N>
+struct CNJobs {  // member m's at j[m * n]
+  CNJob j[5 * N];
   int n;
 };
 
-template <int U, int TPB>
-__global__ void __launch_bounds__(TPB) k_cn_column(NSDev D, CNJobs J, double a3, double rkdt) {
+template <int U, int TPB, int N>
+__global__ void __launch_bounds__(TPB) k_cn_column(const __grid_constant__ NSMany<N> P,
+                                                   const __grid_constant__ CNJobs<N> J, double a3,
+                                                   const __grid_constant__ NSScal<N> rkdts) {
+  const int m = N > 1 ? blockIdx.z / J.n : 0;
+  const NSDev& D = P.d[m];
+  const double rkdt = rkdts.v[m];
   const CNJob& c = J.j[blockIdx.z];
   if (c.var == 3) cn_column<3, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R);
   else cn_column<1, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R);
@@ -895,7 +914,7 @@ __device__ __forceinline__ void cn_column_les(const NSDev& D, double* __restrict
 }
 
 template <bool kU, int U, int TPB>
-__global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, CNJobs J, double a3, double rkdt) {
+__global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, CNJobs<1> J, double a3, double rkdt) {
   const CNJob& c = J.j[blockIdx.z];
   switch (c.var) {
     case 1: cn_column_les<1, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
@@ -949,7 +968,11 @@ __global__ void k_clip(NSDev D, double* a, double vmin, double vmax) {
 // ------------------------------------------------------------ Psource
 // NSsolver.F90:2167-2223 (its ghost pass is not needed: the multigrid
 // reads the interior of the right-hand side only).
-__global__ void __launch_bounds__(kCellCols) k_psource(NSDev D, double rdt, int per) {
+template <int N>
+__global__ void __launch_bounds__(kCellCols) k_psource(const __grid_constant__ NSMany<N> P,
+                                                       const __grid_constant__ NSScal<N> rdts, int per) {
+  const NSDev& D = P.d[N > 1 ? blockIdx.z : 0];
+  const double rdt = rdts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
   for (int k = k0; k < kend; ++k) {
     const double rk = D.rz[k - 1];
@@ -970,8 +993,12 @@ __global__ void __launch_bounds__(kCellCols) k_psource(NSDev D, double rdt, int 
 // hist (may be null): the interior of p is also copied there (the history
 // of the pressure initial guess).  kU: r is 1 on every plane, so the
 // divisions by r are left out (x / 1.0 == x exactly in IEEE arithmetic).
-template <bool kU>
-__global__ void __launch_bounds__(kCellCols) k_pgrad(NSDev D, double dt, double* __restrict__ hist, int per) {
+template <bool kU, int N>
+__global__ void __launch_bounds__(kCellCols) k_pgrad(const __grid_constant__ NSMany<N> P,
+                                                     const __grid_constant__ NSScal<N> dts,
+                                                     double* __restrict__ hist, int per) {
+  const NSDev& D = P.d[N > 1 ? blockIdx.z : 0];
+  const double dt = dts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
   const int kend_w = D.nz + 1 - D.ew;
   const double* __restrict__ p = D.p;
@@ -1025,24 +1052,36 @@ __global__ void __launch_bounds__(256) k_cfl_max(NSDev D, unsigned long long* ou
   }
 }
 
-// divergence (Routines.F90:121-146): max |div| (exact) and the
-// volume-weighted sums of |div| and volume (block partials, fixed order)
-// divergence() (Routines.F90:54-183): kDivRows consecutive z-cells per
-// thread (w of the cell below kept from the previous row), per-block sums
-// of |div|*vol and vol in a fixed order, and one atomic maximum per block
-// on the bit pattern of max |div| (exact in any order).
+// divergence (Routines.F90:54-183): kDivRows consecutive z-cells per thread
+// (w of the cell below kept from the previous row), per-block sums of
+// |div|*vol and vol and maxima on the bit patterns; the member's last block
+// to arrive adds the blocks' sums in block order and writes the results to
+// out and to mapped host memory, so the pass is one launch and needs no
+// zeroing, fold or copy (seven launches of 4 us each before).
+// With cfl the same pass also takes calcdt's maximum of rdxc |u| + rdzc |w|
+// + rdyc |v| of the cell averages (the expression of k_cfl_max, in its
+// order) over the same cells and neighbours, for the next step's time step.
 constexpr int kDivRows = 8;
-// With cfl non-null the same pass also takes calcdt's maximum of
-// rdxc |ū| + rdzc |w̄| + rdyc |v̄| (the expression of k_cfl_max, in its
-// order) over the same cells and neighbours, for the next step's time
-// step: one read of u, v, w at the end of a step serves both.
-__global__ void __launch_bounds__(128) k_divergence(NSDev D, unsigned long long* mx, double* part,
-                                                    unsigned long long* cfl) {
+template <int N>
+struct DivOut {
+  double* part[N];       // 4 doubles per block
+  unsigned* count[N];
+  double* out[N];        // 4 doubles: sum |div| vol, sum vol, max |div|, CFL maximum
+  double* host[N];       // its mirror in mapped host memory
+};
+
+template <int N>
+__global__ void __launch_bounds__(128) k_divergence(const __grid_constant__ NSMany<N> P,
+                                                    const __grid_constant__ DivOut<N> O, int cfl, int zb) {
   __shared__ double sh[2][4];
   __shared__ unsigned long long shm[2][4];
+  __shared__ int last;
+  const int m_ = N > 1 ? blockIdx.z / zb : 0;
+  const NSDev& D = P.d[m_];
   const int i = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = 2 + blockIdx.y;
-  const int k0 = 2 + blockIdx.z * kDivRows;
+  const int bz = blockIdx.z - m_ * zb;
+  const int k0 = 2 + bz * kDivRows;
   double s1 = 0.0, s2 = 0.0;
   unsigned long long m = 0, mc = 0;
   if (i <= D.nx + 1) {
@@ -1066,51 +1105,226 @@ __global__ void __launch_bounds__(128) k_divergence(NSDev D, unsigned long long*
       wb = wt;
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
-    m = w > m ? w : m;
-    const unsigned long long wc = __shfl_xor_sync(0xffffffffu, mc, o);
-    mc = wc > mc ? wc : mc;
+  // the block's values to thread 0
+  auto reduce = [&]() {
+    for (int o = 16; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      const unsigned long long w = __shfl_xor_sync(0xffffffffu, m, o);
+      m = w > m ? w : m;
+      const unsigned long long wc = __shfl_xor_sync(0xffffffffu, mc, o);
+      mc = wc > mc ? wc : mc;
+    }
+    const int wid = threadIdx.x >> 5;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+      sh[0][wid] = s1;
+      sh[1][wid] = s2;
+      shm[0][wid] = m;
+      shm[1][wid] = mc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 1; q < 4; ++q) {
+        s1 += sh[0][q];
+        s2 += sh[1][q];
+        m = shm[0][q] > m ? shm[0][q] : m;
+        mc = shm[1][q] > mc ? shm[1][q] : mc;
+      }
+    }
+  };
+  reduce();
+  const int nb = gridDim.x * gridDim.y * zb;
+  double* part = O.part[m_];
+  if (threadIdx.x == 0) {
+    double* p = part + 4 * (int64_t)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * bz));
+    p[0] = s1;
+    p[1] = s2;
+    p[2] = __longlong_as_double(m);
+    p[3] = __longlong_as_double(mc);
+    __threadfence();
+    last = atomicAdd(O.count[m_], 1u) == (unsigned)nb - 1;
   }
-  const int wid = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sh[0][wid] = s1;
-    sh[1][wid] = s2;
-    shm[0][wid] = m;
-    shm[1][wid] = mc;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s1 = s2 = 0.0;
+  m = mc = 0;
+  for (int q = threadIdx.x; q < nb; q += 128) {
+    const double* p = part + 4 * (int64_t)q;
+    s1 += __ldcg(p);
+    s2 += __ldcg(p + 1);
+    const unsigned long long a = __double_as_longlong(__ldcg(p + 2)), b = __double_as_longlong(__ldcg(p + 3));
+    m = a > m ? a : m;
+    mc = b > mc ? b : mc;
+  }
+  reduce();
+  if (threadIdx.x == 0) {
+    *O.count[m_] = 0;
+    double *o = O.out[m_], *h = O.host[m_];
+    o[0] = h[0] = s1;
+    o[1] = h[1] = s2;
+    o[2] = h[2] = __longlong_as_double(m);
+    o[3] = h[3] = __longlong_as_double(mc);
+  }
+}
+
+// ---------------------------------------- Crank-Nicolson factors
+// The column-independent factors of the CN system of each variable for up
+// to three values of rkdt (var_advance_CN_PL, NSsolver.F90:3102-3296), then
+// the elimination of the Thomas routine (mg_relax.F90:563-568) applied to
+// them: one block per (variable, rkdt, member), rows in parallel, the
+// elimination by one thread.  On the host they cost a stream
+// synchronisation, 5 n divisions and a copy before each sub-step's columns.
+// nz = 512: the elimination's chain takes about 60 us once per step.
+template <int N>
+struct CNFactorJobs {
+  double* dst[N];     // 3 slots x 5 variables x 9 arrays x Z
+  double rkdt[N][3];
+  int type[5][2];     // z wall types and values of the variables
+  double val[5][2];
+};
+
+template <int N>
+__global__ void __launch_bounds__(128) k_cn_factors(const __grid_constant__ NSMany<N> P,
+                                                    const __grid_constant__ CNFactorJobs<N> J, int slot0) {
+  extern __shared__ double cn_sm[];
+  const int me = N > 1 ? blockIdx.z : 0;
+  const NSDev& D = P.d[me];
+  const int vi = blockIdx.x, slot = slot0 + blockIdx.y;
+  const int vars[5] = {1, 2, 3, 5, 8};
+  const int var = vars[vi];
+  const double rkdt = J.rkdt[me][slot];
+  const int n = D.nz + 2, sz = 2, ez = D.nz + 1;
+  const double H = 0.5;
+  double* base = J.dst[me] + ((int64_t)(slot * 5 + vi) * 9) * n;
+  double *ap = base, *bp = base + n, *c = base + 2 * n, *t1a = base + 3 * n, *t2a = base + 4 * n, *rba = base + 5 * n,
+         *isbc = base + 6 * n, *suba = base + 7 * n, *diaga = base + 8 * n;
+  double *s_sub = cn_sm, *s_dia = cn_sm + n, *s_sup = cn_sm + 2 * n;
+  auto R = [&](int k) { return D.rz[k - 1]; };
+  auto rdze = [&](int k) { return D.rdze[k - 1]; };
+  auto rdzc = [&](int k) { return D.rdzc[k - 1]; };
+  auto dze = [&](int k) { return D.dze[k - 1]; };
+  auto dzc = [&](int k) { return D.dzc[k - 1]; };
+  const int tbmin = J.type[vi][0], tbmax = J.type[vi][1];
+  const double vbmin = J.val[vi][0], vbmax = J.val[vi][1];
+  for (int k = 1 + threadIdx.x; k <= n; k += blockDim.x) {
+    double t1 = 0.0, t2 = 0.0, sub = 0.0, dia = 0.0, sup = 0.0, rb = 0.0, bc = 0.0;
+    if (k >= sz && k <= ez) {
+      if (var != 3) {
+        const double ra1 = H * (R(k + 1) + R(k));
+        const double ra2 = H * (R(k) + R(k - 1));
+        if (var == 1 || var == 2) {
+          t1 = (D.rRe + 0.0) * ra1 / R(k);
+          t2 = (D.rRe + 0.0) * ra2 / R(k);
+        } else if (var == 5) {
+          t1 = (D.rRe * D.rPr + 0.0) * ra1 / R(k);
+          t2 = (D.rRe * D.rPr + 0.0) * ra2 / R(k);
+        } else {
+          t1 = D.rRe * D.rSc + 0.0;
+          t2 = D.rRe * D.rSc + 0.0;
+        }
+        sub = -0.5 * rkdt * t1 * rdze(k - 1) * rdzc(k);
+        sup = -0.5 * rkdt * t2 * rdze(k) * rdzc(k);
+        dia = 1.0 + 0.5 * rkdt * (t1 * rdze(k - 1) + t2 * rdze(k)) * rdzc(k);
+      } else {
+        t1 = (D.rRe + 0.0) * R(k) / (H * (R(k + 1) + R(k)));
+        t2 = (D.rRe + 0.0) * R(k + 1) / (H * (R(k + 1) + R(k)));
+        sub = -0.5 * rkdt * t1 * rdze(k) * rdzc(k);
+        sup = -0.5 * rkdt * t2 * rdze(k) * rdzc(k + 1);
+        dia = 1.0 + 0.5 * rkdt * (t1 * rdzc(k) + t2 * rdzc(k + 1)) * rdze(k);
+      }
+    }
+    // wall rows (NSsolver.F90:3297-3429)
+    auto set = [&](double a, double b, double cc, double d) {
+      sub = a;
+      dia = b;
+      sup = cc;
+      rb = d;
+      bc = 1.0;
+    };
+    const bool sc = var == 5 || var == 8;
+    if (k == sz - 1) {
+      if (tbmin == 1) set(0.0, 1.0, 0.0, vbmin);
+      else if (tbmin == 2) set(0.0, -1.0, 1.0, (var == 3 ? dzc(sz - 1) : dze(sz - 1)) * vbmin);
+      else if (tbmin == 6) set(0.0, 1.0, 1.0, 2.0 * vbmin);
+    }
+    if (k == sz && tbmin == 2 && sc) set(0.0, -1.0, 1.0, dze(sz) * vbmin);
+    if (k == ez && tbmax == 2 && sc) set(-1.0, 1.0, 0.0, dze(ez) * vbmax);
+    if (k == ez && tbmax == 7) set(0.0, 1.0, 0.0, 0.0);
+    if (k == ez + 1) {
+      if (tbmax == 1) set(0.0, 1.0, 0.0, vbmax);
+      else if (tbmax == 2) set(-1.0, 1.0, 0.0, (var == 3 ? dzc(ez + 1) : dze(ez + 1)) * vbmax);
+      else if (tbmax == 6) set(1.0, 1.0, 0.0, 2.0 * vbmax);
+      else if (tbmax == 7) set(0.0, 1.0, 0.0, 0.0);
+    }
+    s_sub[k - 1] = sub;
+    s_dia[k - 1] = dia;
+    s_sup[k - 1] = sup;
+    t1a[k - 1] = t1;
+    t2a[k - 1] = t2;
+    rba[k - 1] = rb;
+    isbc[k - 1] = bc;
+    suba[k - 1] = sub;
+    diaga[k - 1] = dia;
+    c[k - 1] = sup;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    unsigned long long mm = 0, mmc = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-      a += sh[0][q];
-      b += sh[1][q];
-      mm = shm[0][q] > mm ? shm[0][q] : mm;
-      mmc = shm[1][q] > mmc ? shm[1][q] : mmc;
+    double b = s_dia[0];
+    for (int j = 1; j < n; ++j) {
+      const double a = -s_sub[j] / b;
+      b = s_dia[j] + a * s_sup[j - 1];
+      s_sub[j] = a;
+      s_dia[j] = b;
     }
-    atomicMax(mx, mm);
-    if (cfl) atomicMax(cfl, mmc);
-    const int64_t bid = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
-    part[2 * bid] = a;
-    part[2 * bid + 1] = b;
+    s_sub[0] = 0.0;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    ap[q] = s_sub[q];
+    bp[q] = s_dia[q];
   }
 }
 
 // ------------------------------------------------------------ launchers
-static void launch_images(const NSDev& D, const ImageFields& F, cudaStream_t s) {
+static void launch_images(const NSDev& D, const ImageFields& F, int n, cudaStream_t s) {
   const int ring = 2 * D.ny + 2 * D.nx + 4;
-  k_images<<<dim3((unsigned)((ring + 127) / 128), (unsigned)D.Z, 1u), 128, 0, s>>>(D, F);
+  k_images<<<dim3((unsigned)((ring + 127) / 128), (unsigned)D.Z, (unsigned)n), 128, 0, s>>>(D, F);
   count_launch();
 }
 
-static void launch_ghost_images(const NSDev& D, const GhostFields& F, int n, cudaStream_t s) {
+template <int N>
+static void launch_ghost_images(const NSMany<N>& P, const GhostFields<N>& F, int members, cudaStream_t s) {
+  const NSDev& D = P.d[0];
   const int nba = (D.nx * D.ny + 127) / 128;
   const int64_t copies = D.nz > 2 ? (int64_t)(2 * D.ny + 2 * D.nx + 4) * (D.nz - 2) : 0;
-  k_ghost_images<<<dim3((unsigned)(nba + (copies + 127) / 128), (unsigned)n), 128, 0, s>>>(D, F, nba);
+  const dim3 g((unsigned)(nba + (copies + 127) / 128), (unsigned)(F.n * members));
+  k_ghost_images<N><<<g, 128, 0, s>>>(P, F, nba);
   count_launch();
+}
+
+// f(std::integral_constant<int, N>, first member, members) over the members
+// in chunks: N = 1 for one, kNSMany for more
+template <class F>
+static void by_members(int n, F f) {
+  if (n == 1) {
+    f(std::integral_constant<int, 1>{}, 0, 1);
+    return;
+  }
+  for (int b = 0; b < n; b += kNSMany) f(std::integral_constant<int, kNSMany>{}, b, n - b < kNSMany ? n - b : kNSMany);
+}
+template <int N>
+static NSMany<N> many(const NSDev* const* D, int b, int n) {
+  NSMany<N> P;
+  for (int m = 0; m < N; ++m) P.d[m] = *D[b + (m < n ? m : 0)];
+  return P;
+}
+template <int N>
+static NSScal<N> scal(const double* v, int b, int n) {
+  NSScal<N> S;
+  for (int m = 0; m < N; ++m) S.v[m] = v[b + (m < n ? m : 0)];
+  return S;
 }
 
 static dim3 cell_grid(const NSDev& D, int tx) {
@@ -1124,45 +1338,55 @@ static int fill_planes(const NSDev& D, int64_t cols, int most, int least) {
   return per;
 }
 // kernels whose thread takes *per planes of one (i, j)
-static dim3 cell_grid_k(const NSDev& D, int* per) {
+static dim3 cell_grid_k(const NSDev& D, int* per, int members = 1) {
   const int64_t cols = ((int64_t)D.nx * D.ny + kCellCols - 1) / kCellCols;
-  *per = fill_planes(D, cols, kCellK, 1);
-  return dim3((unsigned)cols, (unsigned)((D.nz + *per - 1) / *per), 1u);
+  *per = fill_planes(D, cols * members, kCellK, 1);
+  return dim3((unsigned)cols, (unsigned)((D.nz + *per - 1) / *per), (unsigned)members);
 }
 static dim3 col_grid(const NSDev& D, int tx) {
   return dim3((unsigned)((D.nx + tx - 1) / tx), (unsigned)D.ny, 1u);
 }
 
-template <bool kFirst, bool kU, bool kL>
-static void rhs_launch(const NSDev& D, dim3 g, int per, double a1, double a2, double dt, cudaStream_t s) {
-  const size_t sm = rhs_smem_bytes(kL);
-  if (kL) set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL>, (int)sm);
-  k_rhs_accum<kFirst, kU, kL><<<g, kRT_I * kRT_J, sm, s>>>(D, a1, a2, dt, per);
-}
-
-void launch_rhs_accum(const NSDev& D, double a1, double a2, double dt, bool first, cudaStream_t s) {
+template <bool kFirst, bool kU, bool kL, int N>
+static void rhs_launch(const NSMany<N>& P, const NSScal<N>& dt, int members, double a1, double a2, cudaStream_t s) {
+  const NSDev& D = P.d[0];
   dim3 g((unsigned)((D.nx + kRT_I - 1) / kRT_I), (unsigned)((D.ny + kRT_J - 1) / kRT_J));
-  const int per = fill_planes(D, (int64_t)g.x * g.y, kRT_K, 4);
-  g.z = (unsigned)((D.nz + per - 1) / per);
-  const bool les = D.nuT && D.kT;
-  const int sel = (first ? 4 : 0) + (D.unit_r ? 2 : 0) + (les ? 1 : 0);
-  switch (sel) {
-    case 0: rhs_launch<false, false, false>(D, g, per, a1, a2, dt, s); break;
-    case 1: rhs_launch<false, false, true>(D, g, per, a1, a2, dt, s); break;
-    case 2: rhs_launch<false, true, false>(D, g, per, a1, a2, dt, s); break;
-    case 3: rhs_launch<false, true, true>(D, g, per, a1, a2, dt, s); break;
-    case 4: rhs_launch<true, false, false>(D, g, per, a1, a2, dt, s); break;
-    case 5: rhs_launch<true, false, true>(D, g, per, a1, a2, dt, s); break;
-    case 6: rhs_launch<true, true, false>(D, g, per, a1, a2, dt, s); break;
-    default: rhs_launch<true, true, true>(D, g, per, a1, a2, dt, s); break;
-  }
-  count_launch();
+  const int per = fill_planes(D, (int64_t)g.x * g.y * members, kRT_K, 4);
+  const int zb = (D.nz + per - 1) / per;
+  g.z = (unsigned)(zb * members);
+  const size_t sm = rhs_smem_bytes(kL);
+  if (kL) set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL, N>, (int)sm);
+  k_rhs_accum<kFirst, kU, kL, N><<<g, kRT_I * kRT_J, sm, s>>>(P, a1, a2, dt, per, zb);
 }
 
-static CNJobs cn_jobs(const CNSet* set, int n) {
-  CNJobs J{};
+void launch_rhs_accum(const NSDev* const* Ds, const double* dts, int n, double a1, double a2, bool first,
+                      cudaStream_t s) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    const auto dt = scal<N>(dts, b, m);
+    const NSDev& D = P.d[0];
+    const bool les = D.nuT && D.kT;
+    const int sel = (first ? 4 : 0) + (D.unit_r ? 2 : 0) + (les ? 1 : 0);
+    switch (sel) {
+      case 0: rhs_launch<false, false, false, N>(P, dt, m, a1, a2, s); break;
+      case 1: rhs_launch<false, false, true, N>(P, dt, m, a1, a2, s); break;
+      case 2: rhs_launch<false, true, false, N>(P, dt, m, a1, a2, s); break;
+      case 3: rhs_launch<false, true, true, N>(P, dt, m, a1, a2, s); break;
+      case 4: rhs_launch<true, false, false, N>(P, dt, m, a1, a2, s); break;
+      case 5: rhs_launch<true, false, true, N>(P, dt, m, a1, a2, s); break;
+      case 6: rhs_launch<true, true, false, N>(P, dt, m, a1, a2, s); break;
+      default: rhs_launch<true, true, true, N>(P, dt, m, a1, a2, s); break;
+    }
+    count_launch();
+  });
+}
+
+// n column solves of each of `members` members (member m's at set[m * n])
+template <int N>
+static CNJobs<N> cn_jobs(const CNSet* set, int n, int members) {
+  CNJobs<N> J;
   J.n = n;
-  for (int v = 0; v < n; ++v) {
+  for (int v = 0; v < n * members; ++v) {
     const CNFacHost& F = set[v].F;
     J.j[v] = CNJob{set[v].fld, set[v].q, set[v].kT, set[v].b,
                    CNFac{F.ap, F.bp, F.c, F.t1, F.t2, F.rb, F.isbc, F.sub, F.diag}, set[v].R, set[v].var};
@@ -1171,36 +1395,43 @@ static CNJobs cn_jobs(const CNSet* set, int n) {
 }
 
 static void cn_images(const NSDev& D, const CNSet* set, int n, cudaStream_t s) {
-  ImageFields F{};
-  F.n = n;
+  ImageFields F;
   for (int v = 0; v < n; ++v) F.a[v] = set[v].fld;
-  launch_images(D, F, s);
+  launch_images(D, F, n, s);
 }
 
-template <int U, int TPB>
-static void cn_launch(const NSDev& D, const CNJobs& J, double a3, double rkdt, cudaStream_t s) {
+template <int U, int TPB, int N>
+static void cn_launch(const NSMany<N>& P, const CNJobs<N>& J, int members, double a3, const NSScal<N>& rkdt,
+                      cudaStream_t s) {
+  const NSDev& D = P.d[0];
   const size_t sm = 9 * (size_t)(D.nz + 3) * sizeof(double);
-  set_smem_limit_once((const void*)k_cn_column<U, TPB>, 200 * 1024);
+  set_smem_limit_once((const void*)k_cn_column<U, TPB, N>, 200 * 1024);
   dim3 g = col_grid(D, TPB);
-  g.z = (unsigned)J.n;
-  k_cn_column<U, TPB><<<g, TPB, sm, s>>>(D, J, a3, rkdt);
+  g.z = (unsigned)(J.n * members);
+  k_cn_column<U, TPB, N><<<g, TPB, sm, s>>>(P, J, a3, rkdt);
 }
 
-void launch_cn(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s) {
-  const CNJobs J = cn_jobs(set, n);
-  switch (variant) {
-    case 1: cn_launch<16, 128>(D, J, a3, rkdt, s); break;
-    case 2: cn_launch<16, 256>(D, J, a3, rkdt, s); break;
-    case 3: cn_launch<32, 128>(D, J, a3, rkdt, s); break;
-    case 4: cn_launch<16, 32>(D, J, a3, rkdt, s); break;
-    default: cn_launch<kCNU, kCNThreads>(D, J, a3, rkdt, s); break;
-  }
-  count_launch();
-  cn_images(D, set, n, s);
+void launch_cn(const NSDev* const* Ds, const CNSet* set, int nset, const double* rkdts, int n, double a3, int variant,
+               cudaStream_t s) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    const auto rkdt = scal<N>(rkdts, b, m);
+    const CNSet* sb = set + (size_t)b * nset;
+    const auto J = cn_jobs<N>(sb, nset, m);
+    switch (variant) {
+      case 1: cn_launch<16, 128, N>(P, J, m, a3, rkdt, s); break;
+      case 2: cn_launch<16, 256, N>(P, J, m, a3, rkdt, s); break;
+      case 3: cn_launch<32, 128, N>(P, J, m, a3, rkdt, s); break;
+      case 4: cn_launch<16, 32, N>(P, J, m, a3, rkdt, s); break;
+      default: cn_launch<kCNU, kCNThreads, N>(P, J, m, a3, rkdt, s); break;
+    }
+    count_launch();
+    cn_images(P.d[0], sb, nset * m, s);
+  });
 }
 
 template <bool kU, int U, int TPB>
-static void cn_les_launch(const NSDev& D, const CNJobs& J, double a3, double rkdt, cudaStream_t s) {
+static void cn_les_launch(const NSDev& D, const CNJobs<1>& J, double a3, double rkdt, cudaStream_t s) {
   const size_t sm = 10 * (size_t)(D.nz + 3) * sizeof(double);
   set_smem_limit_once((const void*)k_cn_column_les<kU, U, TPB>, 200 * 1024);
   dim3 g = col_grid(D, TPB);
@@ -1209,7 +1440,7 @@ static void cn_les_launch(const NSDev& D, const CNJobs& J, double a3, double rkd
 }
 
 template <bool kU>
-static void cn_les_variant(const NSDev& D, const CNJobs& J, double a3, double rkdt, int variant, cudaStream_t s) {
+static void cn_les_variant(const NSDev& D, const CNJobs<1>& J, double a3, double rkdt, int variant, cudaStream_t s) {
   switch (variant) {
     case 1: cn_les_launch<kU, 4, 128>(D, J, a3, rkdt, s); break;
     case 2: cn_les_launch<kU, 8, 128>(D, J, a3, rkdt, s); break;
@@ -1220,7 +1451,7 @@ static void cn_les_variant(const NSDev& D, const CNJobs& J, double a3, double rk
 }
 
 void launch_cn_les(const NSDev& D, const CNSet* set, int n, double a3, double rkdt, int variant, cudaStream_t s) {
-  const CNJobs J = cn_jobs(set, n);
+  const CNJobs<1> J = cn_jobs<1>(set, n, 1);
   if (D.unit_r) cn_les_variant<true>(D, J, a3, rkdt, variant, s);
   else cn_les_variant<false>(D, J, a3, rkdt, variant, s);
   count_launch();
@@ -1232,7 +1463,7 @@ void launch_sgs(const NSDev& D, const ZRule& cfluc, cudaStream_t s) {
   const dim3 g = cell_grid_k(D, &per);
   k_sgs<<<g, kCellCols, 0, s>>>(D, per);
   count_launch();
-  launch_ghost_images(D, GhostFields{{D.nuT, D.kT, D.nT}, {cfluc, cfluc, cfluc}}, 3, s);
+  launch_ghost_images<1>({D}, {{D.nuT, D.kT, D.nT}, {cfluc, cfluc, cfluc}, 3}, 1, s);
 }
 
 // ------------------------------------------------------ plane statistics
@@ -1431,11 +1662,16 @@ void launch_clip(const NSDev& D, double* a, double vmin, double vmax, cudaStream
   count_launch();
 }
 
-void launch_psource(const NSDev& D, double dt, cudaStream_t s) {
-  int per;
-  const dim3 g = cell_grid_k(D, &per);
-  k_psource<<<g, kCellCols, 0, s>>>(D, 1.0 / dt, per);
-  count_launch();
+void launch_psource(const NSDev* const* Ds, const double* dts, int n, cudaStream_t s) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    auto rdt = scal<N>(dts, b, m);
+    for (double& v : rdt.v) v = 1.0 / v;
+    int per;
+    const dim3 g = cell_grid_k(P.d[0], &per, m);
+    k_psource<N><<<g, kCellCols, 0, s>>>(P, rdt, per);
+    count_launch();
+  });
 }
 
 void launch_extrap(const NSDev& D, double* p, const double* h1, const double* h2, cudaStream_t s) {
@@ -1443,24 +1679,32 @@ void launch_extrap(const NSDev& D, double* p, const double* h1, const double* h2
   count_launch();
 }
 
-void launch_pgrad(const NSDev& D, double dt, const ZRule& Ru, const ZRule& Rv, const ZRule& Rw,
-                  cudaStream_t s, double* hist) {
-  int per;
-  const dim3 g = cell_grid_k(D, &per);
-  if (D.unit_r)
-    k_pgrad<true><<<g, kCellCols, 0, s>>>(D, dt, hist, per);
-  else
-    k_pgrad<false><<<g, kCellCols, 0, s>>>(D, dt, hist, per);
-  count_launch();
-  launch_ghost_images(D, GhostFields{{D.u, D.v, D.w}, {Ru, Rv, Rw}}, 3, s);
+void launch_pgrad(const NSDev* const* Ds, const double* dts, int n, const ZRule& Ru, const ZRule& Rv,
+                  const ZRule& Rw, cudaStream_t s, double* hist) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    const auto dt = scal<N>(dts, b, m);
+    int per;
+    const dim3 g = cell_grid_k(P.d[0], &per, m);
+    if (P.d[0].unit_r) k_pgrad<true, N><<<g, kCellCols, 0, s>>>(P, dt, hist, per);
+    else k_pgrad<false, N><<<g, kCellCols, 0, s>>>(P, dt, hist, per);
+    count_launch();
+    GhostFields<N> F{{}, {Ru, Rv, Rw}, 3};
+    for (int q = 0; q < m; ++q) {
+      F.a[3 * q] = P.d[q].u;
+      F.a[3 * q + 1] = P.d[q].v;
+      F.a[3 * q + 2] = P.d[q].w;
+    }
+    launch_ghost_images<N>(P, F, m, s);
+  });
 }
 
 void launch_ghost_field(const NSDev& D, double* a, const ZRule& R, cudaStream_t s) {
-  launch_ghost_images(D, GhostFields{{a, nullptr, nullptr}, {R, R, R}}, 1, s);
+  launch_ghost_images<1>({D}, {{a, nullptr, nullptr}, {R, R, R}, 1}, 1, s);
 }
 
 void launch_ghost_fields2(const NSDev& D, double* a, double* b, const ZRule& R, cudaStream_t s) {
-  launch_ghost_images(D, GhostFields{{a, b, nullptr}, {R, R, R}}, 2, s);
+  launch_ghost_images<1>({D}, {{a, b, nullptr}, {R, R, R}, 2}, 1, s);
 }
 
 void launch_cfl_max(const NSDev& D, unsigned long long* out, cudaStream_t s) {
@@ -1475,15 +1719,47 @@ static dim3 divergence_grid(const NSDev& D) {
   return dim3((unsigned)((D.nx + 127) / 128), (unsigned)D.ny, (unsigned)((D.nz + kDivRows - 1) / kDivRows));
 }
 
-int64_t divergence_blocks(const NSDev& D) {
+int64_t divergence_part_doubles(const NSDev& D) {
   const dim3 g = divergence_grid(D);
-  return (int64_t)g.x * g.y * g.z;
+  return 4 * (int64_t)g.x * g.y * g.z;
 }
 
-void launch_divergence(const NSDev& D, unsigned long long* mx, double* part, cudaStream_t s,
-                       unsigned long long* cfl) {
-  k_divergence<<<divergence_grid(D), 128, 0, s>>>(D, mx, part, cfl);
-  count_launch();
+void launch_divergence(const NSDev* const* Ds, const DivSet* set, int n, bool cfl, cudaStream_t s) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    DivOut<N> O{};
+    for (int q = 0; q < m; ++q) {
+      O.part[q] = set[b + q].part;
+      O.count[q] = set[b + q].count;
+      O.out[q] = set[b + q].out;
+      O.host[q] = set[b + q].host;
+    }
+    dim3 g = divergence_grid(P.d[0]);
+    const int zb = (int)g.z;
+    g.z = (unsigned)(zb * m);
+    k_divergence<N><<<g, 128, 0, s>>>(P, O, cfl ? 1 : 0, zb);
+    count_launch();
+  });
+}
+
+void launch_cn_factors(const NSDev* const* Ds, const CNFactorSet* set, int n, int slot0, int nslots, cudaStream_t s) {
+  by_members(n, [&](auto N, int b, int m) {
+    const auto P = many<N>(Ds, b, m);
+    CNFactorJobs<N> J{};
+    for (int q = 0; q < m; ++q) {
+      J.dst[q] = set[b + q].dst;
+      for (int r = 0; r < 3; ++r) J.rkdt[q][r] = set[b + q].rkdt[r];
+    }
+    for (int v = 0; v < 5; ++v)
+      for (int f = 0; f < 2; ++f) {
+        J.type[v][f] = set[b].type[v][f];
+        J.val[v][f] = set[b].val[v][f];
+      }
+    const size_t sm = 3 * (size_t)(P.d[0].nz + 2) * sizeof(double);
+    set_smem_limit_once((const void*)k_cn_factors<N>, 64 * 1024);
+    k_cn_factors<N><<<dim3(5, (unsigned)nslots, (unsigned)m), 128, sm, s>>>(P, J, slot0);
+    count_launch();
+  });
 }
 
 }  // namespace anel

@@ -40,7 +40,6 @@ NSSolver::~NSSolver() {
   cudaFree(d_part_);
   for (auto& h : hist_)
     for (double* a : h) cudaFree(a);
-  if (h_cn_) cudaFreeHost(h_cn_);
   if (h_red_) cudaFreeHost(h_red_);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
@@ -201,9 +200,11 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
   ANEL_CUDA_TRY(cudaMalloc(&d_prof_, 2 * (size_t)Z * sizeof(double)));
   const size_t ncn = 3 * 5 * 9 * (size_t)Z;
   ANEL_CUDA_TRY(cudaMalloc(&d_cn_, ncn * sizeof(double)));
-  ANEL_CUDA_TRY(cudaHostAlloc(&h_cn_, ncn * sizeof(double), cudaHostAllocMapped));
-  ANEL_CUDA_TRY(cudaMalloc(&d_red_, 4 * sizeof(unsigned long long)));
-  ANEL_CUDA_TRY(cudaHostAlloc(&h_red_, 4 * sizeof(double), cudaHostAllocMapped));
+  // [0] the CFL maximum of k_cfl_max, [1] arrival counter and [4..7] results
+  // of the divergence pass
+  ANEL_CUDA_TRY(cudaMalloc(&d_red_, 8 * sizeof(unsigned long long)));
+  ANEL_CUDA_TRY(cudaMemset(d_red_, 0, 8 * sizeof(unsigned long long)));
+  ANEL_CUDA_TRY(cudaHostAlloc(&h_red_, 8 * sizeof(double), cudaHostAllocMapped));
   // device view
   D_.nx = nx_;
   D_.ny = ny_;
@@ -322,7 +323,9 @@ int NSSolver::tune_cn() {
   };
   int st = pick("k_cn_column", kCNVariants, "ANEL_CN_VARIANT", [&](int q) {
     CNSet set[5];
-    launch_cn(D_, set, cn_set(0, set), 1.0 / 3.0, 1e-3, q, stream_);
+    const NSDev* d = &D_;
+    const double rkdt = 1e-3;
+    launch_cn(&d, set, cn_set(0, set), &rkdt, 1, 1.0 / 3.0, q, stream_);
   }, &cnvar_);
   if (st == ANEL_OK && D_.vles)
     st = pick("k_cn_column_les", kCNLesVariants, "ANEL_CN_LES_VARIANT", [&](int q) {
@@ -407,107 +410,38 @@ ZRule NSSolver::zrule(int vt) const {
   return R;
 }
 
-// Column-independent factors of the CN system of each variable for one
-// rkdt (var_advance_CN_PL, NSsolver.F90:3102-3296), then the elimination
-// of the Thomas routine (mg_relax.F90:563-568) applied to them.
+// The CN factors of slots slot0 .. slot0 + n - 1 for their rkdt (cn_rkdt_):
+// what launch_cn_factors needs of this member.
+CNFactorSet NSSolver::cn_factor_set() const {
+  CNFactorSet c{};
+  c.dst = d_cn_;
+  for (int q = 0; q < 3; ++q) c.rkdt[q] = cn_rkdt_[q];
+  for (int vi = 0; vi < 5; ++vi)
+    for (int f = 0; f < 2; ++f) {
+      c.type[vi][f] = prm_.tb[2][f][kVarCode[vi] - 1];
+      c.val[vi][f] = prm_.vb[2][f][kVarCode[vi] - 1];
+    }
+  return c;
+}
+
 int NSSolver::cn_factors(int slot, double rkdt, cudaStream_t s) {
   if (cn_rkdt_[slot] == rkdt) return ANEL_OK;
-  // the pinned staging slot may still feed an earlier asynchronous copy
-  ANEL_CUDA_TRY(cudaStreamSynchronize(s));
-  const int Z = nz_ + 2, n = Z, sz = 2, ez = nz_ + 1;
-  const double H = 0.5;
-  auto R = [&](int k) { return rz_[k - 1]; };
-  auto rdze = [&](int k) { return m_[2][4][k - 1]; };
-  auto rdzc = [&](int k) { return m_[2][5][k - 1]; };
-  auto dze = [&](int k) { return m_[2][2][k - 1]; };
-  auto dzc = [&](int k) { return m_[2][3][k - 1]; };
-  for (int vi = 0; vi < 5; ++vi) {
-    const int var = kVarCode[vi];
-    double* base = h_cn_ + ((size_t)(slot * 5 + vi) * 9) * Z;
-    double *ap = base, *bp = base + Z, *c = base + 2 * Z, *t1a = base + 3 * Z, *t2a = base + 4 * Z,
-           *rb = base + 5 * Z, *isbc = base + 6 * Z, *suba = base + 7 * Z, *diaga = base + 8 * Z;
-    std::vector<double> sub(n, 0.0), diag(n, 0.0), sup(n, 0.0);
-    for (int q = 0; q < n; ++q) {
-      t1a[q] = t2a[q] = rb[q] = isbc[q] = 0.0;
-    }
-    for (int k = sz; k <= ez; ++k) {
-      double t1, t2;
-      if (var != 3) {
-        const double ra1 = H * (R(k + 1) + R(k));
-        const double ra2 = H * (R(k) + R(k - 1));
-        if (var == 1 || var == 2) {
-          t1 = (rRe_ + 0.0) * ra1 / R(k);
-          t2 = (rRe_ + 0.0) * ra2 / R(k);
-        } else if (var == 5) {
-          t1 = (rRe_ * rPr_ + 0.0) * ra1 / R(k);
-          t2 = (rRe_ * rPr_ + 0.0) * ra2 / R(k);
-        } else {
-          t1 = rRe_ * rSc_ + 0.0;
-          t2 = rRe_ * rSc_ + 0.0;
-        }
-        sub[k - 1] = -0.5 * rkdt * t1 * rdze(k - 1) * rdzc(k);
-        sup[k - 1] = -0.5 * rkdt * t2 * rdze(k) * rdzc(k);
-        diag[k - 1] = 1.0 + 0.5 * rkdt * (t1 * rdze(k - 1) + t2 * rdze(k)) * rdzc(k);
-      } else {
-        t1 = (rRe_ + 0.0) * R(k) / (H * (R(k + 1) + R(k)));
-        t2 = (rRe_ + 0.0) * R(k + 1) / (H * (R(k + 1) + R(k)));
-        sub[k - 1] = -0.5 * rkdt * t1 * rdze(k) * rdzc(k);
-        sup[k - 1] = -0.5 * rkdt * t2 * rdze(k) * rdzc(k + 1);
-        diag[k - 1] = 1.0 + 0.5 * rkdt * (t1 * rdzc(k) + t2 * rdzc(k + 1)) * rdze(k);
-      }
-      t1a[k - 1] = t1;
-      t2a[k - 1] = t2;
-    }
-    // wall rows (NSsolver.F90:3297-3429)
-    const int tbmin = prm_.tb[2][0][var - 1], tbmax = prm_.tb[2][1][var - 1];
-    const double vbmin = prm_.vb[2][0][var - 1], vbmax = prm_.vb[2][1][var - 1];
-    auto set = [&](int k, double a, double b, double cc, double d) {
-      sub[k - 1] = a;
-      diag[k - 1] = b;
-      sup[k - 1] = cc;
-      rb[k - 1] = d;
-      isbc[k - 1] = 1.0;
-    };
-    if (tbmin == 1) set(sz - 1, 0.0, 1.0, 0.0, vbmin);
-    else if (tbmin == 2) {
-      if (var == 3) set(sz - 1, 0.0, -1.0, 1.0, dzc(sz - 1) * vbmin);
-      else if (var == 5 || var == 8) {
-        set(sz - 1, 0.0, -1.0, 1.0, dze(sz - 1) * vbmin);
-        set(sz, 0.0, -1.0, 1.0, dze(sz) * vbmin);
-      } else set(sz - 1, 0.0, -1.0, 1.0, dze(sz - 1) * vbmin);
-    } else if (tbmin == 6) set(sz - 1, 0.0, 1.0, 1.0, 2.0 * vbmin);
-    if (tbmax == 1) set(ez + 1, 0.0, 1.0, 0.0, vbmax);
-    else if (tbmax == 2) {
-      if (var == 3) set(ez + 1, -1.0, 1.0, 0.0, dzc(ez + 1) * vbmax);
-      else if (var == 5 || var == 8) {
-        set(ez + 1, -1.0, 1.0, 0.0, dze(ez + 1) * vbmax);
-        set(ez, -1.0, 1.0, 0.0, dze(ez) * vbmax);
-      } else set(ez + 1, -1.0, 1.0, 0.0, dze(ez + 1) * vbmax);
-    } else if (tbmax == 6) set(ez + 1, 1.0, 1.0, 0.0, 2.0 * vbmax);
-    else if (tbmax == 7) {
-      set(ez + 1, 0.0, 1.0, 0.0, 0.0);
-      set(ez, 0.0, 1.0, 0.0, 0.0);
-    }
-    // elimination (a, b overwritten, c untouched)
-    std::vector<double> a(sub), b(diag);
-    for (int j = 1; j <= n - 1; ++j) {
-      a[j] = -a[j] / b[j - 1];
-      b[j] = b[j] + a[j] * sup[j - 1];
-    }
-    for (int q = 0; q < n; ++q) {
-      ap[q] = (q == 0) ? 0.0 : a[q];
-      bp[q] = b[q];
-      c[q] = sup[q];
-      suba[q] = sub[q];
-      diaga[q] = diag[q];
-    }
-  }
-  double* dst = d_cn_ + (size_t)slot * 5 * 9 * Z;
-  // by a kernel from the mapped staging slot: a copy-engine upload would
-  // queue behind large uploads other streams have in flight
-  copy_words(h_cn_ + (size_t)slot * 5 * 9 * Z, dst, 5 * 9 * (int64_t)Z, s);
   cn_rkdt_[slot] = rkdt;
+  const NSDev* d = &D_;
+  const CNFactorSet c = cn_factor_set();
+  launch_cn_factors(&d, &c, 1, slot, 1, s);
   return ANEL_OK;
+}
+
+// A step's three factor sets; false when they are there already.
+bool NSSolver::cn_step_slots(double delt) {
+  const double dtr[3] = {1.0 / 3.0 * delt, 5.0 / 12.0 * delt, 1.0 / 4.0 * delt};
+  bool make = false;
+  for (int q = 0; q < 3; ++q) {
+    make = make || cn_rkdt_[q] != dtr[q];
+    cn_rkdt_[q] = dtr[q];
+  }
+  return make;
 }
 
 CNFacHost NSSolver::fac(int slot, int vi) const {
@@ -530,7 +464,7 @@ int NSSolver::set_fields(const anel_fields* f, int mem, cudaStream_t s) {
     if (!src[q] || !d_fields_[q]) continue;  // LES fields exist only with a subgrid model
     ANEL_CUDA_TRY(cudaMemcpyAsync(d_fields_[q], src[q], G_ * sizeof(double), kind, s));
     if (q == 6 || q == 7) density = true;
-    if (q >= 8 && q <= 12) temps_clean_ = false;
+    if (q >= 8 && q <= 13) temps_clean_ = false;
   }
   if (density) {
     // profiles of r and densityBG: both must be functions of z only
@@ -602,16 +536,18 @@ int NSSolver::substep_pre(double a1, double a2, double a3, double dt_rk, double 
     if (st != ANEL_OK) return st;
   }
   D_.g = gnow_;
-  launch_rhs_accum(D_, a1, a2, dt, q_zero && a1 == 0.0, s);
+  const NSDev* d = &D_;
+  launch_rhs_accum(&d, &dt, 1, a1, a2, q_zero && a1 == 0.0, s);
   // var_advance_CN_PL: with Vmodel = SSM every variable gets the eddy
   // terms (the LES block is gated on Vmodel, NSsolver.F90:3160-3190)
   if (D_.vles) {
     cn_solve_les(slot, a3, dt_rk, cnlesvar_, s);
   } else {
     CNSet set[5];
-    launch_cn(D_, set, cn_set(slot, set), a3, dt_rk, cnvar_, s);
+    const int ns = cn_set(slot, set);
+    launch_cn(&d, set, ns, &dt_rk, 1, a3, cnvar_, s);
   }
-  launch_psource(D_, dt_rk, s);
+  launch_psource(&d, &dt_rk, 1, s);
   if (prm_.pguess && cur_sub_ >= 0 && nhist_[cur_sub_] >= 2) {
     const int q = cur_sub_;
     launch_extrap(D_, D_.p, hist_[q][last_[q]], hist_[q][last_[q] ^ 1], s);
@@ -633,7 +569,7 @@ int NSSolver::substep_pre(double a1, double a2, double a3, double dt_rk, double 
   return ANEL_OK;
 }
 
-int NSSolver::substep_post(const anel_mg_report& rep, cudaStream_t s, int* iters, double* relmax) {
+int NSSolver::substep_post(const anel_mg_report& rep, cudaStream_t s, int* iters, double* relmax, bool pgrad) {
   if (io_last_sub_ && io_out_ && io_out_->p) {  // p is final: copy it out during Pgrad
     ANEL_CUDA_TRY(cudaEventRecord(io_ev_[2], s));
     ANEL_CUDA_TRY(cudaStreamWaitEvent(io_stream_, io_ev_[2], 0));
@@ -651,7 +587,8 @@ int NSSolver::substep_post(const anel_mg_report& rep, cudaStream_t s, int* iters
     hist = hist_[q][last_[q]];
     nhist_[q] = nhist_[q] < 2 ? nhist_[q] + 1 : 2;
   }
-  launch_pgrad(D_, pend_dtrk_, zrule(NV_U), zrule(NV_V), zrule(NV_W), s, hist);
+  const NSDev* d = &D_;
+  if (pgrad) launch_pgrad(&d, &pend_dtrk_, 1, zrule(NV_U), zrule(NV_V), zrule(NV_W), s, hist);
   fields_changed();
   if (iters) *iters = rep.iter;
   if (relmax) *relmax = rep.relmax;
@@ -794,10 +731,12 @@ int NSSolver::les_coeffs(cudaStream_t s) {
 // time step from it (take)
 void NSSolver::calcdt_issue(cudaStream_t s) {
   if (cfl_ready_) {
-    // the previous step's divergence pass took it from these fields
-    copy_words(d_red_ + 2, h_red_, 1, s);
+    // the previous step's divergence pass took it from these fields and
+    // wrote it to h_red_ too
+    cfl_word_ = 7;
     cfl_ready_ = false;
   } else {
+    cfl_word_ = 0;
     cudaMemsetAsync(d_red_, 0, sizeof(unsigned long long), s);
     launch_cfl_max(D_, d_red_, s);
     copy_words(d_red_, h_red_, 1, s);
@@ -805,7 +744,7 @@ void NSSolver::calcdt_issue(cudaStream_t s) {
 }
 
 double NSSolver::calcdt_take() const {
-  double dt = prm_.cfl / h_red_[0];
+  double dt = prm_.cfl / h_red_[cfl_word_];
   if (dt >= prm_.dtmax) dt = prm_.dtmax;
   return dt;
 }
@@ -839,7 +778,14 @@ static const double kA3[3] = {1.0 / 3.0, 15.0 / 16.0, 8.0 / 15.0};
 int NSSolver::step_begin(cudaStream_t s, double* delt_out) {
   step_begin_issue(s);
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
-  return step_begin_finish(s, delt_out);
+  const int st = step_begin_finish(s, delt_out);
+  if (st != ANEL_OK) return st;
+  if (cn_step_slots(*delt_out)) {
+    const NSDev* d = &D_;
+    const CNFactorSet c = cn_factor_set();
+    launch_cn_factors(&d, &c, 1, 0, 3, s);
+  }
+  return ANEL_OK;
 }
 
 void NSSolver::step_begin_issue(cudaStream_t s) {
@@ -847,10 +793,10 @@ void NSSolver::step_begin_issue(cudaStream_t s) {
   // q_w, q_rho, q_s are written, never read, by the first sub-step
   // (a1 = 0) on every interior cell, and no kernel writes their ghost
   // cells, so once zeroed they need no zeroing again until set_fields,
-  // reset or a scratch use touches them (temps_clean_); the Poisson
-  // right-hand side is zeroed every step.
+  // reset or a scratch use touches them (temps_clean_); so does Psource
+  // with the Poisson right-hand side.
   for (int q : {8, 9, 10, 11, 12, 13})
-    if (q == 13 || !temps_clean_) cudaMemsetAsync(d_fields_[q], 0, G_ * sizeof(double), s);
+    if (!temps_clean_) cudaMemsetAsync(d_fields_[q], 0, G_ * sizeof(double), s);
   temps_clean_ = true;
   calcdt_issue(s);
 }
@@ -882,7 +828,7 @@ int NSSolver::step_begin_finish(cudaStream_t s, double* delt_out) {
 }
 
 // End of a step: the clock (NSsolver.F90:272-274) and the diagnostics.
-int NSSolver::step_end(double delt, cudaStream_t s, anel_step_report* r) {
+int NSSolver::step_end(double delt, cudaStream_t s, anel_step_report* r, bool div) {
   told_ = time_;  // told = time; time = time + delt
   time_ = time_ + delt;
   if (diag_on_) {
@@ -901,9 +847,12 @@ int NSSolver::step_end(double delt, cudaStream_t s, anel_step_report* r) {
   r->dt = delt;
   r->time = time_;
   nstep_ += 1;
-  // divergence of the step's result and the next step's CFL maximum
-  const int st = divergence_pass(s, true);
-  if (st != ANEL_OK) return st;
+  // divergence of the step's result and the next step's CFL maximum (a
+  // cohort takes its members' together)
+  if (div) {
+    const int st = divergence_pass(s, true);
+    if (st != ANEL_OK) return st;
+  }
   cfl_ready_ = div_ready_ = true;
   return ANEL_OK;
 }
@@ -1005,17 +954,64 @@ int NSSolver::step_cohort(NSSolver* const* ms, int n, int nsteps, MGSolver* bmg,
     phis[b] = m->D_.p;
     rhss[b] = m->D_.psrc;
   }
+  // Members that differ in physics, time step and state only take every
+  // stepper kernel in one launch (the values are those of the launches they
+  // would have of their own); subgrid models and the extrapolated guess keep
+  // their members' own launches.
+  const NSSolver* m0 = ms[0];
+  bool together = true;
+  for (int b = 0; b < n; ++b) {
+    const NSSolver* m = ms[b];
+    together = together && !m->les_any_ && !m->prm_.pguess && m->D_.unit_r == m0->D_.unit_r &&
+               m->prm_.scal1_on == m0->prm_.scal1_on && m->prm_.ew == m0->prm_.ew && m->cnvar_ == m0->cnvar_ &&
+               std::memcmp(m->prm_.tb, m0->prm_.tb, sizeof(m0->prm_.tb)) == 0 &&
+               std::memcmp(m->prm_.vb, m0->prm_.vb, sizeof(m0->prm_.vb)) == 0;
+    const int st = ms[b]->divergence_prepare();
+    if (st != ANEL_OK) return st;
+  }
+  std::vector<const NSDev*> devs(n);
+  std::vector<DivSet> divs(n);
+  std::vector<CNFactorSet> facs(n);
+  std::vector<CNSet> sets((size_t)5 * n);
+  std::vector<double> dtr(n);
+  for (int b = 0; b < n; ++b) {
+    devs[b] = &ms[b]->D_;
+    divs[b] = ms[b]->divergence_set();
+  }
   ANEL_CUDA_TRY(cudaEventRecord(ms[0]->ev0_, s));
   for (int step = 0; step < nsteps; ++step) {
     // every member's time step with one synchronisation
     for (int b = 0; b < n; ++b) ms[b]->step_begin_issue(s);
     ANEL_CUDA_TRY(cudaStreamSynchronize(s));
+    bool make = false;
     for (int b = 0; b < n; ++b) {
       const int st = ms[b]->step_begin_finish(s, &delt[b]);
       if (st != ANEL_OK) return st;
+      make = ms[b]->cn_step_slots(delt[b]) || make;
+      facs[b] = ms[b]->cn_factor_set();
+    }
+    if (make) {
+      if (together) launch_cn_factors(devs.data(), facs.data(), n, 0, 3, s);
+      else
+        for (int b = 0; b < n; ++b) launch_cn_factors(&devs[b], &facs[b], 1, 0, 3, s);
     }
     for (int q = 0; q < 3; ++q) {
-      for (int b = 0; b < n; ++b) {
+      if (together) {
+        int ns = 0;
+        for (int b = 0; b < n; ++b) {
+          NSSolver* m = ms[b];
+          m->D_.g = m->gnow_;
+          const double DTR[3] = {1.0 / 3.0 * delt[b], 5.0 / 12.0 * delt[b], 1.0 / 4.0 * delt[b]};
+          m->pend_dtrk_ = dtr[b] = DTR[q];
+          ns = m->cn_set(q, sets.data() + (size_t)b * ns);
+        }
+        launch_rhs_accum(devs.data(), delt.data(), n, kA1[q], 1.0, kA1[q] == 0.0, s);
+        launch_cn(devs.data(), sets.data(), ns, dtr.data(), n, kA3[q], m0->cnvar_, s);
+        launch_psource(devs.data(), dtr.data(), n, s);
+        const int st = check_launch("cohort sub-step");
+        if (st != ANEL_OK) return st;
+      }
+      for (int b = 0; b < n && !together; ++b) {
         NSSolver* m = ms[b];
         if (m->D_.vles && m->nstep_ > m->prm_.les_start) launch_sgs(m->D_, m->zrule(NV_CFLUC), s);
         const double DTR[3] = {1.0 / 3.0 * delt[b], 5.0 / 12.0 * delt[b], 1.0 / 4.0 * delt[b]};
@@ -1025,18 +1021,21 @@ int NSSolver::step_cohort(NSSolver* const* ms, int n, int nsteps, MGSolver* bmg,
       }
       const int sb = bmg->solve_batch(n, phis.data(), rhss.data(), s, mrep.data());
       if (sb != ANEL_OK && sb != ANEL_ERR_NOCONV) return sb;
+      if (together)
+        launch_pgrad(devs.data(), dtr.data(), n, m0->zrule(NV_U), m0->zrule(NV_V), m0->zrule(NV_W), s);
       for (int b = 0; b < n; ++b) {
         mrep[b].ms /= n;  // the batch's device time, shared out
-        const int st = ms[b]->substep_post(mrep[b], s, &r[b].mg_iter[q], &r[b].mg_relmax[q]);
+        const int st = ms[b]->substep_post(mrep[b], s, &r[b].mg_iter[q], &r[b].mg_relmax[q], !together);
         ms[b]->cur_sub_ = -1;
         if (st != ANEL_OK) return st;
         ms[b]->clip_scalars(s);
       }
     }
     for (int b = 0; b < n; ++b) {
-      const int st = ms[b]->step_end(delt[b], s, &r[b]);
+      const int st = ms[b]->step_end(delt[b], s, &r[b], false);
       if (st != ANEL_OK) return st;
     }
+    launch_divergence(devs.data(), divs.data(), n, true, s);
   }
   ANEL_CUDA_TRY(cudaEventRecord(ms[0]->ev1_, s));
   ANEL_CUDA_TRY(cudaEventSynchronize(ms[0]->ev1_));
@@ -1044,7 +1043,6 @@ int NSSolver::step_cohort(NSSolver* const* ms, int n, int nsteps, MGSolver* bmg,
   cudaEventElapsedTime(&tms, ms[0]->ev0_, ms[0]->ev1_);
   // the divergence of every member's last step (step_end's passes), with
   // one synchronisation
-  for (int b = 0; b < n; ++b) ms[b]->divergence_issue(s);
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
   for (int b = 0; b < n; ++b) {
     NSSolver* m = ms[b];
@@ -1259,47 +1257,47 @@ int NSSolver::project(cudaStream_t s, int* iters, double* relmax) {
   launch_ghost_field(D_, D_.u, zrule(NV_U), s);
   launch_ghost_field(D_, D_.v, zrule(NV_V), s);
   launch_ghost_field(D_, D_.w, zrule(NV_W), s);
-  launch_psource(D_, 1.0, s);
+  const NSDev* d = &D_;
+  const double one = 1.0;
+  launch_psource(&d, &one, 1, s);
   anel_mg_report rep{};
   const int st = mg_->solve_device(D_.p, D_.psrc, s, &rep);
   if (st != ANEL_OK && st != ANEL_ERR_NOCONV) return st;
-  launch_pgrad(D_, 1.0, zrule(NV_U), zrule(NV_V), zrule(NV_W), s);
+  launch_pgrad(&d, &one, 1, zrule(NV_U), zrule(NV_V), zrule(NV_W), s);
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
   if (iters) *iters = rep.iter;
   if (relmax) *relmax = rep.relmax;
   return check_launch("project");
 }
 
-// divergence (Routines.F90:54-183) of the current fields into device
-// memory: max |div| in d_red_[1], the volume-weighted sums after the fold;
-// with_cfl also the CFL maximum in d_red_[2]
-int NSSolver::divergence_pass(cudaStream_t s, bool with_cfl) {
-  const int64_t nb = divergence_blocks(D_);
-  // partial pairs, fold scratch, the two sums
-  if (!d_part_)
-    ANEL_CUDA_TRY(cudaMalloc(&d_part_, (2 * nb + fold_scratch_doubles() + 2) * sizeof(double)));
-  double* sums = d_part_ + 2 * nb + fold_scratch_doubles();
-  ANEL_CUDA_TRY(cudaMemsetAsync(d_red_ + 1, 0, (with_cfl ? 2 : 1) * sizeof(unsigned long long), s));
-  launch_divergence(D_, d_red_ + 1, d_part_, s, with_cfl ? d_red_ + 2 : nullptr);
-  launch_fold_pairs(d_part_, nb, d_part_ + 2 * nb, sums, s);
+// divergence (Routines.F90:54-183) of the current fields; with_cfl also the
+// CFL maximum: results in d_red_[4..7] and, once the stream has been waited
+// for, in h_red_[4..7]
+int NSSolver::divergence_prepare() {
+  if (!d_part_) ANEL_CUDA_TRY(cudaMalloc(&d_part_, divergence_part_doubles(D_) * sizeof(double)));
   return ANEL_OK;
 }
 
-void NSSolver::divergence_issue(cudaStream_t s) {
-  const int64_t nb = divergence_blocks(D_);
-  const double* sums = d_part_ + 2 * nb + fold_scratch_doubles();
-  copy_words(d_red_ + 1, h_red_ + 1, 1, s);
-  copy_words(sums, h_red_ + 2, 2, s);
+DivSet NSSolver::divergence_set() const {
+  return DivSet{d_part_, reinterpret_cast<unsigned*>(d_red_ + 1), reinterpret_cast<double*>(d_red_ + 4), h_red_ + 4};
+}
+
+int NSSolver::divergence_pass(cudaStream_t s, bool with_cfl) {
+  const int st = divergence_prepare();
+  if (st != ANEL_OK) return st;
+  const NSDev* d = &D_;
+  const DivSet set = divergence_set();
+  launch_divergence(&d, &set, 1, with_cfl, s);
+  return ANEL_OK;
 }
 
 int NSSolver::divergence_take(double* out) {
-  out[0] = h_red_[2] / h_red_[3];
-  out[1] = h_red_[1];
+  out[0] = h_red_[4] / h_red_[5];
+  out[1] = h_red_[6];
   return check_launch("divergence");
 }
 
 int NSSolver::divergence_read(cudaStream_t s, double* out) {
-  divergence_issue(s);
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
   return divergence_take(out);
 }
@@ -1309,7 +1307,7 @@ int NSSolver::divergence(cudaStream_t s, double* out) {
   if (!s) s = stream_;
   const int st = divergence_pass(s, false);
   if (st != ANEL_OK) return st;
-  div_ready_ = false;  // d_red_[1] and the sums now hold this pass
+  cfl_ready_ = div_ready_ = false;  // the results now hold this pass
   return divergence_read(s, out);
 }
 

@@ -86,13 +86,13 @@ class NSSolver {
   void calcdt_issue(cudaStream_t s);
   double calcdt_take() const;
   int substep_pre(double a1, double a2, double a3, double dt_rk, double dt, cudaStream_t s, bool q_zero);
-  int substep_post(const anel_mg_report& rep, cudaStream_t s, int* iters, double* relmax);
-  int step_end(double delt, cudaStream_t s, anel_step_report* r);
+  int substep_post(const anel_mg_report& rep, cudaStream_t s, int* iters, double* relmax, bool pgrad = true);
+  int step_end(double delt, cudaStream_t s, anel_step_report* r, bool div = true);
   int step_finish(cudaStream_t s, int64_t launches0, anel_step_report* r);
   void clip_scalars(cudaStream_t s);
   double pend_dtrk_ = 0.0;  // the sub-step between substep_pre and substep_post
   // step_end's divergence pass also takes the CFL maximum of the fields it
-  // leaves (d_red_[2]) and its divergence results stay on the device:
+  // leaves (h_red_[7]) and keeps its divergence results (h_red_[4..6]):
   // cfl_ready_ lets the next calcdt use that maximum, div_ready_ lets
   // step_finish report those results, without another read of u, v, w.
   // Every call that changes u, v or w afterwards clears both.
@@ -108,7 +108,11 @@ class NSSolver {
   int ensure_hist();
   int divergence_pass(cudaStream_t s, bool with_cfl);
   int divergence_read(cudaStream_t s, double* out);
-  void divergence_issue(cudaStream_t s);
+  int divergence_prepare();
+  DivSet divergence_set() const;
+  CNFactorSet cn_factor_set() const;
+  bool cn_step_slots(double delt);
+  int cfl_word_ = 0;  // of h_red_: where calcdt_take finds the CFL maximum
   int divergence_take(double* out);
   int les_coeffs(cudaStream_t s);
 
@@ -180,7 +184,6 @@ class NSSolver {
   bool les_any_ = false;            // a subgrid model is on: nuT/kappaT/nappaT exist
   bool les_coeffs_done_ = false;
   double* d_cn_ = nullptr;          // CN factors: 3 slots x 5 vars x 9 arrays x (nz+2)
-  double* h_cn_ = nullptr;          // pinned staging of the same
   double cn_rkdt_[3] = {-1, -1, -1};
   int cnvar_ = 0;     // launch variant of the DNS column solve (tune_cn)
   int cnlesvar_ = 0;  // and of the LES column solve
