@@ -9,47 +9,69 @@
 
 namespace anel {
 
-__device__ __forceinline__ double spec_block_sum(double v, double* sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += sh[q];
-  return s;
-}
+// The end of a norm pass in two halves.  spec_norm_arrive: the block's sums
+// to its slot of the member's partials and its arrival; spec_norm_finish:
+// the member's last block to arrive adds all partials in slot order (fixed
+// for a launch shape, so the sums are deterministic) and sets the member's
+// state.  Work between the two hides the arrival's round trip.  corrected:
+// the pass follows a correction.
+struct SpecNorm {
+  double sh[2][8];
+  int last;
+};
 
-// The end of a norm pass: the block's sums to its slot of the member's
-// partials; the member's last block to arrive adds all of them in slot
-// order (fixed for a launch shape, so the sums are deterministic) and sets
-// the member's state.  corrected: the pass follows a correction.
-__device__ __forceinline__ void spec_norm_finish(const SpecDev& D, int b, int slot, int nslots, double rr, double ff,
-                                                 bool corrected) {
-  __shared__ double sh[32];
-  __shared__ int last;
-  const double s1 = spec_block_sum(rr, sh), s2 = spec_block_sum(ff, sh);
-  double* part = D.part + (int64_t)b * D.pstride;
-  if (threadIdx.x == 0) {
-    part[2 * slot] = s1;
-    part[2 * slot + 1] = s2;
-    __threadfence();
-    last = atomicAdd(D.count + b, 1u) == (unsigned)nslots - 1;
+__device__ __forceinline__ void spec_norm_arrive(SpecNorm& N, const SpecDev& D, int b, int slot, int nslots, double rr,
+                                                 double ff) {
+  for (int o = 16; o > 0; o >>= 1) {
+    rr += __shfl_xor_sync(0xffffffffu, rr, o);
+    ff += __shfl_xor_sync(0xffffffffu, ff, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    N.sh[0][threadIdx.x >> 5] = rr;
+    N.sh[1][threadIdx.x >> 5] = ff;
   }
   __syncthreads();
-  if (!last) return;
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
+      rr += N.sh[0][q];
+      ff += N.sh[1][q];
+    }
+    double* part = D.part + (int64_t)b * D.pstride;
+    part[2 * slot] = rr;
+    part[2 * slot + 1] = ff;
+    __threadfence();
+    N.last = atomicAdd(D.count + b, 1u) == (unsigned)nslots - 1;
+  }
+}
+
+__device__ __forceinline__ void spec_norm_finish(SpecNorm& N, const SpecDev& D, int b, int nslots, bool corrected) {
+  __syncthreads();
+  if (!N.last) return;
   __threadfence();
+  const double* part = D.part + (int64_t)b * D.pstride;
   double a = 0.0, c = 0.0;
   for (int q = threadIdx.x; q < nslots; q += blockDim.x) {
     a += __ldcg(part + 2 * q);
     c += __ldcg(part + 2 * q + 1);
   }
-  const double n1 = spec_block_sum(a, sh), n2 = spec_block_sum(c, sh);
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    N.sh[0][threadIdx.x >> 5] = a;
+    N.sh[1][threadIdx.x >> 5] = c;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
+    for (int q = 1; q < (int)(blockDim.x >> 5); ++q) {
+      a += N.sh[0][q];
+      c += N.sh[1][q];
+    }
     D.count[b] = 0;
     SpecState s = D.st[b];
-    s.ff = n2;
-    s.rel = n2 > 0.0 ? sqrt(n1 / n2) : sqrt(n1);
+    s.ff = c;
+    s.rel = c > 0.0 ? sqrt(a / c) : sqrt(a);
     s.iter = corrected ? s.iter + 1 : 0;
     s.conv = s.rel <= D.tol;
     s.act = !s.conv && s.iter < D.maxcy;
@@ -97,10 +119,12 @@ __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
   auto at = [&](int q, int i) { return q * row + spec_pad(i); };
   auto none = [](int, int, double2) {};
   double2* z = spec_fft<0, true>(D.px, nb, xsm, xsm + D.pairs * row, in, none, at);
+  __shared__ SpecNorm norm;
+  if (test) spec_norm_arrive(norm, D, b, blockIdx.x + gridDim.x * blockIdx.y, gridDim.x * gridDim.y, rr, ff);
   const int h = D.nxh;
   double2* w = D.work + (int64_t)b * D.nz * D.nu + (int64_t)(k - 2) * D.nu + (int64_t)(2 * pair0) * h;
   for (int it = threadIdx.x; it < nb * h; it += blockDim.x) {
-    const int q = it / h, c = it - q * h;
+    const int q = spec_div(it, D.dnh), c = it - q * h;
     const double2 u = z[at(q, c)];
     double2 A, B;
     if (c == 0) {
@@ -115,12 +139,12 @@ __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
     w[(int64_t)(2 * q) * h + c] = A;
     w[(int64_t)(2 * q + 1) * h + c] = B;
   }
-  if (test) spec_norm_finish(D, b, blockIdx.x + gridDim.x * blockIdx.y, gridDim.x * gridDim.y, rr, ff, false);
+  if (test) spec_norm_finish(norm, D, b, gridDim.x * gridDim.y, false);
 }
 
 // Inverse x transform of row pairs and phi += e.  The inverse transform is
 // the forward one with real and imaginary parts exchanged before and after.
-__global__ void __launch_bounds__(256, 2) k_spec_update(SpecDev D) {
+__global__ void __launch_bounds__(256, 3) k_spec_update(SpecDev D) {
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!D.st[b].act) return;
@@ -141,18 +165,40 @@ __global__ void __launch_bounds__(256, 2) k_spec_update(SpecDev D) {
     else z = make_double2(A.x - B.y, A.y + B.x);
     return make_double2(z.y, z.x);
   };
-  auto out = [&](int q, int i, double2 v) {
-    const int64_t c = base + (int64_t)(2 * q) * D.X + i;
-    phi[c] += D.scale * v.y;
-    phi[c + D.X] += D.scale * v.x;
-  };
+  auto none = [](int, int, double2) {};
   auto at = [&](int q, int i) { return q * row + spec_pad(i); };
-  spec_fft<0, false>(D.px, nb, xsm, xsm + D.pairs * row, in, out, at);
+  const double2* z = spec_fft<0, true>(D.px, nb, xsm, xsm + D.pairs * row, in, none, at);
+  // a thread's loads of phi before its stores: as a last-stage accessor
+  // each phi += e waited for the one before it (833 us at 512x256x512)
+  constexpr int U = 4;
+  const int total = nb * n;
+  for (int it = threadIdx.x; it < total; it += U * blockDim.x) {
+    double p0[U], p1[U];
+    int64_t c[U];
+    int o[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = it + u * blockDim.x;
+      if (t >= total) break;
+      const int q = spec_div(t, D.dnx), i = t - q * n;
+      c[u] = base + (int64_t)(2 * q) * D.X + i;
+      o[u] = at(q, i);
+      p0[u] = phi[c[u]];
+      p1[u] = phi[c[u] + D.X];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (it + u * (int)blockDim.x >= total) break;
+      const double2 v = z[o[u]];
+      phi[c[u]] = p0[u] + D.scale * v.y;
+      phi[c[u] + D.X] = p1[u] + D.scale * v.x;
+    }
+  }
 }
 
 // y transform of W columns of a plane, in place.
 template <bool kInv, int W>
-__global__ void __launch_bounds__(256, 2) k_spec_y(SpecDev D) {
+__global__ void __launch_bounds__(256, 3) k_spec_y(SpecDev D) {
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!D.st[b].act) return;
@@ -195,6 +241,18 @@ __global__ void __launch_bounds__(256, 2) k_spec_y(SpecDev D) {
       }
     }
   }
+}
+
+// 1 / x for a normal x: the hardware's approximation (20 bits) and two
+// Newton steps y <- y + y (1 - x y), each doubling its correct bits, so
+// within a unit in the last place.  A division branches to its special
+// cases, which a chain of them waits for.
+__device__ __forceinline__ double spec_rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+#pragma unroll
+  for (int q = 0; q < 2; ++q) y = fma(y, fma(-x, y, 1.0), y);
+  return y;
 }
 
 // The z-systems of eight modes at a time.  Thread (mode w, segment g) holds
@@ -258,7 +316,7 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
     auto sub = [&](int q) { return pin && r0 + q == D.nz - 1 ? 0.0 : t_sub[q * S + g]; };
     auto dia = [&](int q) { return pin && r0 + q == D.nz - 1 ? 1.0 : t_dia[q * S + g] - (r0 + q < D.nz ? sh : 0.0); };
     double inv[M - 1];
-    inv[0] = 1.0 / dia(0);
+    inv[0] = spec_rcp(dia(0));
     v[0].x *= inv[0];
     v[0].y *= inv[0];
     double L = -sub(0) * inv[0];
@@ -268,7 +326,7 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
 #pragma unroll
     for (int q = 1; q < M - 1; ++q) {
       const double cp = t_sup[(q - 1) * S + g] * inv[q - 1], sb = sub(q);
-      inv[q] = 1.0 / (dia(q) - sb * cp);
+      inv[q] = spec_rcp(dia(q) - sb * cp);
       v[q].x = (v[q].x - sb * v[q - 1].x) * inv[q];
       v[q].y = (v[q].y - sb * v[q - 1].y) * inv[q];
       L = -sb * L * inv[q];
@@ -290,7 +348,7 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
       const double4 nx = g + 1 < S ? e0[threadIdx.x + 8] : make_double4(0.0, 0.0, 0.0, 0.0);
       const double sb = sub(M - 1), sp = t_sup[(M - 1) * S + g];
       const double spn = pin && r0 + M - 1 == D.nz - 1 ? 0.0 : sp;
-      const double ib = 1.0 / (dia(M - 1) - sb * cl + spn * nx.z);
+      const double ib = spec_rcp(dia(M - 1) - sb * cl + spn * nx.z);
       A = sb * L * ib;
       C = spn * nx.w * ib;
       F.x = (v[M - 1].x - sb * v[M - 2].x - spn * nx.x) * ib;
@@ -303,7 +361,7 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
       const double4 z4 = make_double4(0.0, 0.0, 0.0, 0.0);
       const double4 um = g >= d ? e[threadIdx.x - 8 * d] : z4;
       const double4 up = g + d < S ? e[threadIdx.x + 8 * d] : z4;
-      const double kk = 1.0 / (1.0 - A * um.y - C * up.x);
+      const double kk = spec_rcp(1.0 - A * um.y - C * up.x);
       F.x = (F.x - A * um.z - C * up.z) * kk;
       F.y = (F.y - A * um.w - C * up.w) * kk;
       A = -A * um.x * kk;
@@ -359,44 +417,63 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
   }
 }
 
-// |f - A phi|: a thread takes K planes of one (i, j), the z neighbours kept
-// in registers; grid (ceil(nx*ny/256), ceil(nz/K) * members).  K = 8, or 2
-// on the grids that 8 planes leave with less than two blocks per SM.
-template <int K>
-__global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int nzb) {
-  const int b = blockIdx.y / nzb;
+// |f - A phi|: a block owns 32 x 8 columns (a row's y neighbours come from
+// L1 then) and marches `per` planes, the z neighbours kept in registers;
+// grid (ceil(nx/32), ceil(ny/8), ceil(nz/per) * members).  per = 32, fewer
+// where that leaves less than two blocks per SM: a block ends in two sums
+// and an arrival, as long as about four planes (337 us with 8 planes and
+// flat columns at 512x256x512).
+constexpr int kCheckK = 4;
+__global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int per, int nzb) {
+  const int b = blockIdx.z / nzb;
   if (!D.st[b].act) return;
   const double* __restrict__ phi = D.mt ? D.mt[b].phi : D.phi;
   const double* __restrict__ rhs = D.mt ? D.mt[b].rhs : D.rhs;
-  const int col = blockIdx.x * 256 + threadIdx.x;
-  const int zb = blockIdx.y - b * nzb;
-  const int k0 = 2 + zb * K;
+  const int i = 2 + blockIdx.x * 32 + (threadIdx.x & 31), j = 2 + blockIdx.y * 8 + (threadIdx.x >> 5);
+  const int zb = blockIdx.z - b * nzb;
+  const int k0 = 2 + zb * per, kend = min(k0 + per, D.nz + 2);  // exclusive
   double rr = 0.0, ff = 0.0;
-  if (col < D.nx * D.ny) {
-    const int j = 2 + col / D.nx, i = 2 + col - (j - 2) * D.nx;
+  if (i <= D.nx + 1 && j <= D.ny + 1) {
     int64_t c = cidx(i, j, k0, D.X, D.XY);
     double pm = phi[c - D.XY], pc = phi[c];
+    const double a0 = 2.0 * D.a1 + 2.0 * D.a3;
+    auto cell = [&](int k, double pp, double f, double pw, double pe, double ps, double pn) {
+      const double dg = -(a0 + D.coef[2 * D.Z + k - 1] + D.coef[3 * D.Z + k - 1]);
+      double acc = D.a1 * (pw + pe);
+      acc += D.a3 * (ps + pn);
+      acc += D.coef[k - 1] * pm;
+      acc += D.coef[D.Z + k - 1] * pp;
+      acc += dg * pc;
+      const double r = f - acc;
+      rr += r * r;
+      ff += f * f;
+      pm = pc;
+      pc = pp;
+    };
+    int k = k0;
+    for (; k + kCheckK <= kend; k += kCheckK) {
+      double v[kCheckK][6];
 #pragma unroll
-    for (int q = 0; q < K; ++q) {
-      const int k = k0 + q;
-      if (k <= D.nz + 1) {
-        const double pp = phi[c + D.XY], f = rhs[c];
-        const double dg = -(2.0 * D.a1 + 2.0 * D.a3 + D.coef[2 * D.Z + k - 1] + D.coef[3 * D.Z + k - 1]);
-        double acc = D.a1 * (phi[c - 1] + phi[c + 1]);
-        acc += D.a3 * (phi[c - D.X] + phi[c + D.X]);
-        acc += D.coef[k - 1] * pm;
-        acc += D.coef[D.Z + k - 1] * pp;
-        acc += dg * pc;
-        const double r = f - acc;
-        rr += r * r;
-        ff += f * f;
-        pm = pc;
-        pc = pp;
-        c += D.XY;
+      for (int q = 0; q < kCheckK; ++q) {
+        const int64_t o = c + q * D.XY;
+        v[q][0] = phi[o + D.XY];
+        v[q][1] = rhs[o];
+        v[q][2] = phi[o - 1];
+        v[q][3] = phi[o + 1];
+        v[q][4] = phi[o - D.X];
+        v[q][5] = phi[o + D.X];
       }
+#pragma unroll
+      for (int q = 0; q < kCheckK; ++q) cell(k + q, v[q][0], v[q][1], v[q][2], v[q][3], v[q][4], v[q][5]);
+      c += kCheckK * D.XY;
     }
+    for (; k < kend; ++k, c += D.XY)
+      cell(k, phi[c + D.XY], rhs[c], phi[c - 1], phi[c + 1], phi[c - D.X], phi[c + D.X]);
   }
-  spec_norm_finish(D, b, blockIdx.x + gridDim.x * zb, gridDim.x * nzb, rr, ff, true);
+  __shared__ SpecNorm norm;
+  const int nslots = gridDim.x * gridDim.y * nzb;
+  spec_norm_arrive(norm, D, b, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * zb), nslots, rr, ff);
+  spec_norm_finish(norm, D, b, nslots, true);
 }
 
 // ------------------------------------------------------------------ host
@@ -444,8 +521,12 @@ bool spec_supported(int nx, int ny, int nz) {
 }
 
 constexpr int kFillBlocks = 2 * 148;
-static int check_cols(const SpecDev& D) { return (D.nx * D.ny + 255) / 256; }
-static int check_planes(const SpecDev& D) { return check_cols(D) * ((D.nz + 7) / 8) < kFillBlocks ? 2 : 8; }
+static int check_cols(const SpecDev& D) { return ((D.nx + 31) / 32) * ((D.ny + 7) / 8); }
+static int check_planes(const SpecDev& D) {
+  int per = 32;
+  while (per > 2 && check_cols(D) * ((D.nz + per - 1) / per) < kFillBlocks) per /= 2;
+  return per;
+}
 static int check_zblocks(const SpecDev& D) { return (D.nz + check_planes(D) - 1) / check_planes(D); }
 static size_t x_smem(const SpecDev& D) { return (size_t)2 * D.pairs * spec_row(D.nx) * sizeof(double2); }
 // columns per block of the y passes: eight fill a 128-byte line; fewer
@@ -489,6 +570,8 @@ int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const 
   D.XY = (int64_t)(nx + 2) * (ny + 2);
   D.Z = nz + 2;
   D.nu = (int64_t)D.nxh * ny;
+  D.dnx = spec_div_magic(nx);
+  D.dnh = spec_div_magic(D.nxh);
   D.a1 = a1;
   D.a3 = a3;
   D.scale = 1.0 / ((double)nx * ny);
@@ -660,9 +743,8 @@ void launch_spec_update(const SpecDev& D, int nm, cudaStream_t s) {
 
 void launch_spec_check(const SpecDev& D, int nm, cudaStream_t s) {
   const int nzb = check_zblocks(D);
-  const dim3 g((unsigned)check_cols(D), (unsigned)(nzb * nm));
-  if (check_planes(D) == 8) k_spec_check<8><<<g, 256, 0, s>>>(D, nzb);
-  else k_spec_check<2><<<g, 256, 0, s>>>(D, nzb);
+  const dim3 g((unsigned)((D.nx + 31) / 32), (unsigned)((D.ny + 7) / 8), (unsigned)(nzb * nm));
+  k_spec_check<<<g, 256, 0, s>>>(D, check_planes(D), nzb);
   count_launch();
 }
 

@@ -54,6 +54,7 @@ struct SpecDev {
   int X;
   int64_t XY;
   int64_t nu;          // nxh * ny complex values of a plane
+  unsigned dnx, dnh;   // reciprocals of nx and nxh (spec_div)
   double a1, a3;       // x and y coefficients
   double scale;        // 1 / (nx * ny)
   const double* coef;  // the fine level's cz5[Z] cz6[Z] dz5[Z] dz6[Z]
