@@ -131,19 +131,26 @@ void dyn_pass_launch(const NSDev& D, const double* src, double* dst, int hf, cud
 }
 
 // The three directions of the test filter in one pass, for fields whose z
-// rule only sets the two ghost rows (dyn_fusable).  As three passes, each
-// with the field's ghost pass after it, a filter is six launches and reads
-// and writes the field three times: 63 us against 14 us at 192x96x96, and
-// an update of the three models runs 48 of them.  A block owns 32 x 8
-// columns and marches `per` planes: the x-filtered rows of a plane (one
-// more on each side, periodic) go through shared memory to the y filter,
-// the y-filtered planes k-1, k, k+1 stay in registers for the z filter,
-// whose ghost values the rule gives from the y-filtered end rows as the
-// ghost pass between the passes did.  The source's zero weights drop out
+// rule only sets the two ghost rows (dyn_fusable; for w also the wall row).
+// As three passes, each with the field's ghost pass after it, a filter is
+// six launches and reads and writes the field three times.  A block owns
+// 32 x 8 columns and marches `per` planes: the raw values of a plane (one
+// column and row more on each side, periodic) go through shared memory to
+// the x and y filters, the filtered planes k-1, k, k+1 stay in registers
+// for the z filter, whose ghost values the rule gives from the filtered
+// end rows as the ghost passes in between did.  The next plane's values are
+// loaded before this one's are used.  The source's zero weights drop out
 // (0 * x + y = y for finite x).
+//
+// The raw values come from a functor In (NF fields at an interior cell) and
+// the filtered ones go to a functor Out, so that the products a model
+// filters and what it does with the results take no passes of their own:
+// DSM's six components were 18 launches each and are two, the scalar
+// models' three directions 20 and are one.
 struct DynZ {
   int type[2];
   double val[2], dz[2];  // wall values; the spacings that multiply them
+  int iw;                // w edge node: row nz+1 is the wall value, nz+2 zero
 };
 
 __device__ __forceinline__ double dyn_w3(double a, double b, double c) {
@@ -151,69 +158,200 @@ __device__ __forceinline__ double dyn_w3(double a, double b, double c) {
 }
 
 constexpr int kDynI = 32, kDynJ = 8;
-__global__ void __launch_bounds__(kDynI * kDynJ) k_dyn_filter3(NSDev D, const double* __restrict__ src,
-                                                               double* __restrict__ dst, DynZ R, int fx, int fy,
-                                                               int fz, int per) {
-  __shared__ double sx[2][kDynJ + 2][kDynI];
+constexpr int kDynW = kDynI + 2, kDynTile = kDynW * (kDynJ + 2);
+constexpr int kDynSlots = (kDynTile + kDynI * kDynJ - 1) / (kDynI * kDynJ);
+
+struct DynFilt {
+  int x, y, z;  // filtered directions
+  int per;      // planes per block
+};
+
+template <int NF, class In, class Out>
+__global__ void __launch_bounds__(kDynI * kDynJ) k_dyn_filter(const __grid_constant__ NSDev D, In in, Out out, DynZ R,
+                                                              DynFilt Q) {
+  __shared__ double sm[2][NF][kDynTile];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int i0 = 2 + blockIdx.x * kDynI, j0 = 2 + blockIdx.y * kDynJ, k0 = 2 + blockIdx.z * per;
+  const int i0 = 2 + blockIdx.x * kDynI, j0 = 2 + blockIdx.y * kDynJ, k0 = 2 + blockIdx.z * Q.per;
   const int i = i0 + tx, j = j0 + ty;
   const int nx = D.nx, ny = D.ny, nz = D.nz;
-  const int kend = min(k0 + per, nz + 2);  // exclusive
-  const bool in = i <= nx + 1 && j <= ny + 1;
-  int buf = 0;
-  // the y-filtered value of this thread's column on interior plane k (the
-  // whole block calls it)
-  auto plane = [&](int k) {
-    for (int r = ty; r < kDynJ + 2; r += kDynJ) {
-      int jj = j0 - 1 + r;
-      if (jj > ny + 2) break;
+  const int kend = min(k0 + Q.per, nz + 2);  // exclusive
+  const bool live = i <= nx + 1 && j <= ny + 1;
+  double raw[kDynSlots][NF];
+  auto fetch = [&](int k) {
+#pragma unroll
+    for (int q = 0; q < kDynSlots; ++q) {
+      const int e = threadIdx.x + q * kDynI * kDynJ;
+      const int r = e / kDynW;
+      int ii = i0 - 1 + e - r * kDynW, jj = j0 - 1 + r;
+      if (e >= kDynTile || ii > nx + 2 || jj > ny + 2) continue;
+      ii = ii == 1 ? nx + 1 : (ii == nx + 2 ? 2 : ii);
       jj = jj == 1 ? ny + 1 : (jj == ny + 2 ? 2 : jj);
-      if (i <= nx + 1) {
-        const double* p = src + NS_IX(i, jj, k);
-        sx[buf][r][tx] = !fx ? p[0] : (i == nx + 1 ? dyn_w3(p[1], p[0], p[-1]) : dyn_w3(p[-1], p[0], p[1]));
-      }
+      in(D, ii, jj, k, raw[q]);
+    }
+  };
+  int buf = 0;
+  // x- and y-filtered values of this thread's column on interior plane k
+  // (already fetched); starts the fetch of plane `next` (0: none)
+  auto plane = [&](int next, double (&v)[NF]) {
+#pragma unroll
+    for (int q = 0; q < kDynSlots; ++q) {
+      const int e = threadIdx.x + q * kDynI * kDynJ;
+      if (e < kDynTile)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) sm[buf][f][e] = raw[q][f];
     }
     __syncthreads();
-    double v = 0.0;
-    if (in) {
-      const double a = sx[buf][ty][tx], b = sx[buf][ty + 1][tx], c = sx[buf][ty + 2][tx];
-      v = !fy ? b : (j == ny + 1 ? dyn_w3(c, b, a) : dyn_w3(a, b, c));
+    if (next) fetch(next);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      const double* s = &sm[buf][f][ty * kDynW + tx];
+      auto xf = [&](int r) {
+        const double* p = s + r * kDynW;
+        return !Q.x ? p[1] : (i == nx + 1 ? dyn_w3(p[2], p[1], p[0]) : dyn_w3(p[0], p[1], p[2]));
+      };
+      if (!Q.y) v[f] = xf(1);
+      else v[f] = j == ny + 1 ? dyn_w3(xf(2), xf(1), xf(0)) : dyn_w3(xf(0), xf(1), xf(2));
     }
     buf ^= 1;  // the next call's stores do not meet this one's loads
-    return v;
   };
-  double ym = k0 > 2 && fz ? plane(k0 - 1) : 0.0;
-  double yc = plane(k0);
-  if (k0 == 2) {
-    ym = R.type[0] == 1 ? R.val[0] : (R.type[0] == 6 ? 2.0 * R.val[0] - 1.0 * yc : yc - R.val[0] * R.dz[0]);
-  }
+  double ym[NF], yc[NF], yp[NF];
+  const bool below = k0 > 2 && Q.z;
+  fetch(below ? k0 - 1 : k0);
+  if (below) plane(k0, ym);
+  plane(k0 + 1 < kend || (Q.z && k0 <= nz) ? k0 + 1 : 0, yc);
+  if (R.iw && k0 == nz + 1)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) yc[f] = R.val[1];
+  if (k0 == 2)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      ym[f] = R.type[0] == 1 ? R.val[0]
+                             : (R.type[0] == 6 ? 2.0 * R.val[0] - 1.0 * yc[f] : yc[f] - R.val[0] * R.dz[0]);
   for (int k = k0; k < kend; ++k) {
-    double yp = 0.0;
     if (k <= nz) {
-      if (fz || k + 1 < kend) yp = plane(k + 1);
+      if (Q.z || k + 1 < kend) plane(k + 2 < kend || (Q.z && k + 1 < kend && k + 1 <= nz) ? k + 2 : 0, yp);
+      if (R.iw && k == nz)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) yp[f] = R.val[1];
     } else {
-      yp = R.type[1] == 1 ? R.val[1] : (R.type[1] == 6 ? 2.0 * R.val[1] - 1.0 * yc : yc + R.val[1] * R.dz[1]);
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+        yp[f] = R.iw ? 0.0
+                     : (R.type[1] == 1 ? R.val[1]
+                                       : (R.type[1] == 6 ? 2.0 * R.val[1] - 1.0 * yc[f] : yc[f] + R.val[1] * R.dz[1]));
     }
-    if (in) dst[NS_IX(i, j, k)] = !fz ? yc : (k == nz + 1 ? dyn_w3(yp, yc, ym) : dyn_w3(ym, yc, yp));
-    ym = yc;
-    yc = yp;
+    double v[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      v[f] = !Q.z ? yc[f] : (k == nz + 1 ? dyn_w3(yp[f], yc[f], ym[f]) : dyn_w3(ym[f], yc[f], yp[f]));
+    if (live) out(D, NS_IX(i, j, k), k, v);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      ym[f] = yc[f];
+      yc[f] = yp[f];
+    }
   }
 }
+
+// a field to a field
+struct DynFieldIn {
+  const double* __restrict__ a;
+  __device__ __forceinline__ void operator()(const NSDev& D, int i, int j, int k, double (&v)[1]) const {
+    v[0] = a[NS_IX(i, j, k)];
+  }
+};
+struct DynFieldOut {
+  double* __restrict__ a;
+  __device__ __forceinline__ void operator()(const NSDev&, int64_t o, int, const double (&v)[1]) const { a[o] = v[0]; }
+};
+
+// DSM's component ij with strain l1 (DSM.F90:88-190): filters of
+// delg**2 modS l1, l1 and the product of the centred velocities, then
+//   l3 = F(delg**2 modS l1) - (rt delg)**2 fmodS F(l1)
+//   l4 = l4 + w (l3 F(ca cb) - l3 fa fb),  C = C + w l3 l3
+// with the weight w = 2 off the diagonal in the source's order.
+struct DsmIn {
+  const double *l1, *modS, *ca, *cb, *dg;
+  __device__ __forceinline__ void operator()(const NSDev& D, int i, int j, int k, double (&v)[3]) const {
+    const int64_t o = NS_IX(i, j, k);
+    const double g = dg[k - 1];
+    v[1] = l1[o];
+    v[0] = g * g * modS[o] * v[1];
+    v[2] = ca[o] * cb[o];
+  }
+};
+struct DsmOut {
+  const double *fmodS, *fa, *fb, *dg;
+  double *l4, *C;
+  double rt;
+  int off, first;
+  __device__ __forceinline__ void operator()(const NSDev&, int64_t o, int k, const double (&v)[3]) const {
+    const double rd = rt * dg[k - 1];
+    const double l3 = v[0] - rd * rd * fmodS[o] * v[1];
+    double a = first ? 0.0 : l4[o], c = first ? 0.0 : C[o];
+    if (off) {
+      a = a + 2.0 * l3 * v[2];
+      a = a - 2.0 * l3 * fa[o] * fb[o];
+      c = c + 2.0 * l3 * l3;
+    } else {
+      a = a + l3 * v[2];
+      a = a - l3 * fa[o] * fb[o];
+      c = c + l3 * l3;
+    }
+    l4[o] = a;
+    C[o] = c;
+  }
+};
+
+// DSMrho / DSMscal1 in direction dir (DSMrho.F90:30-140): filters of the
+// weighted and the plain gradient of the scalar, of its flux and of itself,
+//   l2 = F(delg**2 modS grad) - (rt delg)**2 fmodS F(grad)
+//   l3 = F(flux) - F(c) fvel
+//   l4 = l4 + l2 l2,  C = C + l2 l3
+struct DsmScalarIn {
+  const double *c, *modS, *vel, *dg;
+  int dir;
+  __device__ __forceinline__ void operator()(const NSDev& D, int i, int j, int k, double (&v)[4]) const {
+    const int64_t o = NS_IX(i, j, k), st = dir == 0 ? 1 : (dir == 1 ? (int64_t)D.X : D.XY);
+    const double c0 = c[o], t1 = 0.5 * (c0 + c[o - st]), t2 = 0.5 * (c0 + c[o + st]);
+    const double rd = dir == 0 ? MT(D.rdxc, i) : (dir == 1 ? MT(D.rdyc, j) : MT(D.rdzc, k));
+    const double g = dg[k - 1];
+    v[0] = g * g * modS[o] * (t2 - t1) * rd;
+    v[1] = (t2 - t1) * rd;
+    v[2] = c0 * 0.5 * (vel[o - st] + vel[o]);
+    v[3] = c0;
+  }
+};
+struct DsmScalarOut {
+  const double *fmodS, *fvel, *dg;
+  double *l4, *C;
+  double rt;
+  int first;
+  __device__ __forceinline__ void operator()(const NSDev&, int64_t o, int k, const double (&v)[4]) const {
+    const double rd = rt * dg[k - 1];
+    const double l2 = v[0] - rd * rd * fmodS[o] * v[1];
+    const double l3 = v[2] - v[3] * fvel[o];
+    l4[o] = (first ? 0.0 : l4[o]) + l2 * l2;
+    C[o] = (first ? 0.0 : C[o]) + l2 * l3;
+  }
+};
 
 // rules whose ghost pass leaves the interior rows alone
 bool dyn_fusable(const ZRule& R) {
   auto ok = [](int t) { return t == 1 || t == 2 || t == 4 || t == 6; };
-  return R.iw == 0 && R.rt == 0 && ok(R.type[0]) && ok(R.type[1]);
+  return (R.iw == 0 || R.type[1] == 1) && R.rt == 0 && ok(R.type[0]) && ok(R.type[1]);
 }
 
-void launch_dyn_filter3(const NSDev& D, const double* src, double* dst, const DynZ& R, const int* filt,
-                        cudaStream_t s) {
+template <int NF, class In, class Out>
+void launch_dyn_filter(const NSDev& D, const In& in, const Out& out, const DynZ& R, const int* filt, cudaStream_t s) {
   dim3 g((unsigned)((D.nx + kDynI - 1) / kDynI), (unsigned)((D.ny + kDynJ - 1) / kDynJ));
-  int per = 32;  // fewer planes per block until there are two blocks per SM
-  while (per > 4 && (int64_t)g.x * g.y * ((D.nz + per - 1) / per) < 2 * 148) per /= 2;
-  g.z = (unsigned)((D.nz + per - 1) / per);
-  k_dyn_filter3<<<g, kDynI * kDynJ, 0, s>>>(D, src, dst, R, filt[0], filt[1], filt[2], per);
+  // planes per block: 32, fewer until there are four blocks per SM (two
+  // more planes are filtered than written)
+  DynFilt Q{filt[0], filt[1], filt[2], 32};
+  while (Q.per > 4 && (int64_t)g.x * g.y * ((D.nz + Q.per - 1) / Q.per) < 4 * 148) Q.per /= 2;
+  g.z = (unsigned)((D.nz + Q.per - 1) / Q.per);
+  k_dyn_filter<NF, In, Out><<<g, kDynI * kDynJ, 0, s>>>(D, in, out, R, Q);
+  count_launch();
 }
 
 void launch_dyn_pass(const NSDev& D, const double* src, double* dst, int dir, int hf, cudaStream_t s) {
@@ -225,6 +363,8 @@ void launch_dyn_pass(const NSDev& D, const double* src, double* dst, int dir, in
     dyn_pass_launch<2>(D, src, dst, hf, s);
 }
 
+// The general path (z rules that are not dyn_fusable): the source's whole-
+// array operations one by one.
 // whole-array assignments of the source (ghost cells included)
 enum { EW_SUB, EW_MUL, EW_ACC, EW_ACC2, EW_DEC1, EW_DEC, EW_DEC2 };
 // (out may alias a or b: no __restrict__)
@@ -290,7 +430,7 @@ __global__ void k_dyn_bcast(NSDev D, const double* __restrict__ prof, int clip, 
 }
 
 // out = 0.5 num / den, 1e-20 where den == 0 (DSM.F90:242-250)
-__global__ void k_dyn_ratio(NSDev D, const double* __restrict__ num, const double* __restrict__ den,
+__global__ void k_dyn_ratio_cells(NSDev D, const double* __restrict__ num, const double* __restrict__ den,
                             double* __restrict__ out) {
   DYN_CELL();
   out[o] = den[o] == 0.0 ? 1.0e-20 : 0.5 * num[o] / den[o];
@@ -301,6 +441,49 @@ __global__ void k_dyn_column(NSDev D, const double* __restrict__ a, double* __re
   const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
   if (k > D.Z) return;
   prof[k - 1] = a[NS_IX(2, 2, k)];
+}
+
+// The coefficient from the plane partial sums of its numerator and
+// denominator (k_plane_part: nb per plane): the plane averages, the
+// numerator's negative values to 0, 0.5 num / den (1e-20 where den == 0),
+// then filterHF (DSM.F90:196-256).  Everything after the averages is
+// constant on planes, where filterHF's x and y passes change nothing, so it
+// is a computation on profiles; prof(k), k = 2..nz+1.
+__global__ void __launch_bounds__(256) k_dyn_ratio(NSDev D, const double* __restrict__ pn,
+                                                   const double* __restrict__ pd, int nb, double area, DynZ R,
+                                                   double* __restrict__ prof) {
+  extern __shared__ double sr[];
+  const int nz = D.nz;
+  for (int k = 2 + threadIdx.x; k <= nz + 1; k += blockDim.x) {
+    double n = 0.0, d = 0.0;
+    for (int b = 0; b < nb; ++b) {
+      n += pn[(int64_t)(k - 1) * nb + b];
+      d += pd[(int64_t)(k - 1) * nb + b];
+    }
+    n = n / area;
+    d = d / area;
+    if (n < 0.0) n = 0.0;
+    sr[k - 1] = d == 0.0 ? 1.0e-20 : 0.5 * n / d;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const double b = sr[1], t = sr[nz];
+    sr[0] = R.type[0] == 1 ? R.val[0] : (R.type[0] == 6 ? 2.0 * R.val[0] - 1.0 * b : b - R.val[0] * R.dz[0]);
+    sr[nz + 1] = R.type[1] == 1 ? R.val[1] : (R.type[1] == 6 ? 2.0 * R.val[1] - 1.0 * t : t + R.val[1] * R.dz[1]);
+  }
+  __syncthreads();
+  for (int k = 2 + threadIdx.x; k <= nz + 1; k += blockDim.x) {
+    const double p0 = sr[k - 1], pm = sr[k - 2], pp = sr[k];
+    double r = p0;
+    if (p0 < pp && p0 < pm) {
+      const double x = dyn_w3(pm, p0, pp);
+      if (x < pp && x < pm) r = x;
+    } else if (p0 > pp && p0 > pm) {
+      const double x = dyn_w3(pm, p0, pp);
+      if (x > pp && x > pm) r = x;
+    }
+    prof[k - 1] = r;
+  }
 }
 
 #undef DYN_CELL
@@ -330,7 +513,7 @@ int NSSolver::ensure_dyn() {
   h.insert(h.end(), dg.begin(), dg.end());
   h.resize(h.size() + 2 * (size_t)Z, 0.0);
   const size_t nm = h.size();
-  ANEL_CUDA_TRY(cudaMalloc(&d_dyn_m_, (nm + (size_t)plane_part_doubles(D_)) * sizeof(double)));
+  ANEL_CUDA_TRY(cudaMalloc(&d_dyn_m_, (nm + 2 * (size_t)plane_part_doubles(D_)) * sizeof(double)));
   ANEL_CUDA_TRY(cudaMemcpy(d_dyn_m_, h.data(), nm * sizeof(double), cudaMemcpyHostToDevice));
   dyn_part_ = d_dyn_m_ + nm;
   // coordinates for center_velocity: xe xc ye yc ze zc
@@ -357,16 +540,20 @@ int NSSolver::ensure_dyn() {
   return ANEL_OK;
 }
 
+static DynZ make_dyn_z(const ZRule& R, const std::vector<double>& dzc, const std::vector<double>& dze, int nz) {
+  const std::vector<double>& d = R.dzt_is_zc ? dzc : dze;
+  return DynZ{{R.type[0], R.type[1]}, {R.val[0], R.val[1]}, {d[1 + R.of1], d[nz + R.of2]}, R.iw};
+}
+#define dyn_z(R) make_dyn_z(R, m_[2][3], m_[2][2], nz_)
+
 // filter(in, out, 2, xfil, yfil, zfil, vt) (hf = 0) or filterHF(in, out,
-// 2, 1, 1, 1, vt) (hf = 1): in is not modified
-void NSSolver::dyn_filter(const double* in, double* out, int vt, int hf, cudaStream_t s, double* tmp) {
+// 2, 1, 1, 1, vt) (hf = 1): in is not modified; ghosts = false: only out's
+// interior is wanted
+void NSSolver::dyn_filter(const double* in, double* out, int vt, int hf, cudaStream_t s, double* tmp, bool ghosts) {
   const ZRule R = zrule(vt);
   if (!hf && in != out && dyn_fusable(R)) {
-    auto dzt = [&](int k) { return R.dzt_is_zc ? m_[2][3][k - 1] : m_[2][2][k - 1]; };
-    const DynZ z{{R.type[0], R.type[1]}, {R.val[0], R.val[1]}, {dzt(2 + R.of1), dzt(nz_ + 1 + R.of2)}};
-    launch_dyn_filter3(D_, in, out, z, prm_.filt, s);
-    count_launch();
-    launch_ghost_field(D_, out, R, s);
+    launch_dyn_filter<1>(D_, DynFieldIn{in}, DynFieldOut{out}, dyn_z(R), prm_.filt, s);
+    if (ghosts) launch_ghost_field(D_, out, R, s);
     return;
   }
   if (!tmp) tmp = d_dyn_ + (size_t)DY_TMP * G_;
@@ -427,13 +614,15 @@ int NSSolver::dyn_prepare(cudaStream_t s) {
   double *l1 = F + (size_t)DY_L1 * G_, *l2 = F + (size_t)DY_L2 * G_, *l3 = F + (size_t)DY_L3 * G_;
   k_dyn_modS<<<g, 128, 0, s>>>(D_, D_.u, D_.v, D_.w, modS);
   count_launch();
-  launch_ghost_field(D_, modS, zrule(NV_CFLUC), s);
+  // the fused models read the interior of these fields only
+  const bool fused = dyn_fusable(zrule(NV_CFLUC));
+  if (!fused) launch_ghost_field(D_, modS, zrule(NV_CFLUC), s);
   dyn_filter(D_.u, l1, NV_U, 0, s);
   dyn_filter(D_.v, l2, NV_V, 0, s);
   dyn_filter(D_.w, l3, NV_W, 0, s);
   k_dyn_modS<<<g, 128, 0, s>>>(D_, l1, l2, l3, fmodS);
   count_launch();
-  launch_ghost_field(D_, fmodS, zrule(NV_CFLUC), s);
+  if (!fused) launch_ghost_field(D_, fmodS, zrule(NV_CFLUC), s);
   const double* vel[3] = {D_.u, D_.v, D_.w};
   const double* ax_e[3] = {d_dyn_ax_[0], d_dyn_ax_[2], d_dyn_ax_[4]};
   const double* ax_c[3] = {d_dyn_ax_[1], d_dyn_ax_[3], d_dyn_ax_[5]};
@@ -442,7 +631,7 @@ int NSSolver::dyn_prepare(cudaStream_t s) {
     launch_center(D_, vel[d], c, d + 1, prm_.stretched[d], prm_.interp == ANEL_DIAG_CORRECTED, ax_e[d], ax_c[d],
                   s);
     launch_ghost_field(D_, c, zrule(d == 0 ? NV_U : (d == 1 ? NV_V : NV_W)), s);
-    dyn_filter(c, F + (size_t)(DY_FC0 + d) * G_, NV_CFLUC, 0, s);
+    dyn_filter(c, F + (size_t)(DY_FC0 + d) * G_, NV_CFLUC, 0, s, nullptr, !fused);
   }
   ANEL_CUDA_TRY(cudaGetLastError());
   return ANEL_OK;
@@ -465,7 +654,7 @@ int NSSolver::dyn_ratio(double* num, double* den, double* out, cudaStream_t s) {
   k_dyn_bcast<<<g, 128, 0, s>>>(D_, pd, 0, den);
   count_launch(2);
   launch_ghost_fields2(D_, num, den, cf, s);
-  k_dyn_ratio<<<g, 128, 0, s>>>(D_, num, den, out);
+  k_dyn_ratio_cells<<<g, 128, 0, s>>>(D_, num, den, out);
   count_launch();
   launch_ghost_field(D_, out, cf, s);
   double* P = d_dyn_ + (size_t)DY_P * G_;
@@ -486,12 +675,44 @@ int NSSolver::dyn_profile(const double* a, double* host, cudaStream_t s) {
   return ANEL_OK;
 }
 
+// The profile 0.5 <num> / <den>, smoothed, of interior fields num and den
+int NSSolver::dyn_coefficient(const double* num, const double* den, double* host, cudaStream_t s) {
+  const int X = nx_ + 2, Y = ny_ + 2, Z = nz_ + 2;
+  const double* dxc = d_dyn_m_;
+  const double* dyc = dxc + X;
+  double* pr = d_dyn_m_ + X + Y + Z;
+  double* pd = dyn_part_ + plane_part_doubles(D_);
+  const int nb = launch_plane_part(D_, num, dxc, dyc, dyn_part_, s);
+  launch_plane_part(D_, den, dxc, dyc, pd, s);
+  k_dyn_ratio<<<1, 256, Z * sizeof(double), s>>>(D_, dyn_part_, pd, nb, dyn_area_, dyn_z(zrule(NV_CFLUC)), pr);
+  count_launch();
+  ANEL_CUDA_TRY(cudaGetLastError());
+  ANEL_CUDA_TRY(cudaMemcpyAsync(host, pr, Z * sizeof(double), cudaMemcpyDeviceToHost, s));
+  ANEL_CUDA_TRY(cudaStreamSynchronize(s));
+  return ANEL_OK;
+}
+
 // DSM (DSM.F90:1-258): the Csgs profile into cs (Z values)
 int NSSolver::dsm_velocity(cudaStream_t s, double* cs) {
   int st = ensure_dyn();
   if (st != ANEL_OK) return st;
   if ((st = dyn_prepare(s)) != ANEL_OK) return st;
   double* F = d_dyn_;
+  if (dyn_fusable(zrule(NV_CFLUC))) {
+    const double* dg = d_dyn_m_ + (nx_ + 2) + (ny_ + 2);
+    double *l1 = F + (size_t)DY_L1 * G_, *l4 = F + (size_t)DY_L4 * G_, *C = F + (size_t)DY_B * G_;
+    const double *modS = F + (size_t)DY_MODS * G_, *fmodS = F + (size_t)DY_FMODS * G_;
+    static const int qa[7] = {0, 0, 1, 2, 0, 0, 1}, qb[7] = {0, 0, 1, 2, 1, 2, 2};
+    for (int ij = 1; ij <= 6; ++ij) {
+      k_dyn_comp<<<interior_grid(D_), 128, 0, s>>>(D_, ij, l1);
+      count_launch();
+      const DsmIn in{l1, modS, F + (size_t)(DY_C0 + qa[ij]) * G_, F + (size_t)(DY_C0 + qb[ij]) * G_, dg};
+      const DsmOut out{fmodS, F + (size_t)(DY_FC0 + qa[ij]) * G_, F + (size_t)(DY_FC0 + qb[ij]) * G_, dg, l4, C,
+                       prm_.test_ratio, ij > 3, ij == 1};
+      launch_dyn_filter<3>(D_, in, out, dyn_z(zrule(NV_CFLUC)), prm_.filt, s);
+    }
+    return dyn_coefficient(l4, C, cs, s);
+  }
   const dim3 g = interior_grid(D_);
   const double* dg = d_dyn_m_ + (nx_ + 2) + (ny_ + 2);
   const double* modS = F + (size_t)DY_MODS * G_;
@@ -547,16 +768,24 @@ int NSSolver::dsm_scalar(const double* c, cudaStream_t s, double* out) {
   if (st != ANEL_OK) return st;
   if ((st = dyn_prepare(s)) != ANEL_OK) return st;
   double* F = d_dyn_;
-  const dim3 g = interior_grid(D_);
   const double* dg = d_dyn_m_ + (nx_ + 2) + (ny_ + 2);
   const double* modS = F + (size_t)DY_MODS * G_;
   const double* fmodS = F + (size_t)DY_FMODS * G_;
-  double *l1 = F + (size_t)DY_L1 * G_, *l2 = F + (size_t)DY_L2 * G_, *l3 = F + (size_t)DY_L3 * G_;
-  double *l4 = F + (size_t)DY_L4 * G_, *A = F + (size_t)DY_A * G_, *C = F + (size_t)DY_B * G_;
+  double *l4 = F + (size_t)DY_L4 * G_, *C = F + (size_t)DY_B * G_;
   const ZRule cf = zrule(NV_CFLUC);
+  const double* vel[3] = {D_.u, D_.v, D_.w};
+  if (dyn_fusable(cf)) {
+    for (int d = 0; d < 3; ++d) {
+      const DsmScalarOut o{fmodS, F + (size_t)(DY_FC0 + d) * G_, dg, l4, C, prm_.test_ratio, d == 0};
+      launch_dyn_filter<4>(D_, DsmScalarIn{c, modS, vel[d], dg, d}, o, dyn_z(cf), prm_.filt, s);
+    }
+    return dyn_coefficient(C, l4, out, s);
+  }
+  const dim3 g = interior_grid(D_);
+  double *l1 = F + (size_t)DY_L1 * G_, *l2 = F + (size_t)DY_L2 * G_, *l3 = F + (size_t)DY_L3 * G_;
+  double* A = F + (size_t)DY_A * G_;
   ANEL_CUDA_TRY(cudaMemsetAsync(l4, 0, G_ * sizeof(double), s));
   ANEL_CUDA_TRY(cudaMemsetAsync(C, 0, G_ * sizeof(double), s));
-  const double* vel[3] = {D_.u, D_.v, D_.w};
   for (int d = 0; d < 3; ++d) {
     k_dyn_sgrad<<<g, 128, 0, s>>>(D_, c, modS, dg, d, 1, l1);
     count_launch();

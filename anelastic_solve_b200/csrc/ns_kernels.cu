@@ -1602,6 +1602,13 @@ void launch_fluct_sq(const NSDev& D, const double* a, const double* mean, double
 
 int64_t plane_part_doubles(const NSDev& D) { return (int64_t)kPlaneBlocks * D.Z; }
 
+int launch_plane_part(const NSDev& D, const double* a, const double* wx, const double* wy, double* part,
+                      cudaStream_t s) {
+  k_plane_part<<<dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s>>>(D, a, wx, wy, part);
+  count_launch();
+  return kPlaneBlocks;
+}
+
 void launch_plane_avg(const NSDev& D, const double* a, const double* wx, const double* wy, double area,
                       double* part, double* out, cudaStream_t s) {
   k_plane_part<<<dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s>>>(D, a, wx, wy, part);

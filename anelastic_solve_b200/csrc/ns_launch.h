@@ -82,6 +82,9 @@ void launch_center(const NSDev& D, const double* in, double* out, int dir, int s
                    const double* e, const double* c, cudaStream_t s);
 void launch_fluct_sq(const NSDev& D, const double* a, const double* mean, double* out, cudaStream_t s);
 int64_t plane_part_doubles(const NSDev& D);
+// the partial sums alone; returns their number per plane
+int launch_plane_part(const NSDev& D, const double* a, const double* wx, const double* wy, double* part,
+                      cudaStream_t s);
 void launch_plane_avg(const NSDev& D, const double* a, const double* wx, const double* wy, double area,
                       double* part, double* out, cudaStream_t s);
 void launch_diag_update(int Z, double dtt, const double* m, double* dg, cudaStream_t s);
