@@ -813,24 +813,25 @@ __device__ __forceinline__ T restrict_value(const DevLevel<T>& F, int ic, int jc
 // another by the compiler, so interleaving would serialise the cells).
 constexpr int kZBatch = 4;
 
-// Coarse cells: grid (ceil(nx/128), Y, ceil(Z/kZBatch)); thread ic covers
+// Coarse cells, ZB in z per thread (kZBatch, or 1 on the grids that leaves
+// with less than four blocks per SM): grid (ceil(nx/128), Y, ceil(Z/ZB)); thread ic covers
 // interior column ic, and the threads of columns 2 and nx+1 also zero the
 // ghost columns 1 and nx+2.  Coarse phi <- 0 everywhere, coarse f <- 0 on
 // ghosts.
-template <typename T, int CD>
+template <typename T, int CD, int ZB>
 __global__ void __launch_bounds__(128) k_restrict(DevLevel<T> F, DevLevel<T> Cl) {
   const int ic = 2 + blockIdx.x * blockDim.x + threadIdx.x;
   if (ic > Cl.nx + 1) return;
   const int jc = 1 + blockIdx.y;
-  const int k0 = 1 + blockIdx.z * kZBatch;
+  const int k0 = 1 + blockIdx.z * ZB;
   const bool row_in = jc >= 2 && jc <= Cl.ny + 1;
-  T v[kZBatch];
-  if (row_in && k0 >= 2 && k0 + kZBatch - 1 <= Cl.nz + 1) {
+  T v[ZB];
+  if (row_in && k0 >= 2 && k0 + ZB - 1 <= Cl.nz + 1) {
 #pragma unroll
-    for (int q = 0; q < kZBatch; ++q) v[q] = restrict_value<T, CD>(F, ic, jc, k0 + q);
+    for (int q = 0; q < ZB; ++q) v[q] = restrict_value<T, CD>(F, ic, jc, k0 + q);
   } else {
 #pragma unroll
-    for (int q = 0; q < kZBatch; ++q) {
+    for (int q = 0; q < ZB; ++q) {
       const int kc = k0 + q;
       v[q] = (row_in && kc >= 2 && kc <= Cl.nz + 1) ? restrict_value<T, CD>(F, ic, jc, kc) : T(0);
     }
@@ -838,7 +839,7 @@ __global__ void __launch_bounds__(128) k_restrict(DevLevel<T> F, DevLevel<T> Cl)
   const int64_t t0 = cidx(ic, jc, k0, Cl.X, Cl.XY);
   const bool g_lo = ic == 2, g_hi = ic == Cl.nx + 1;  // ghost columns beside this one
 #pragma unroll
-  for (int q = 0; q < kZBatch; ++q) {
+  for (int q = 0; q < ZB; ++q) {
     if (k0 + q > Cl.Z) break;
     const int64_t t = t0 + q * Cl.XY;
     Cl.phi[t] = T(0);

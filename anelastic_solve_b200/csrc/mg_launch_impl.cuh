@@ -60,21 +60,30 @@ void launch_zline_seg(const DevLevel<T>& L, int color, const SegFac<T>& F, cudaS
   k_zline_seg<T, kZSeg, kZSegRows><<<(unsigned)((cols + 31) / 32), block, sm, s>>>(L, color, F);
   count_launch();
 }
-template <typename T>
-void launch_restrict(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaStream_t s) {
-  const dim3 g((unsigned)((C.nx + 127) / 128), (unsigned)C.Y, (unsigned)((C.Z + kZBatch - 1) / kZBatch));
+template <typename T, int ZB>
+void launch_restrict_zb(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaStream_t s) {
+  const dim3 g((unsigned)((C.nx + 127) / 128), (unsigned)C.Y, (unsigned)((C.Z + ZB - 1) / ZB));
   switch (cdir & 7) {
-    case 0: k_restrict<T, 0><<<g, 128, 0, s>>>(F, C); break;
-    case 1: k_restrict<T, 1><<<g, 128, 0, s>>>(F, C); break;
-    case 2: k_restrict<T, 2><<<g, 128, 0, s>>>(F, C); break;
-    case 3: k_restrict<T, 3><<<g, 128, 0, s>>>(F, C); break;
-    case 4: k_restrict<T, 4><<<g, 128, 0, s>>>(F, C); break;
-    case 5: k_restrict<T, 5><<<g, 128, 0, s>>>(F, C); break;
-    case 6: k_restrict<T, 6><<<g, 128, 0, s>>>(F, C); break;
-    default: k_restrict<T, 7><<<g, 128, 0, s>>>(F, C); break;
+    case 0: k_restrict<T, 0, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 1: k_restrict<T, 1, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 2: k_restrict<T, 2, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 3: k_restrict<T, 3, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 4: k_restrict<T, 4, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 5: k_restrict<T, 5, ZB><<<g, 128, 0, s>>>(F, C); break;
+    case 6: k_restrict<T, 6, ZB><<<g, 128, 0, s>>>(F, C); break;
+    default: k_restrict<T, 7, ZB><<<g, 128, 0, s>>>(F, C); break;
   }
   count_launch();
 }
+template <typename T>
+void launch_restrict(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaStream_t s) {
+  // 4 blocks per SM: a block is 128 threads, few of them live on short rows
+  if ((int64_t)((C.nx + 127) / 128) * C.Y * ((C.Z + kZBatch - 1) / kZBatch) >= 4 * 148)
+    launch_restrict_zb<T, kZBatch>(F, C, cdir, s);
+  else
+    launch_restrict_zb<T, 1>(F, C, cdir, s);
+}
+
 template <typename T>
 void launch_prolong(const DevLevel<T>& F, const DevLevel<T>& C, int cdir, cudaStream_t s) {
   const dim3 g((unsigned)((F.nx + 127) / 128), (unsigned)F.ny, (unsigned)((F.nz + kZBatch - 1) / kZBatch));

@@ -5,6 +5,24 @@
 
 namespace anel {
 
+// v at interior cell (i, j, k), offset c, and at the ghosts that copy it
+__device__ __forceinline__ void rb_put(const RBLevel& L, int64_t c, int i, int64_t oy, int k, double v) {
+  const int ox = i == 2 ? L.nx : (i == L.nx + 1 ? -L.nx : 0);
+  auto put = [&](int64_t at, double x) {
+    L.phi[at] = x;
+    if (ox) L.phi[at + ox] = x;
+    if (oy) L.phi[at + oy] = x;
+    if (ox && oy) L.phi[at + ox + oy] = x;
+  };
+  put(c, v);
+  if (k == 2 && L.n1) put(c - L.XY, v - L.add1);
+  if (k == L.nz + 1 && L.nZ) put(c + L.XY, v + L.addZ);
+}
+// the y shift to the image of row j (0: none)
+__device__ __forceinline__ int64_t rb_yshift(const RBLevel& L, int j) {
+  return j == 2 ? (int64_t)L.ny * L.X : (j == L.ny + 1 ? -(int64_t)L.ny * L.X : 0);
+}
+
 // One half-sweep of mg_relaxRB (mg_relax.F90:146-168) and the boundary pass
 // after it.  The boundary pass rewrites every ghost from the interior cell
 // it copies; here the thread that updates such a cell writes its images, so
@@ -41,22 +59,10 @@ __global__ void __launch_bounds__(128) k_rb_march(RBLevel L, int color) {
       v[u] = (L.src[c[u]] - acc) / L.zc[2 * Z + k - 1];
     }
   }
-  const int64_t oy = j == 2 ? (int64_t)L.ny * X : (j == L.ny + 1 ? -(int64_t)L.ny * X : 0);
+  const int64_t oy = rb_yshift(L, j);
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int k = k0 + u;
-    if (k > L.nz + 1) break;
-    const int ox = ii[u] == 2 ? L.nx : (ii[u] == L.nx + 1 ? -L.nx : 0);
-    auto put = [&](int64_t at, double x) {
-      L.phi[at] = x;
-      if (ox) L.phi[at + ox] = x;
-      if (oy) L.phi[at + oy] = x;
-      if (ox && oy) L.phi[at + ox + oy] = x;
-    };
-    put(c[u], v[u]);
-    if (k == 2 && L.n1) put(c[u] - XY, v[u] - L.add1);
-    if (k == L.nz + 1 && L.nZ) put(c[u] + XY, v[u] + L.addZ);
-  }
+  for (int u = 0; u < U; ++u)
+    if (k0 + u <= L.nz + 1) rb_put(L, c[u], ii[u], oy, k0 + u, v[u]);
 }
 
 void launch_rb_march(const RBLevel& L, int color, cudaStream_t s) {
@@ -69,12 +75,48 @@ void launch_rb_march(const RBLevel& L, int color, cudaStream_t s) {
   count_launch();
 }
 
+// mg_cor.F90:102-290 (k_prolong) with the boundary pass after it.
+constexpr int kRBProlongK = 4;
+template <int CD>
+__global__ void __launch_bounds__(128) k_rb_prolong(RBLevel L, DevLevel<double> F, DevLevel<double> C) {
+  const int col = blockIdx.x * 128 + threadIdx.x;
+  if (col >= L.nx * L.ny) return;
+  const int j = 2 + col / L.nx, i = 2 + col - (j - 2) * L.nx;
+  const int k0 = 2 + blockIdx.y * kRBProlongK;
+  const int64_t c0 = cidx(i, j, k0, L.X, L.XY), oy = rb_yshift(L, j);
+  double v[kRBProlongK];
+#pragma unroll
+  for (int u = 0; u < kRBProlongK; ++u)
+    if (k0 + u <= L.nz + 1) v[u] = L.phi[c0 + u * L.XY] + prolong_corr<double, CD>(C, i, j, k0 + u);
+#pragma unroll
+  for (int u = 0; u < kRBProlongK; ++u)
+    if (k0 + u <= L.nz + 1) rb_put(L, c0 + u * L.XY, i, oy, k0 + u, v[u]);
+}
+
+void launch_rb_prolong(const RBLevel& L, const DevLevel<double>& F, const DevLevel<double>& C, int cdir,
+                       cudaStream_t s) {
+  const dim3 g((unsigned)((L.nx * L.ny + 127) / 128), (unsigned)((L.nz + kRBProlongK - 1) / kRBProlongK));
+  switch (cdir & 7) {
+    case 0: k_rb_prolong<0><<<g, 128, 0, s>>>(L, F, C); break;
+    case 1: k_rb_prolong<1><<<g, 128, 0, s>>>(L, F, C); break;
+    case 2: k_rb_prolong<2><<<g, 128, 0, s>>>(L, F, C); break;
+    case 3: k_rb_prolong<3><<<g, 128, 0, s>>>(L, F, C); break;
+    case 4: k_rb_prolong<4><<<g, 128, 0, s>>>(L, F, C); break;
+    case 5: k_rb_prolong<5><<<g, 128, 0, s>>>(L, F, C); break;
+    case 6: k_rb_prolong<6><<<g, 128, 0, s>>>(L, F, C); break;
+    default: k_rb_prolong<7><<<g, 128, 0, s>>>(L, F, C); break;
+  }
+  count_launch();
+}
+
 // ---------------------------------------------------- coarse levels
 // The levels of at most kRBSharedCells cells and everything below them in
 // one block: their half-sweeps are 1000 to 4 cells long and as separate
-// launches cost 6 us each, about 80 of them per cycle.  phi and f stay in
-// shared memory (an 8192-cell level and its coarser ones take 212 KB);
-// boundary passes go by the ghost tables.
+// launches cost 6 us each, about 60 of them per cycle.  phi and f stay in
+// shared memory; boundary passes go by the ghost tables.  An 8192-cell
+// level fits too, but one SM takes longer over it than its launches
+// (256x128x128 solve: 39.1 ms with it, 34.3 without; 128x64x128 step with
+// the 2048-cell level 20.0, without 20.2).
 constexpr int kRBThreads = 512;
 
 __device__ __forceinline__ unsigned rb_magic(int d) { return (unsigned)((0x100000000ull + d - 1) / (unsigned)d); }
@@ -204,28 +246,36 @@ void launch_rb_shared(const RBShared& S, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------- stop test
-// mg_residual.F90:60-105.  A warp per row of x (ghost rows are copied only);
-// the maxima of non-negative doubles by their bit patterns, exact in any
-// order, one atomic pair per block.
-__global__ void __launch_bounds__(256) k_relmax_rows(DevLevel<double> L, const double* __restrict__ phin,
+// mg_residual.F90:60-105 over the whole ghosted array, four values per
+// thread loaded before the first is stored (ghosts are copied only); the
+// maxima of non-negative doubles by their bit patterns, exact in any order,
+// one atomic pair per block.  256x128x128: 66 us with one value at a time.
+constexpr int kMaxU = 4;
+__global__ void __launch_bounds__(256) k_relmax_copy(DevLevel<double> L, const double* __restrict__ phin,
                                                      double* __restrict__ phio, unsigned long long* out) {
   __shared__ unsigned long long sh[2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int rows = L.Y * L.Z;
   unsigned long long m1 = 0, m2 = 0;
-  for (int r = blockIdx.x * 8 + wid; r < rows; r += gridDim.x * 8) {
-    const int k = 1 + r / L.Y, j = 1 + r - (k - 1) * L.Y;
-    const bool in = j >= 2 && j <= L.ny + 1 && k >= 2 && k <= L.nz + 1;
-    const int64_t base = (int64_t)r * L.X;
-    for (int i = lane; i < L.X; i += 32) {
-      const double n = phin[base + i];
-      if (in && i >= 1 && i <= L.nx) {
-        const unsigned long long a = __double_as_longlong(fabs(n));
-        const unsigned long long d = __double_as_longlong(fabs(n - phio[base + i]));
+  for (int64_t t0 = (int64_t)blockIdx.x * 256 * kMaxU + threadIdx.x; t0 < L.G; t0 += (int64_t)gridDim.x * 256 * kMaxU) {
+    double n[kMaxU], o[kMaxU];
+#pragma unroll
+    for (int u = 0; u < kMaxU; ++u) {
+      const int64_t t = t0 + u * 256;
+      n[u] = t < L.G ? phin[t] : 0.0;
+      o[u] = t < L.G ? phio[t] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kMaxU; ++u) {
+      const int64_t t = t0 + u * 256;
+      if (t >= L.G) break;
+      phio[t] = n[u];
+      const int k = (int)(t / L.XY), r = (int)(t - k * L.XY), j = r / L.X, i = r - j * L.X;
+      if (i >= 1 && i <= L.nx && j >= 1 && j <= L.ny && k >= 1 && k <= L.nz) {
+        const unsigned long long a = __double_as_longlong(fabs(n[u]));
+        const unsigned long long d = __double_as_longlong(fabs(n[u] - o[u]));
         m1 = a > m1 ? a : m1;
         m2 = d > m2 ? d : m2;
       }
-      phio[base + i] = n;
     }
   }
   for (int o = 16; o > 0; o >>= 1) {
@@ -245,10 +295,10 @@ __global__ void __launch_bounds__(256) k_relmax_rows(DevLevel<double> L, const d
   }
 }
 
-void launch_relmax_rows(const DevLevel<double>& L, const double* phin, double* phio, unsigned long long* out,
+void launch_relmax_copy(const DevLevel<double>& L, const double* phin, double* phio, unsigned long long* out,
                         cudaStream_t s) {
-  const int64_t b = ((int64_t)L.Y * L.Z + 7) / 8;
-  k_relmax_rows<<<(unsigned)(b < 148 * 8 ? b : 148 * 8), 256, 0, s>>>(L, phin, phio, out);
+  const int64_t b = (L.G + 256 * kMaxU - 1) / (256 * kMaxU);
+  k_relmax_copy<<<(unsigned)(b < 148 * 8 ? b : 148 * 8), 256, 0, s>>>(L, phin, phio, out);
   count_launch();
 }
 

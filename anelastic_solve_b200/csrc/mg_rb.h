@@ -22,7 +22,7 @@ void launch_rb_march(const RBLevel& L, int color, cudaStream_t s);
 
 // Levels 1..lc of the cycle in one block, phi and f in shared memory.
 constexpr int kRBSharedLevels = 10;
-constexpr int kRBSharedCells = 8192;         // most interior cells of level lc
+constexpr int kRBSharedCells = 2048;         // most interior cells of level lc
 constexpr size_t kRBSharedBytes = 220 << 10;
 struct RBShared {
   int lc;
@@ -31,14 +31,17 @@ struct RBShared {
   int pre[kRBSharedLevels + 1], post[kRBSharedLevels + 1];
   int cd[kRBSharedLevels + 1];               // directions coarsened from l + 1 to l
 };
+// phi += the interpolated correction of the coarse level, ghosts included
+void launch_rb_prolong(const RBLevel& L, const DevLevel<double>& F, const DevLevel<double>& C, int cdir,
+                       cudaStream_t s);
 // shared memory of levels 1..lc
 size_t rb_shared_bytes(const RBShared& S);
 void rb_shared_prepare();
 // level lc's f from global memory, its corrected phi (ghosts too) to it
 void launch_rb_shared(const RBShared& S, cudaStream_t s);
 
-// max|phin|, max|phin - phio| over the interior and phio <- phin, by rows
-void launch_relmax_rows(const DevLevel<double>& L, const double* phin, double* phio, unsigned long long* out,
+// max|phin|, max|phin - phio| over the interior and phio <- phin on the whole array
+void launch_relmax_copy(const DevLevel<double>& L, const double* phin, double* phio, unsigned long long* out,
                         cudaStream_t s);
 
 }  // namespace anel

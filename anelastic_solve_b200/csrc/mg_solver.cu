@@ -1378,8 +1378,12 @@ void MGSolver::cycle64(cudaStream_t s) {
   for (int l = lc > 0 ? lc : 1; l <= ng - 1; ++l) {
     if (l > lc) relax64(l, post[l - 1], s);
     const DevLevel<double> F = L64(l + 1);
-    launch_prolong(F, L64(l), coarsen_dirs(l), s);
-    launch_bdry(F, F.phi, s);
+    if (rb_ok_[l + 1] && !any_ghosts_) {
+      launch_rb_prolong(rb_[l + 1], F, L64(l), coarsen_dirs(l), s);
+    } else {
+      launch_prolong(F, L64(l), coarsen_dirs(l), s);
+      launch_bdry(F, F.phi, s);
+    }
   }
   relax64(ng, post[ng - 1], s);
 }
@@ -1732,7 +1736,7 @@ int MGSolver::solve_fp64(double* d_phi, const double* d_rhs, cudaStream_t s,
       }
     } else {
       ANEL_CUDA_TRY(cudaMemsetAsync(d_max_, 0, 2 * sizeof(unsigned long long), s));
-      launch_relmax_rows(W, W.phi, d_phi, d_max_, s);
+      launch_relmax_copy(W, W.phi, d_phi, d_max_, s);
       copy_words(d_max_, h_pin_, 2, s);
       ANEL_CUDA_TRY(cudaStreamSynchronize(s));
       const double v1 = h_pin_[0], v2 = h_pin_[1];  // bit patterns of the maxima
