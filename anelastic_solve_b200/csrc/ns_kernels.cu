@@ -550,13 +550,29 @@ struct CNFac {
 };
 
 // The per-row factors and z metrics are staged in shared memory (stride
-// n+1 doubles each: ap, bp, c, t1, t2, rb, isbc, rdze, rdzc) and both
+// n+1 doubles each: ap, bp, c, t1, t2, rb, isbc, rdze, rdzc, 1/bp) and both
 // sweeps run in batches of kCNU rows whose global loads are issued before
 // any of the batch's stores, so a column costs n/kCNU memory latencies
 // instead of n.  The arithmetic and its order are those of the
 // row-by-row Thomas algorithm.
 constexpr int kCNU = 8;
 constexpr int kCNThreads = 256;
+
+// a / b, correctly rounded, from y = 1 / b rounded to nearest: two
+// corrections q <- q + (a - b q) y.  The first makes q faithful, and then the
+// second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990);
+// outside the exponents where no step can over- or underflow (for which y is
+// NaN where |b| is not within 2^-100..2^100), and for zero, infinite and NaN
+// quotients, the division itself.  b is a row's eliminated
+// diagonal, the same for every column, so its reciprocal is formed once per
+// block, and the back substitution's chain of divisions is half as long.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+  const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
+  const unsigned e = (unsigned)(__double2hiint(q0) >> 20) & 0x7ffu;
+  return e - 200u < 1600u ? q2 : a / b;
+}
 
 // U rows per batch: with the columns per block, the launch variants the
 // autotuner chooses from (launch_cn); the arithmetic does not depend on
@@ -576,10 +592,13 @@ __device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ f
   double* s_bc = s_rb + S;
   double* s_re = s_bc + S;  // rdze
   double* s_rc = s_re + S;  // rdzc
+  double* s_y = s_rc + S;   // 1 / bp
   for (int r = threadIdx.x; r < S; r += blockDim.x) {
     const bool in = r < n;
     s_ap[r] = in ? F.ap[r] : 0.0;
     s_bp[r] = in ? F.bp[r] : 1.0;
+    const unsigned eb = (unsigned)(__double2hiint(s_bp[r]) >> 20) & 0x7ffu;
+    s_y[r] = eb - 923u <= 200u ? 1.0 / s_bp[r] : __longlong_as_double(0x7ff8000000000000LL);
     s_c[r] = in ? F.c[r] : 0.0;
     s_t1[r] = in ? F.t1[r] : 0.0;
     s_t2[r] = in ? F.t2[r] : 0.0;
@@ -649,7 +668,7 @@ __device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ f
     for (int u = 0; u < U; ++u) {
       const int k = kb - u;
       if (k >= 1) {
-        gn = (gv[u] - s_c[k - 1] * gn) / s_bp[k - 1];
+        gn = div_by(gv[u] - s_c[k - 1] * gn, s_bp[k - 1], s_y[k - 1]);
         fld[base + (int64_t)(k - 1) * XY] = gn;
       }
     }
@@ -1404,7 +1423,7 @@ template <int U, int TPB, int N>
 static void cn_launch(const NSMany<N>& P, const CNJobs<N>& J, int members, double a3, const NSScal<N>& rkdt,
                       cudaStream_t s) {
   const NSDev& D = P.d[0];
-  const size_t sm = 9 * (size_t)(D.nz + 3) * sizeof(double);
+  const size_t sm = 10 * (size_t)(D.nz + 3) * sizeof(double);
   set_smem_limit_once((const void*)k_cn_column<U, TPB, N>, 200 * 1024);
   dim3 g = col_grid(D, TPB);
   g.z = (unsigned)(J.n * members);
