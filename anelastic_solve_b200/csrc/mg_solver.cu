@@ -260,7 +260,8 @@ int MGSolver::init(const anel_grid_desc* g, const anel_mg_params* p, int device)
   if (col_) npart = std::max(npart, col_resid_part_doubles(L64(ngrid_)));
   ANEL_CUDA_TRY(cudaMalloc(&d_part_, (size_t)npart * sizeof(double)));
   ANEL_CUDA_TRY(cudaMalloc(&d_norm_, 2 * sizeof(double)));
-  ANEL_CUDA_TRY(cudaHostAlloc(&h_pin_, 4 * sizeof(double), cudaHostAllocMapped));
+  // 4 doubles of small readbacks, then the direct solve's state
+  ANEL_CUDA_TRY(cudaHostAlloc(&h_pin_, 4 * sizeof(double) + sizeof(SpecState), cudaHostAllocMapped));
   choose_direct_level();
   {
     // The direct fine-level solve is the faster correction at every size
@@ -1209,8 +1210,8 @@ int MGSolver::build_spec() {
   for (int j = G.s[1]; j <= G.e[1]; ++j)
     if (!(c.cy3[j - 1] == a3 && c.cy4[j - 1] == a3)) return ANEL_OK;
   const double* coef = d_coef64_[ngrid_] + 2 * (size_t)G.X + 2 * (size_t)G.Y;
-  return spec_build(spec_, G.n[0], G.n[1], G.n[2], a1, a3, c.cz5.data(), c.cz6.data(), c.dz5.data(), c.dz6.data(),
-                    prm_.tbc[1] == 1, prm_.tbc[3] == 1, coef);
+  return spec_build(spec_, reinterpret_cast<SpecState*>(h_pin_ + 4), G.n[0], G.n[1], G.n[2], a1, a3, c.cz5.data(),
+                    c.cz6.data(), c.dz5.data(), c.dz6.data(), prm_.tbc[1] == 1, prm_.tbc[3] == 1, coef);
 }
 
 int MGSolver::set_density_host(const double* r) {

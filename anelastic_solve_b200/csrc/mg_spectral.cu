@@ -557,7 +557,7 @@ static void z_kernel(int M, F f) {
   }
 }
 
-int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const double* cz5, const double* cz6,
+int spec_build(SpecHost& H, SpecState* h_one, int nx, int ny, int nz, double a1, double a3, const double* cz5, const double* cz6,
                const double* dz5, const double* dz6, int z1, int zZ, const double* coef) {
   SpecDev& D = H.d;
   H.ok = false;
@@ -664,6 +664,7 @@ int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const 
     y_kernel(inv, y_cols(D), [&](auto* k) { set_smem_limit_once((const void*)k, (int)y_smem(D)); });
   z_kernel(D.M, [&](auto* k) { set_smem_limit_once((const void*)k, (int)z_smem(D)); });
   ANEL_CUDA_TRY(cudaGetLastError());
+  H.h_one = h_one;
   const int st = spec_reserve(H, 1);
   if (st != ANEL_OK) return st;
   H.ok = true;
@@ -673,36 +674,31 @@ int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const 
 int spec_reserve(SpecHost& H, int n) {
   SpecDev& D = H.d;
   if (n <= H.cap) return ANEL_OK;
-  cudaFree(H.d_part);
-  cudaFree(H.d_st);
-  cudaFree(H.d_count);
-  if (H.h_st) cudaFreeHost(H.h_st);
-  H.d_part = nullptr;
-  H.d_st = H.h_st = nullptr;
-  H.d_count = nullptr;
+  cudaFree(H.d_buf);
+  H.d_buf = nullptr;
+  if (H.h_st && H.h_st != H.h_one) cudaFreeHost(H.h_st);
+  H.h_st = nullptr;
   H.cap = 0;
   const int64_t fwd = (int64_t)((D.ny / 2 + D.pairs - 1) / D.pairs) * D.nz;
   D.pstride = 2 * std::max<int64_t>(fwd, (int64_t)check_cols(D) * check_zblocks(D));
-  ANEL_CUDA_TRY(cudaMalloc(&H.d_part, (size_t)n * D.pstride * sizeof(double)));
-  ANEL_CUDA_TRY(cudaMalloc(&H.d_st, (size_t)n * sizeof(SpecState)));
-  ANEL_CUDA_TRY(cudaMalloc(&H.d_count, (size_t)n * sizeof(unsigned)));
-  ANEL_CUDA_TRY(cudaMemset(H.d_st, 0, (size_t)n * sizeof(SpecState)));
-  ANEL_CUDA_TRY(cudaMemset(H.d_count, 0, (size_t)n * sizeof(unsigned)));
-  ANEL_CUDA_TRY(cudaHostAlloc(&H.h_st, (size_t)n * sizeof(SpecState), cudaHostAllocMapped));
-  ANEL_CUDA_TRY(cudaHostGetDevicePointer((void**)&D.hst, H.h_st, 0));
-  D.part = H.d_part;
-  D.st = H.d_st;
-  D.count = H.d_count;
+  const size_t st = (size_t)n * sizeof(SpecState), cnt = ((size_t)n * sizeof(unsigned) + 15) / 16 * 16;
+  ANEL_CUDA_TRY(cudaMalloc(&H.d_buf, st + cnt + (size_t)n * D.pstride * sizeof(double)));
+  ANEL_CUDA_TRY(cudaMemset(H.d_buf, 0, st + cnt));
+  if (n == 1) H.h_st = H.h_one;
+  else ANEL_CUDA_TRY(cudaHostAlloc(&H.h_st, (size_t)n * sizeof(SpecState), cudaHostAllocMapped));
+  D.hst = H.h_st;
+  char* p = reinterpret_cast<char*>(H.d_buf);
+  D.st = reinterpret_cast<SpecState*>(p);
+  D.count = reinterpret_cast<unsigned*>(p + st);
+  D.part = reinterpret_cast<double*>(p + st + cnt);
   H.cap = n;
   return ANEL_OK;
 }
 
 void spec_free(SpecHost& H) {
   cudaFree(H.d_tab);
-  cudaFree(H.d_part);
-  cudaFree(H.d_st);
-  cudaFree(H.d_count);
-  if (H.h_st) cudaFreeHost(H.h_st);
+  cudaFree(H.d_buf);
+  if (H.h_st && H.h_st != H.h_one) cudaFreeHost(H.h_st);
   H = SpecHost{};
 }
 

@@ -10,10 +10,9 @@ namespace anel {
 struct SpecHost {
   SpecDev d{};
   double* d_tab = nullptr;    // twiddles, eigenvalues, z tables
-  double* d_part = nullptr;   // partial sums
-  SpecState* d_st = nullptr;
-  SpecState* h_st = nullptr;  // mapped
-  unsigned* d_count = nullptr;
+  double* d_buf = nullptr;    // states, arrival counters, partial sums
+  SpecState* h_st = nullptr;  // the states' mirror, mapped
+  SpecState* h_one = nullptr; // the caller's mapped memory for one member
   int cap = 0;                // members the buffers above have room for
   bool ok = false;
 };
@@ -23,7 +22,8 @@ bool spec_supported(int nx, int ny, int nz);
 // Tables of a fine level with line coefficients a1 (x), a3 (y), z
 // coefficients indexed k-1 and homogeneous z-ghosts z1/zZ (1: copy of the
 // adjacent row, 0: zero).  coef: the level's device cz5[Z] cz6[Z] dz5[Z] dz6[Z].
-int spec_build(SpecHost& H, int nx, int ny, int nz, double a1, double a3, const double* cz5, const double* cz6,
+// h_one: mapped host memory for one member's state.
+int spec_build(SpecHost& H, SpecState* h_one, int nx, int ny, int nz, double a1, double a3, const double* cz5, const double* cz6,
                const double* dz5, const double* dz6, int z1, int zZ, const double* coef);
 void spec_free(SpecHost& H);
 // buffers for n members
