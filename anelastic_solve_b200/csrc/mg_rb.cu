@@ -2,6 +2,7 @@
 // levels.  Compiled with -fmad=false: every value is rounded as in
 // k_rb_sweep, k_restrict and k_prolong, whose expressions these are.
 #include "mg_rb.h"
+#include "pdl.cuh"
 
 namespace anel {
 
@@ -32,6 +33,7 @@ __device__ __forceinline__ int64_t rb_yshift(const RBLevel& L, int j) {
 // launches before.
 template <int U>
 __global__ void __launch_bounds__(128) k_rb_march(RBLevel L, int color) {
+  chain_enter();
   const int hx = L.nx >> 1;
   const int col = blockIdx.x * 128 + threadIdx.x;
   if (col >= hx * L.ny) return;
@@ -69,9 +71,9 @@ void launch_rb_march(const RBLevel& L, int color, cudaStream_t s) {
   const int cols = ((L.nx / 2) * L.ny + 127) / 128;
   // four planes per thread where that still gives two blocks per SM
   if ((int64_t)cols * ((L.nz + 3) / 4) >= 2 * 148)
-    k_rb_march<4><<<dim3((unsigned)cols, (unsigned)((L.nz + 3) / 4)), 128, 0, s>>>(L, color);
+    launch_chained(k_rb_march<4>, dim3((unsigned)cols, (unsigned)((L.nz + 3) / 4)), 128, 0, s, L, color);
   else
-    k_rb_march<1><<<dim3((unsigned)cols, (unsigned)L.nz), 128, 0, s>>>(L, color);
+    launch_chained(k_rb_march<1>, dim3((unsigned)cols, (unsigned)L.nz), 128, 0, s, L, color);
   count_launch();
 }
 
@@ -79,6 +81,7 @@ void launch_rb_march(const RBLevel& L, int color, cudaStream_t s) {
 constexpr int kRBProlongK = 4;
 template <int CD>
 __global__ void __launch_bounds__(128) k_rb_prolong(RBLevel L, DevLevel<double> F, DevLevel<double> C) {
+  chain_enter();
   const int col = blockIdx.x * 128 + threadIdx.x;
   if (col >= L.nx * L.ny) return;
   const int j = 2 + col / L.nx, i = 2 + col - (j - 2) * L.nx;
@@ -97,14 +100,14 @@ void launch_rb_prolong(const RBLevel& L, const DevLevel<double>& F, const DevLev
                        cudaStream_t s) {
   const dim3 g((unsigned)((L.nx * L.ny + 127) / 128), (unsigned)((L.nz + kRBProlongK - 1) / kRBProlongK));
   switch (cdir & 7) {
-    case 0: k_rb_prolong<0><<<g, 128, 0, s>>>(L, F, C); break;
-    case 1: k_rb_prolong<1><<<g, 128, 0, s>>>(L, F, C); break;
-    case 2: k_rb_prolong<2><<<g, 128, 0, s>>>(L, F, C); break;
-    case 3: k_rb_prolong<3><<<g, 128, 0, s>>>(L, F, C); break;
-    case 4: k_rb_prolong<4><<<g, 128, 0, s>>>(L, F, C); break;
-    case 5: k_rb_prolong<5><<<g, 128, 0, s>>>(L, F, C); break;
-    case 6: k_rb_prolong<6><<<g, 128, 0, s>>>(L, F, C); break;
-    default: k_rb_prolong<7><<<g, 128, 0, s>>>(L, F, C); break;
+    case 0: launch_chained(k_rb_prolong<0>, g, 128, 0, s, L, F, C); break;
+    case 1: launch_chained(k_rb_prolong<1>, g, 128, 0, s, L, F, C); break;
+    case 2: launch_chained(k_rb_prolong<2>, g, 128, 0, s, L, F, C); break;
+    case 3: launch_chained(k_rb_prolong<3>, g, 128, 0, s, L, F, C); break;
+    case 4: launch_chained(k_rb_prolong<4>, g, 128, 0, s, L, F, C); break;
+    case 5: launch_chained(k_rb_prolong<5>, g, 128, 0, s, L, F, C); break;
+    case 6: launch_chained(k_rb_prolong<6>, g, 128, 0, s, L, F, C); break;
+    default: launch_chained(k_rb_prolong<7>, g, 128, 0, s, L, F, C); break;
   }
   count_launch();
 }
@@ -189,6 +192,7 @@ __device__ __forceinline__ void rb_prolong(const DevLevel<double> F, const DevLe
 __host__ __device__ inline int rb_coefs(int X, int Y, int Z) { return 2 * X + 2 * Y + 4 * Z; }
 
 __global__ void __launch_bounds__(kRBThreads) k_rb_shared(const __grid_constant__ RBShared S) {
+  chain_enter();
   extern __shared__ double rsm[];
   __shared__ DevLevel<double> lv[kRBSharedLevels + 1];
   if (threadIdx.x == 0) {
@@ -241,7 +245,7 @@ size_t rb_shared_bytes(const RBShared& S) {
 void rb_shared_prepare() { set_smem_limit_once((const void*)k_rb_shared, (int)kRBSharedBytes); }
 
 void launch_rb_shared(const RBShared& S, cudaStream_t s) {
-  k_rb_shared<<<1, kRBThreads, rb_shared_bytes(S), s>>>(S);
+  launch_chained(k_rb_shared, 1, kRBThreads, rb_shared_bytes(S), s, S);
   count_launch();
 }
 
@@ -253,6 +257,7 @@ void launch_rb_shared(const RBShared& S, cudaStream_t s) {
 constexpr int kMaxU = 4;
 __global__ void __launch_bounds__(256) k_relmax_copy(DevLevel<double> L, const double* __restrict__ phin,
                                                      double* __restrict__ phio, unsigned long long* out) {
+  chain_enter();
   __shared__ unsigned long long sh[2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   unsigned long long m1 = 0, m2 = 0;
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(256) k_relmax_copy(DevLevel<double> L, const d
 void launch_relmax_copy(const DevLevel<double>& L, const double* phin, double* phio, unsigned long long* out,
                         cudaStream_t s) {
   const int64_t b = (L.G + 256 * kMaxU - 1) / (256 * kMaxU);
-  k_relmax_copy<<<(unsigned)(b < 148 * 8 ? b : 148 * 8), 256, 0, s>>>(L, phin, phio, out);
+  launch_chained(k_relmax_copy, (unsigned)(b < 148 * 8 ? b : 148 * 8), 256, 0, s, L, phin, phio, out);
   count_launch();
 }
 

@@ -6,6 +6,7 @@
 #include <cmath>
 
 #include "mg_launch.h"
+#include "pdl.cuh"
 
 namespace anel {
 
@@ -95,6 +96,7 @@ __device__ __forceinline__ double spec_resid(const SpecDev& D, const double* __r
 // Residual of row pairs (j, j+1) of plane k, the two rows as the real and
 // imaginary part of one transform of length nx, then the rows' own modes.
 __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
+  chain_enter();
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!test && !D.st[b].act) return;  // the whole block
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
 // Inverse x transform of row pairs and phi += e.  The inverse transform is
 // the forward one with real and imaginary parts exchanged before and after.
 __global__ void __launch_bounds__(256, 3) k_spec_update(SpecDev D) {
+  chain_enter();
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!D.st[b].act) return;
@@ -199,6 +202,7 @@ __global__ void __launch_bounds__(256, 3) k_spec_update(SpecDev D) {
 // y transform of W columns of a plane, in place.
 template <bool kInv, int W>
 __global__ void __launch_bounds__(256, 3) k_spec_y(SpecDev D) {
+  chain_enter();
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!D.st[b].act) return;
@@ -266,6 +270,7 @@ __device__ __forceinline__ double spec_rcp(double x) {
 // ny/2: one component each.
 template <int M>
 __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
+  chain_enter();
   extern __shared__ double zsm[];
   const int b = blockIdx.y;
   if (!D.st[b].act) return;
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
 // flat columns at 512x256x512).
 constexpr int kCheckK = 4;
 __global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int per, int nzb) {
+  chain_enter();
   const int b = blockIdx.z / nzb;
   if (!D.st[b].act) return;
   const double* __restrict__ phi = D.mt ? D.mt[b].phi : D.phi;
@@ -712,35 +718,35 @@ static int y_threads(const SpecDev& D) {
 
 void launch_spec_forward(const SpecDev& D, int nm, bool test, cudaStream_t s) {
   const dim3 g((unsigned)((D.ny / 2 + D.pairs - 1) / D.pairs), (unsigned)D.nz, (unsigned)nm);
-  k_spec_forward<<<g, x_threads(D), x_smem(D), s>>>(D, test ? 1 : 0);
+  launch_chained(k_spec_forward, g, x_threads(D), x_smem(D), s, D, test ? 1 : 0);
   count_launch();
 }
 
 void launch_spec_y(const SpecDev& D, int nm, bool inverse, cudaStream_t s) {
   const int cols = y_cols(D);
   const dim3 g((unsigned)((D.nxh + cols - 1) / cols), (unsigned)D.nz, (unsigned)nm);
-  y_kernel(inverse, cols, [&](auto* k) { k<<<g, y_threads(D), y_smem(D), s>>>(D); });
+  y_kernel(inverse, cols, [&](auto* k) { launch_chained(k, g, y_threads(D), y_smem(D), s, D); });
   count_launch();
 }
 
 void launch_spec_z(const SpecDev& D, int nm, cudaStream_t s) {
   const int ntiles = (int)((D.nu + 7) / 8) + 1;
   z_kernel(D.M, [&](auto* k) {
-    k<<<dim3((unsigned)std::min(ntiles, 148 * 2), (unsigned)nm), 8 * D.S, z_smem(D), s>>>(D, ntiles);
+    launch_chained(k, dim3((unsigned)std::min(ntiles, 148 * 2), (unsigned)nm), 8 * D.S, z_smem(D), s, D, ntiles);
   });
   count_launch();
 }
 
 void launch_spec_update(const SpecDev& D, int nm, cudaStream_t s) {
   const dim3 g((unsigned)((D.ny / 2 + D.pairs - 1) / D.pairs), (unsigned)D.nz, (unsigned)nm);
-  k_spec_update<<<g, x_threads(D), x_smem(D), s>>>(D);
+  launch_chained(k_spec_update, g, x_threads(D), x_smem(D), s, D);
   count_launch();
 }
 
 void launch_spec_check(const SpecDev& D, int nm, cudaStream_t s) {
   const int nzb = check_zblocks(D);
   const dim3 g((unsigned)((D.nx + 31) / 32), (unsigned)((D.ny + 7) / 8), (unsigned)(nzb * nm));
-  k_spec_check<<<g, 256, 0, s>>>(D, check_planes(D), nzb);
+  launch_chained(k_spec_check, g, 256, 0, s, D, check_planes(D), nzb);
   count_launch();
 }
 

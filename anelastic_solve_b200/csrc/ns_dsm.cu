@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "ns_solver.h"
+#include "pdl.cuh"
 
 namespace anel {
 
@@ -35,6 +36,7 @@ dim3 interior_grid(const NSDev& D) {
 
 __global__ void k_dyn_modS(NSDev D, const double* __restrict__ l1, const double* __restrict__ l2,
                            const double* __restrict__ l3, double* __restrict__ out) {
+  chain_enter();
   DYN_CELL();
   out[o] = strain_mag(D, l1, l2, l3, i, j, k);
 }
@@ -43,6 +45,7 @@ __global__ void k_dyn_modS(NSDev D, const double* __restrict__ l1, const double*
 // for ij = 4..6 half the difference of the two cross derivatives (the
 // source subtracts where straincal adds).
 __global__ void k_dyn_comp(NSDev D, int ij, double* __restrict__ out) {
+  chain_enter();
   DYN_CELL();
   const double *l1 = D.u, *l2 = D.v, *l3 = D.w;
   double r, t1, t2, t3, t4;
@@ -169,6 +172,7 @@ struct DynFilt {
 template <int NF, class In, class Out>
 __global__ void __launch_bounds__(kDynI * kDynJ) k_dyn_filter(const __grid_constant__ NSDev D, In in, Out out, DynZ R,
                                                               DynFilt Q) {
+  chain_enter();
   __shared__ double sm[2][NF][kDynTile];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int i0 = 2 + blockIdx.x * kDynI, j0 = 2 + blockIdx.y * kDynJ, k0 = 2 + blockIdx.z * Q.per;
@@ -350,7 +354,7 @@ void launch_dyn_filter(const NSDev& D, const In& in, const Out& out, const DynZ&
   DynFilt Q{filt[0], filt[1], filt[2], 32};
   while (Q.per > 4 && (int64_t)g.x * g.y * ((D.nz + Q.per - 1) / Q.per) < 4 * 148) Q.per /= 2;
   g.z = (unsigned)((D.nz + Q.per - 1) / Q.per);
-  k_dyn_filter<NF, In, Out><<<g, kDynI * kDynJ, 0, s>>>(D, in, out, R, Q);
+  launch_chained(k_dyn_filter<NF, In, Out>, g, kDynI * kDynJ, 0, s, D, in, out, R, Q);
   count_launch();
 }
 
@@ -452,6 +456,7 @@ __global__ void k_dyn_column(NSDev D, const double* __restrict__ a, double* __re
 __global__ void __launch_bounds__(256) k_dyn_ratio(NSDev D, const double* __restrict__ pn,
                                                    const double* __restrict__ pd, int nb, double area, DynZ R,
                                                    double* __restrict__ prof) {
+  chain_enter();
   extern __shared__ double sr[];
   const int nz = D.nz;
   for (int k = 2 + threadIdx.x; k <= nz + 1; k += blockDim.x) {
@@ -612,7 +617,7 @@ int NSSolver::dyn_prepare(cudaStream_t s) {
   double* modS = F + (size_t)DY_MODS * G_;
   double* fmodS = F + (size_t)DY_FMODS * G_;
   double *l1 = F + (size_t)DY_L1 * G_, *l2 = F + (size_t)DY_L2 * G_, *l3 = F + (size_t)DY_L3 * G_;
-  k_dyn_modS<<<g, 128, 0, s>>>(D_, D_.u, D_.v, D_.w, modS);
+  launch_chained(k_dyn_modS, g, 128, 0, s, D_, D_.u, D_.v, D_.w, modS);
   count_launch();
   // the fused models read the interior of these fields only
   const bool fused = dyn_fusable(zrule(NV_CFLUC));
@@ -620,7 +625,7 @@ int NSSolver::dyn_prepare(cudaStream_t s) {
   dyn_filter(D_.u, l1, NV_U, 0, s);
   dyn_filter(D_.v, l2, NV_V, 0, s);
   dyn_filter(D_.w, l3, NV_W, 0, s);
-  k_dyn_modS<<<g, 128, 0, s>>>(D_, l1, l2, l3, fmodS);
+  launch_chained(k_dyn_modS, g, 128, 0, s, D_, l1, l2, l3, fmodS);
   count_launch();
   if (!fused) launch_ghost_field(D_, fmodS, zrule(NV_CFLUC), s);
   const double* vel[3] = {D_.u, D_.v, D_.w};
@@ -684,7 +689,7 @@ int NSSolver::dyn_coefficient(const double* num, const double* den, double* host
   double* pd = dyn_part_ + plane_part_doubles(D_);
   const int nb = launch_plane_part(D_, num, dxc, dyc, dyn_part_, s);
   launch_plane_part(D_, den, dxc, dyc, pd, s);
-  k_dyn_ratio<<<1, 256, Z * sizeof(double), s>>>(D_, dyn_part_, pd, nb, dyn_area_, dyn_z(zrule(NV_CFLUC)), pr);
+  launch_chained(k_dyn_ratio, 1, 256, Z * sizeof(double), s, D_, dyn_part_, pd, nb, dyn_area_, dyn_z(zrule(NV_CFLUC)), pr);
   count_launch();
   ANEL_CUDA_TRY(cudaGetLastError());
   ANEL_CUDA_TRY(cudaMemcpyAsync(host, pr, Z * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -704,7 +709,7 @@ int NSSolver::dsm_velocity(cudaStream_t s, double* cs) {
     const double *modS = F + (size_t)DY_MODS * G_, *fmodS = F + (size_t)DY_FMODS * G_;
     static const int qa[7] = {0, 0, 1, 2, 0, 0, 1}, qb[7] = {0, 0, 1, 2, 1, 2, 2};
     for (int ij = 1; ij <= 6; ++ij) {
-      k_dyn_comp<<<interior_grid(D_), 128, 0, s>>>(D_, ij, l1);
+      launch_chained(k_dyn_comp, interior_grid(D_), 128, 0, s, D_, ij, l1);
       count_launch();
       const DsmIn in{l1, modS, F + (size_t)(DY_C0 + qa[ij]) * G_, F + (size_t)(DY_C0 + qb[ij]) * G_, dg};
       const DsmOut out{fmodS, F + (size_t)(DY_FC0 + qa[ij]) * G_, F + (size_t)(DY_FC0 + qb[ij]) * G_, dg, l4, C,
@@ -724,7 +729,7 @@ int NSSolver::dsm_velocity(cudaStream_t s, double* cs) {
   ANEL_CUDA_TRY(cudaMemsetAsync(C, 0, G_ * sizeof(double), s));
   static const int pa[7] = {0, 0, 1, 2, 0, 0, 1}, pb[7] = {0, 0, 1, 2, 1, 2, 2};
   for (int ij = 1; ij <= 6; ++ij) {
-    k_dyn_comp<<<g, 128, 0, s>>>(D_, ij, l1);
+    launch_chained(k_dyn_comp, g, 128, 0, s, D_, ij, l1);
     count_launch();
     launch_ghost_field(D_, l1, cf, s);
     k_dyn_scale<<<g, 128, 0, s>>>(D_, SC_A, l2, l1, modS, dg, 0.0);

@@ -2,6 +2,7 @@
 // -fmad=false: every sum/product is rounded as the reference's Fortran
 // expressions evaluated left to right (citations per kernel).
 #include "ns_launch.h"
+#include "pdl.cuh"
 
 #include <type_traits>
 
@@ -323,6 +324,7 @@ template <bool kFirst, bool kU, bool kL, int N>
 __global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(const __grid_constant__ NSMany<N> P, double a1,
                                                                 double a2, const __grid_constant__ NSScal<N> dts,
                                                                 int per, int zb) {
+  chain_enter();
   extern __shared__ double sm[];
   const int m_ = N > 1 ? blockIdx.z / zb : 0;
   const NSDev& D = P.d[m_];
@@ -475,6 +477,7 @@ __device__ __forceinline__ void ring_column(int t, int nx, int ny, int& di, int&
 }
 
 __global__ void k_images(NSDev D, ImageFields F) {
+  chain_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * D.ny + 2 * D.nx + 4) return;
   const int k = 1 + blockIdx.y;
@@ -504,6 +507,7 @@ struct GhostFields {  // n fields of each member; the rules are the members' com
 template <int N>
 __global__ void __launch_bounds__(128) k_ghost_images(const __grid_constant__ NSMany<N> P,
                                                       const __grid_constant__ GhostFields<N> F, int nba) {
+  chain_enter();
   const int m = N > 1 ? blockIdx.y / F.n : 0;
   const NSDev& D = P.d[m];
   double* a = F.a[blockIdx.y];
@@ -699,6 +703,7 @@ template <int U, int TPB, int N>
 __global__ void __launch_bounds__(TPB) k_cn_column(const __grid_constant__ NSMany<N> P,
                                                    const __grid_constant__ CNJobs<N> J, double a3,
                                                    const __grid_constant__ NSScal<N> rkdts) {
+  chain_enter();
   const int m = N > 1 ? blockIdx.z / J.n : 0;
   const NSDev& D = P.d[m];
   const double rkdt = rkdts.v[m];
@@ -934,6 +939,7 @@ __device__ __forceinline__ void cn_column_les(const NSDev& D, double* __restrict
 
 template <bool kU, int U, int TPB>
 __global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, CNJobs<1> J, double a3, double rkdt) {
+  chain_enter();
   const CNJob& c = J.j[blockIdx.z];
   switch (c.var) {
     case 1: cn_column_les<1, kU, U>(D, c.fld, c.q, c.F, a3, rkdt, c.R, c.kT, c.b); break;
@@ -949,6 +955,7 @@ __global__ void __launch_bounds__(TPB) k_cn_column_les(NSDev D, CNJobs<1> J, dou
 // (:48-73) on the interior: nuT = -(Csgs + 0) delg^2 |S| + 0 and the same
 // with CTsgs (kappaT) and CSsgs (nappaT); x**2.d0 is x*x.
 __global__ void __launch_bounds__(kCellCols) k_sgs(NSDev D, int per) {
+  chain_enter();
   CELL_COLUMN();
   for (int k = k0; k < kend; ++k) {
     const double modS = strain_mag(D, D.u, D.v, D.w, i, j, k);
@@ -990,6 +997,7 @@ __global__ void k_clip(NSDev D, double* a, double vmin, double vmax) {
 template <int N>
 __global__ void __launch_bounds__(kCellCols) k_psource(const __grid_constant__ NSMany<N> P,
                                                        const __grid_constant__ NSScal<N> rdts, int per) {
+  chain_enter();
   const NSDev& D = P.d[N > 1 ? blockIdx.z : 0];
   const double rdt = rdts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
@@ -1016,6 +1024,7 @@ template <bool kU, int N>
 __global__ void __launch_bounds__(kCellCols) k_pgrad(const __grid_constant__ NSMany<N> P,
                                                      const __grid_constant__ NSScal<N> dts,
                                                      double* __restrict__ hist, int per) {
+  chain_enter();
   const NSDev& D = P.d[N > 1 ? blockIdx.z : 0];
   const double dt = dts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
@@ -1092,6 +1101,7 @@ struct DivOut {
 template <int N>
 __global__ void __launch_bounds__(128) k_divergence(const __grid_constant__ NSMany<N> P,
                                                     const __grid_constant__ DivOut<N> O, int cfl, int zb) {
+  chain_enter();
   __shared__ double sh[2][4];
   __shared__ unsigned long long shm[2][4];
   __shared__ int last;
@@ -1207,6 +1217,7 @@ struct CNFactorJobs {
 template <int N>
 __global__ void __launch_bounds__(128) k_cn_factors(const __grid_constant__ NSMany<N> P,
                                                     const __grid_constant__ CNFactorJobs<N> J, int slot0) {
+  chain_enter();
   extern __shared__ double cn_sm[];
   const int me = N > 1 ? blockIdx.z : 0;
   const NSDev& D = P.d[me];
@@ -1309,7 +1320,7 @@ __global__ void __launch_bounds__(128) k_cn_factors(const __grid_constant__ NSMa
 // ------------------------------------------------------------ launchers
 static void launch_images(const NSDev& D, const ImageFields& F, int n, cudaStream_t s) {
   const int ring = 2 * D.ny + 2 * D.nx + 4;
-  k_images<<<dim3((unsigned)((ring + 127) / 128), (unsigned)D.Z, (unsigned)n), 128, 0, s>>>(D, F);
+  launch_chained(k_images, dim3((unsigned)((ring + 127) / 128), (unsigned)D.Z, (unsigned)n), 128, 0, s, D, F);
   count_launch();
 }
 
@@ -1319,7 +1330,7 @@ static void launch_ghost_images(const NSMany<N>& P, const GhostFields<N>& F, int
   const int nba = (D.nx * D.ny + 127) / 128;
   const int64_t copies = D.nz > 2 ? (int64_t)(2 * D.ny + 2 * D.nx + 4) * (D.nz - 2) : 0;
   const dim3 g((unsigned)(nba + (copies + 127) / 128), (unsigned)(F.n * members));
-  k_ghost_images<N><<<g, 128, 0, s>>>(P, F, nba);
+  launch_chained(k_ghost_images<N>, g, 128, 0, s, P, F, nba);
   count_launch();
 }
 
@@ -1375,7 +1386,7 @@ static void rhs_launch(const NSMany<N>& P, const NSScal<N>& dt, int members, dou
   g.z = (unsigned)(zb * members);
   const size_t sm = rhs_smem_bytes(kL);
   if (kL) set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL, N>, (int)sm);
-  k_rhs_accum<kFirst, kU, kL, N><<<g, kRT_I * kRT_J, sm, s>>>(P, a1, a2, dt, per, zb);
+  launch_chained(k_rhs_accum<kFirst, kU, kL, N>, g, kRT_I * kRT_J, sm, s, P, a1, a2, dt, per, zb);
 }
 
 void launch_rhs_accum(const NSDev* const* Ds, const double* dts, int n, double a1, double a2, bool first,
@@ -1427,7 +1438,7 @@ static void cn_launch(const NSMany<N>& P, const CNJobs<N>& J, int members, doubl
   set_smem_limit_once((const void*)k_cn_column<U, TPB, N>, 200 * 1024);
   dim3 g = col_grid(D, TPB);
   g.z = (unsigned)(J.n * members);
-  k_cn_column<U, TPB, N><<<g, TPB, sm, s>>>(P, J, a3, rkdt);
+  launch_chained(k_cn_column<U, TPB, N>, g, TPB, sm, s, P, J, a3, rkdt);
 }
 
 void launch_cn(const NSDev* const* Ds, const CNSet* set, int nset, const double* rkdts, int n, double a3, int variant,
@@ -1455,7 +1466,7 @@ static void cn_les_launch(const NSDev& D, const CNJobs<1>& J, double a3, double 
   set_smem_limit_once((const void*)k_cn_column_les<kU, U, TPB>, 200 * 1024);
   dim3 g = col_grid(D, TPB);
   g.z = (unsigned)J.n;
-  k_cn_column_les<kU, U, TPB><<<g, TPB, sm, s>>>(D, J, a3, rkdt);
+  launch_chained(k_cn_column_les<kU, U, TPB>, g, TPB, sm, s, D, J, a3, rkdt);
 }
 
 template <bool kU>
@@ -1480,7 +1491,7 @@ void launch_cn_les(const NSDev& D, const CNSet* set, int n, double a3, double rk
 void launch_sgs(const NSDev& D, const ZRule& cfluc, cudaStream_t s) {
   int per;
   const dim3 g = cell_grid_k(D, &per);
-  k_sgs<<<g, kCellCols, 0, s>>>(D, per);
+  launch_chained(k_sgs, g, kCellCols, 0, s, D, per);
   count_launch();
   launch_ghost_images<1>({D}, {{D.nuT, D.kT, D.nT}, {cfluc, cfluc, cfluc}, 3}, 1, s);
 }
@@ -1561,6 +1572,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_plane_part(NSDev D, const dou
                                                              const double* __restrict__ wx,
                                                              const double* __restrict__ wy,
                                                              double* __restrict__ part) {
+  chain_enter();
   __shared__ double sh[kPlaneThreads / 32];
   const int k = 1 + blockIdx.y;
   double acc = 0.0;
@@ -1623,14 +1635,14 @@ int64_t plane_part_doubles(const NSDev& D) { return (int64_t)kPlaneBlocks * D.Z;
 
 int launch_plane_part(const NSDev& D, const double* a, const double* wx, const double* wy, double* part,
                       cudaStream_t s) {
-  k_plane_part<<<dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s>>>(D, a, wx, wy, part);
+  launch_chained(k_plane_part, dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s, D, a, wx, wy, part);
   count_launch();
   return kPlaneBlocks;
 }
 
 void launch_plane_avg(const NSDev& D, const double* a, const double* wx, const double* wy, double area,
                       double* part, double* out, cudaStream_t s) {
-  k_plane_part<<<dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s>>>(D, a, wx, wy, part);
+  launch_chained(k_plane_part, dim3(kPlaneBlocks, (unsigned)D.Z), kPlaneThreads, 0, s, D, a, wx, wy, part);
   k_plane_fold<<<(D.Z + 127) / 128, 128, 0, s>>>(D.Z, kPlaneBlocks, part, area, out);
   count_launch(2);
 }
@@ -1695,7 +1707,7 @@ void launch_psource(const NSDev* const* Ds, const double* dts, int n, cudaStream
     for (double& v : rdt.v) v = 1.0 / v;
     int per;
     const dim3 g = cell_grid_k(P.d[0], &per, m);
-    k_psource<N><<<g, kCellCols, 0, s>>>(P, rdt, per);
+    launch_chained(k_psource<N>, g, kCellCols, 0, s, P, rdt, per);
     count_launch();
   });
 }
@@ -1712,8 +1724,8 @@ void launch_pgrad(const NSDev* const* Ds, const double* dts, int n, const ZRule&
     const auto dt = scal<N>(dts, b, m);
     int per;
     const dim3 g = cell_grid_k(P.d[0], &per, m);
-    if (P.d[0].unit_r) k_pgrad<true, N><<<g, kCellCols, 0, s>>>(P, dt, hist, per);
-    else k_pgrad<false, N><<<g, kCellCols, 0, s>>>(P, dt, hist, per);
+    if (P.d[0].unit_r) launch_chained(k_pgrad<true, N>, g, kCellCols, 0, s, P, dt, hist, per);
+    else launch_chained(k_pgrad<false, N>, g, kCellCols, 0, s, P, dt, hist, per);
     count_launch();
     GhostFields<N> F{{}, {Ru, Rv, Rw}, 3};
     for (int q = 0; q < m; ++q) {
@@ -1763,7 +1775,7 @@ void launch_divergence(const NSDev* const* Ds, const DivSet* set, int n, bool cf
     dim3 g = divergence_grid(P.d[0]);
     const int zb = (int)g.z;
     g.z = (unsigned)(zb * m);
-    k_divergence<N><<<g, 128, 0, s>>>(P, O, cfl ? 1 : 0, zb);
+    launch_chained(k_divergence<N>, g, 128, 0, s, P, O, cfl ? 1 : 0, zb);
     count_launch();
   });
 }
@@ -1783,7 +1795,7 @@ void launch_cn_factors(const NSDev* const* Ds, const CNFactorSet* set, int n, in
       }
     const size_t sm = 3 * (size_t)(P.d[0].nz + 2) * sizeof(double);
     set_smem_limit_once((const void*)k_cn_factors<N>, 64 * 1024);
-    k_cn_factors<N><<<dim3(5, (unsigned)nslots, (unsigned)m), 128, sm, s>>>(P, J, slot0);
+    launch_chained(k_cn_factors<N>, dim3(5, (unsigned)nslots, (unsigned)m), 128, sm, s, P, J, slot0);
     count_launch();
   });
 }
