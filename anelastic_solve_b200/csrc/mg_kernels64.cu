@@ -3,6 +3,7 @@
 // contraction, so every value is rounded exactly as the reference's
 // expressions evaluated left to right.
 #include "mg_launch_impl.cuh"
+#include "pdl.cuh"
 
 namespace anel {
 
@@ -81,8 +82,8 @@ __global__ void __launch_bounds__(kResidX) k_resid_norm(DevLevel<double> L, cons
 
 // part[0..2n) -> out2[0..2*gridDim.x): CTA b sums its contiguous chunk
 // (blockIdx.y: member of a batch, its arrays pstride / ostride doubles on)
-__global__ void k_fold_chunks(const double* __restrict__ part, int64_t n, double* __restrict__ out2,
-                              int64_t pstride = 0, int64_t ostride = 0) {
+__global__ void k_fold_chunks(const double* part, int64_t n, double* out2, int64_t pstride, int64_t ostride) {
+  chain_enter();
   __shared__ double sh[kNormThreads / 32];
   part += blockIdx.y * pstride;
   out2 += blockIdx.y * ostride;
@@ -102,7 +103,8 @@ __global__ void k_fold_chunks(const double* __restrict__ part, int64_t n, double
   }
 }
 
-__global__ void k_fold(const double* __restrict__ part, int nb, double* out, int64_t pstride = 0) {
+__global__ void k_fold(const double* part, int nb, double* out, int64_t pstride) {
+  chain_enter();
   __shared__ double sh[kNormThreads / 32];
   part += blockIdx.x * pstride;
   out += 2 * blockIdx.x;
@@ -136,16 +138,16 @@ static void launch_resid(const DevLevel<double>& L, const double* phi, const dou
   const int64_t n = (int64_t)g.x * g.y * g.z;
   k_resid_norm<kStore><<<g, kResidX, 0, s>>>(L, phi, f, r32, part);
   double* part2 = part + 2 * n;
-  k_fold_chunks<<<kFoldBlocks, kNormThreads, 0, s>>>(part, n, part2);
-  k_fold<<<1, kNormThreads, 0, s>>>(part2, kFoldBlocks, out);
+  launch_chained(k_fold_chunks, kFoldBlocks, kNormThreads, 0, s, part, n, part2, 0, 0);
+  launch_chained(k_fold, 1, kNormThreads, 0, s, part2, kFoldBlocks, out, 0);
   count_launch(3);
 }
 
 int64_t fold_scratch_doubles() { return 2 * (int64_t)kFoldBlocks; }
 
 void launch_fold_pairs(const double* part, int64_t n, double* scratch, double* out, cudaStream_t s) {
-  k_fold_chunks<<<kFoldBlocks, kNormThreads, 0, s>>>(part, n, scratch);
-  k_fold<<<1, kNormThreads, 0, s>>>(scratch, kFoldBlocks, out);
+  k_fold_chunks<<<kFoldBlocks, kNormThreads, 0, s>>>(part, n, scratch, 0, 0);
+  k_fold<<<1, kNormThreads, 0, s>>>(scratch, kFoldBlocks, out, 0);
   count_launch(2);
 }
 

@@ -6,18 +6,20 @@
 
 namespace anel {
 
+// x at interior cell or z ghost `at` of column (i, j) and at the x and y
+// ghosts that copy it
+__device__ __forceinline__ void rb_images(const RBLevel& L, double* phi, int64_t at, int i, int64_t oy, double x) {
+  const int ox = i == 2 ? L.nx : (i == L.nx + 1 ? -L.nx : 0);
+  phi[at] = x;
+  if (ox) phi[at + ox] = x;
+  if (oy) phi[at + oy] = x;
+  if (ox && oy) phi[at + ox + oy] = x;
+}
 // v at interior cell (i, j, k), offset c, and at the ghosts that copy it
 __device__ __forceinline__ void rb_put(const RBLevel& L, int64_t c, int i, int64_t oy, int k, double v) {
-  const int ox = i == 2 ? L.nx : (i == L.nx + 1 ? -L.nx : 0);
-  auto put = [&](int64_t at, double x) {
-    L.phi[at] = x;
-    if (ox) L.phi[at + ox] = x;
-    if (oy) L.phi[at + oy] = x;
-    if (ox && oy) L.phi[at + ox + oy] = x;
-  };
-  put(c, v);
-  if (k == 2 && L.n1) put(c - L.XY, v - L.add1);
-  if (k == L.nz + 1 && L.nZ) put(c + L.XY, v + L.addZ);
+  rb_images(L, L.phi, c, i, oy, v);
+  if (k == 2 && L.n1) rb_images(L, L.phi, c - L.XY, i, oy, v - L.add1);
+  if (k == L.nz + 1 && L.nZ) rb_images(L, L.phi, c + L.XY, i, oy, v + L.addZ);
 }
 // the y shift to the image of row j (0: none)
 __device__ __forceinline__ int64_t rb_yshift(const RBLevel& L, int j) {
@@ -113,139 +115,213 @@ void launch_rb_prolong(const RBLevel& L, const DevLevel<double>& F, const DevLev
 }
 
 // ---------------------------------------------------- coarse levels
-// The levels of at most kRBSharedCells cells and everything below them in
-// one block: their half-sweeps are 1000 to 4 cells long and as separate
-// launches cost 6 us each, about 60 of them per cycle.  phi and f stay in
-// shared memory; boundary passes go by the ghost tables.  An 8192-cell
-// level fits too, but one SM takes longer over it than its launches
-// (256x128x128 solve: 39.1 ms with it, 34.3 without; 128x64x128 step with
-// the 2048-cell level 20.0, without 20.2).
+// The levels of at most 2 kRBThreads cells of a colour and everything below
+// them in one block: their half-sweeps are 1024 to 4 cells long and as
+// separate launches cost 6 us each, about 60 of them per cycle.  phi and f
+// stay in shared memory.  What bounds the block is latency: a thread holds
+// its cells' coefficients and f in registers for the sweeps and the residual
+// of a visit, its ghosts as packed words, and the schedule is one loop, so
+// the code is fetched once.  An 8192-cell level fits too, but one SM takes
+// longer over it than its launches (256x128x128 solve: 39.1 ms with it, 34.3
+// without).
 constexpr int kRBThreads = 512;
+constexpr int kRBGhosts = 4;  // ghosts of a thread held in registers
+constexpr unsigned kNoGhost = 0xffffffffu;
 
-__device__ __forceinline__ unsigned rb_magic(int d) { return (unsigned)((0x100000000ull + d - 1) / (unsigned)d); }
+static unsigned rb_magic(int d) { return (unsigned)((0x100000000ull + d - 1) / (unsigned)d); }
 __device__ __forceinline__ int rb_div(int u, int d, unsigned m) { return d == 1 ? u : (int)__umulhi((unsigned)u, m); }
 
-__device__ __forceinline__ int rb_ghosts(const DevLevel<double>& L) { return (int)L.G - L.nx * L.ny * L.nz; }
+// a colour's cell: offset (negative: none), coefficients, diagonal, f
+struct RBCell {
+  int c;
+  double a1, a2, a3, a4, a5, a6, d, f;
+};
 
-__device__ __forceinline__ void rb_bdry(const DevLevel<double> L, const int2* __restrict__ gt) {
-  const int n = rb_ghosts(L);
-  for (int g = threadIdx.x; g < n; g += kRBThreads) {
-    const int2 e = gt[g];
-    L.phi[e.x] = e.y >= 0 ? L.phi[e.y] : 0.0;
-  }
-  __syncthreads();
+__device__ __forceinline__ RBCell rb_cell(const RBShared& S, int l, const double* sm, const double* src, int color,
+                                          int t) {
+  const DevLevel<double>& L = S.L[l];
+  const int hx = (L.nx + 1) >> 1;
+  RBCell q;
+  q.c = -1;
+  if (t >= hx * L.ny * L.nz) return q;
+  const int r = rb_div(t, hx, S.mh[l]), kk = rb_div(r, L.ny, S.my[l]);
+  const int k = 2 + kk, j = 2 + r - kk * L.ny, i = 2 + ((color + j + k) & 1) + 2 * (t - r * hx);
+  if (i > L.nx + 1) return q;
+  q.c = (int)cidx(i, j, k, L.X, L.XY);
+  const double *cx = sm + S.coef[l] + i - 1, *cy = sm + S.coef[l] + 2 * L.X + j - 1,
+               *cz = sm + S.coef[l] + 2 * L.X + 2 * L.Y + k - 1;
+  q.a1 = cx[0];
+  q.a2 = cx[L.X];
+  q.a3 = cy[0];
+  q.a4 = cy[L.Y];
+  q.a5 = cz[0];
+  q.a6 = cz[L.Z];
+  q.d = -(q.a1 + q.a2 + q.a3 + q.a4 + cz[2 * L.Z] + cz[3 * L.Z]);
+  q.f = src[q.c];
+  return q;
 }
 
-__device__ __forceinline__ void rb_relax(const DevLevel<double> L, const int2* __restrict__ gt, int iters) {
-  const int hx = (L.nx + 1) >> 1, n = hx * L.ny * L.nz;
-  const unsigned mx = rb_magic(hx), my = rb_magic(L.ny);
-  for (int it = 0; it < 2 * iters; ++it) {
-    const int color = it & 1;
-    for (int t = threadIdx.x; t < n; t += kRBThreads) {
-      const int r = rb_div(t, hx, mx), q = t - r * hx;
-      const int kk = rb_div(r, L.ny, my);
-      const int k = 2 + kk, j = 2 + r - kk * L.ny;
-      const int i = 2 + ((color + j + k) & 1) + 2 * q;
-      if (i > L.nx + 1) continue;
-      const int64_t c = cidx(i, j, k, L.X, L.XY);
-      L.phi[c] = stencil_update(L, (const double*)L.phi, L.src[c], c, i, j, k);
-    }
-    __syncthreads();
-    rb_bdry(L, gt);
-  }
+// the six neighbours' terms in stencil_update's order
+__device__ __forceinline__ double rb_terms(const RBCell& q, const double* phi, int X, int XY) {
+  const double* p = phi + q.c;
+  double acc = q.a1 * p[-1];
+  acc = acc + q.a2 * p[1];
+  acc = acc + q.a3 * p[-X];
+  acc = acc + q.a4 * p[X];
+  acc = acc + q.a5 * p[-XY];
+  acc = acc + q.a6 * p[XY];
+  return acc;
+}
+
+__device__ __forceinline__ void rb_ghost(double* phi, unsigned w) {
+  if (w != kNoGhost) phi[w >> 16] = (w & 0xffffu) == 0xffffu ? 0.0 : phi[w & 0xffffu];
 }
 
 template <int CD>
-__device__ __forceinline__ void rb_restrict(const DevLevel<double> F, const DevLevel<double> C) {
-  const int n = C.nx * C.ny * C.nz;
-  for (int t = threadIdx.x; t < (int)C.G; t += kRBThreads) C.phi[t] = 0.0;
-  for (int t = threadIdx.x; t < n; t += kRBThreads) {
-    const int i = 2 + t % C.nx, r = t / C.nx, j = 2 + r % C.ny, k = 2 + r / C.ny;
-    C.src[cidx(i, j, k, C.X, C.XY)] = restrict_value<double, CD>(F, i, j, k);
-  }
-  __syncthreads();
-}
-
-template <int CD>
-__device__ __forceinline__ void rb_prolong(const DevLevel<double> F, const DevLevel<double> C) {
+__device__ __forceinline__ void rb_prolong(const RBShared& S, int l, double* phi, const DevLevel<double>& C) {
+  const DevLevel<double>& F = S.L[l];
   const int n = F.nx * F.ny * F.nz;
   for (int t = threadIdx.x; t < n; t += kRBThreads) {
-    const int i = 2 + t % F.nx, r = t / F.nx, j = 2 + r % F.ny, k = 2 + r / F.ny;
-    const int64_t c = cidx(i, j, k, F.X, F.XY);
-    F.phi[c] = F.phi[c] + prolong_corr<double, CD>(C, i, j, k);
+    const int r = rb_div(t, F.nx, S.mx[l]), kk = rb_div(r, F.ny, S.my[l]);
+    const int i = 2 + t - r * F.nx, j = 2 + r - kk * F.ny, k = 2 + kk;
+    const int c = (int)cidx(i, j, k, F.X, F.XY);
+    phi[c] = phi[c] + prolong_corr<double, CD>(C, i, j, k);
   }
-  __syncthreads();
 }
-
-#define RB_BY_CD(cd, call)        \
-  switch ((cd) & 7) {             \
-    case 0: call<0>(F, C); break; \
-    case 1: call<1>(F, C); break; \
-    case 2: call<2>(F, C); break; \
-    case 3: call<3>(F, C); break; \
-    case 4: call<4>(F, C); break; \
-    case 5: call<5>(F, C); break; \
-    case 6: call<6>(F, C); break; \
-    default: call<7>(F, C); break; \
-  }
-
-__host__ __device__ inline int rb_coefs(int X, int Y, int Z) { return 2 * X + 2 * Y + 4 * Z; }
 
 __global__ void __launch_bounds__(kRBThreads) k_rb_shared(const __grid_constant__ RBShared S) {
   chain_enter();
-  extern __shared__ double rsm[];
-  __shared__ DevLevel<double> lv[kRBSharedLevels + 1];
-  if (threadIdx.x == 0) {
-    double* at = rsm;
-    for (int l = 1; l <= S.lc; ++l) {
-      DevLevel<double> L = S.L[l];
-      L.phi = at;
-      L.src = at + L.G;
-      L.coef = at + 2 * L.G;
-      at += 2 * L.G + rb_coefs(L.X, L.Y, L.Z);
-      lv[l] = L;
-    }
+  extern __shared__ double sm[];
+  const int tid = threadIdx.x, lc = S.lc;
+  for (int t = tid; t < S.nblob; t += kRBThreads) sm[t] = S.blob[t];
+  const int G = (int)S.L[lc].G;
+  for (int t = tid; t < G; t += kRBThreads) {
+    sm[S.phi[lc] + t] = 0.0;
+    sm[S.phi[lc] + G + t] = S.L[lc].src[t];
   }
   __syncthreads();
-  for (int l = 1; l <= S.lc; ++l) {
-    const DevLevel<double>& L = lv[l];
-    const int n = rb_coefs(L.X, L.Y, L.Z);
-    for (int t = threadIdx.x; t < n; t += kRBThreads) const_cast<double*>(L.coef)[t] = S.L[l].coef[t];
-  }
-  const int G = (int)lv[S.lc].G;
-  for (int t = threadIdx.x; t < G; t += kRBThreads) {
-    lv[S.lc].phi[t] = 0.0;
-    lv[S.lc].src[t] = S.L[S.lc].src[t];
-  }
-  __syncthreads();
+  double* const res = sm + S.res;
   // the schedule of mg_cycle.F90:186-325 between the restriction to level
   // lc and the prolongation from it
-  for (int l = S.lc; l >= 2; --l) {
-    rb_relax(lv[l], S.gt[l], S.pre[l]);
-    const DevLevel<double>&F = lv[l], &C = lv[l - 1];
-    RB_BY_CD(S.cd[l - 1], rb_restrict);
+#pragma unroll 1
+  for (int v = 0; v < 2 * lc; ++v) {
+    const bool down = v < lc;
+    const int l = down ? lc - v : v - lc + 1;
+    const DevLevel<double>& L = S.L[l];
+    const int X = L.X, XY = (int)L.XY, GL = (int)L.G, iters = down ? S.pre[l] : S.post[l];
+    double* const phi = sm + S.phi[l];
+    const unsigned* const gw = reinterpret_cast<const unsigned*>(sm + S.ghost[l]);
+    const int ng = GL - L.nx * L.ny * L.nz;
+    RBCell q[2][2];
+    unsigned w[kRBGhosts];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) q[h][r] = rb_cell(S, l, sm, phi + GL, h, tid + r * kRBThreads);
+#pragma unroll
+    for (int g = 0; g < kRBGhosts; ++g) w[g] = tid + g * kRBThreads < ng ? gw[tid + g * kRBThreads] : kNoGhost;
+    auto ghosts = [&]() {
+      __syncthreads();
+#pragma unroll
+      for (int g = 0; g < kRBGhosts; ++g) rb_ghost(phi, w[g]);
+      for (int g = tid + kRBGhosts * kRBThreads; g < ng; g += kRBThreads) rb_ghost(phi, gw[g]);
+      __syncthreads();
+    };
+#pragma unroll 1
+    for (int it = 0; it < iters; ++it)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (q[h][r].c >= 0) phi[q[h][r].c] = (q[h][r].f - rb_terms(q[h][r], phi, X, XY)) / q[h][r].d;
+        ghosts();
+      }
+    if (v < lc - 1) {
+      // the children's residuals (fine_resid), then their sums in the order
+      // of restrict_value: a nibble per child, bits x, y, z
+      const DevLevel<double>& C = S.L[l - 1];
+      double* const cphi = sm + S.phi[l - 1];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (q[h][r].c >= 0) {
+            double acc = rb_terms(q[h][r], phi, X, XY);
+            acc = acc + q[h][r].d * phi[q[h][r].c];
+            res[q[h][r].c] = q[h][r].f - acc;
+          }
+      for (int t = tid; t < (int)C.G; t += kRBThreads) cphi[t] = 0.0;
+      __syncthreads();
+      const int cd = S.cd[l - 1], m = 1 << __popc(cd), n = C.nx * C.ny * C.nz;
+      const unsigned seq = cd == 7 ? 0x53716420u : cd == 6 ? 0x6420u : cd == 5 ? 0x5140u : cd == 3 ? 0x3210u : cd << 4;
+      const double wgt = 1.0 / m;
+      for (int t = tid; t < n; t += kRBThreads) {
+        const int r = rb_div(t, C.nx, S.mx[l - 1]), kk = rb_div(r, C.ny, S.my[l - 1]);
+        const int i = 2 + t - r * C.nx, j = 2 + r - kk * C.ny, k = 2 + kk;
+        const double* p =
+            res + cidx(cd & 1 ? 2 * i - 2 : i, cd & 2 ? 2 * j - 2 : j, cd & 4 ? 2 * k - 2 : k, X, XY);
+        double s = p[0];
+        for (int e = 1; e < m; ++e) {
+          const unsigned b = seq >> (4 * e);
+          s = s + p[(b & 1) + ((b >> 1) & 1) * X + ((b >> 2) & 1) * XY];
+        }
+        cphi[C.G + cidx(i, j, k, C.X, C.XY)] = wgt * s;
+      }
+      __syncthreads();
+    } else if (v >= lc && l < lc) {
+      DevLevel<double> C = L;
+      C.phi = phi;
+      double* const fphi = sm + S.phi[l + 1];
+      switch (S.cd[l]) {
+        case 1: rb_prolong<1>(S, l + 1, fphi, C); break;
+        case 2: rb_prolong<2>(S, l + 1, fphi, C); break;
+        case 3: rb_prolong<3>(S, l + 1, fphi, C); break;
+        case 4: rb_prolong<4>(S, l + 1, fphi, C); break;
+        case 5: rb_prolong<5>(S, l + 1, fphi, C); break;
+        case 6: rb_prolong<6>(S, l + 1, fphi, C); break;
+        default: rb_prolong<7>(S, l + 1, fphi, C); break;
+      }
+      __syncthreads();
+      const unsigned* const fw = reinterpret_cast<const unsigned*>(sm + S.ghost[l + 1]);
+      const DevLevel<double>& F = S.L[l + 1];
+      const int nf = (int)F.G - F.nx * F.ny * F.nz;
+      for (int g = tid; g < nf; g += kRBThreads) rb_ghost(fphi, fw[g]);
+      __syncthreads();
+    }
   }
-  rb_relax(lv[1], S.gt[1], S.pre[1]);
-  for (int l = 1; l < S.lc; ++l) {
-    rb_relax(lv[l], S.gt[l], S.post[l]);
-    const DevLevel<double>&F = lv[l + 1], &C = lv[l];
-    RB_BY_CD(S.cd[l], rb_prolong);
-    rb_bdry(lv[l + 1], S.gt[l + 1]);
-  }
-  rb_relax(lv[S.lc], S.gt[S.lc], S.post[S.lc]);
-  for (int t = threadIdx.x; t < G; t += kRBThreads) S.L[S.lc].phi[t] = lv[S.lc].phi[t];
+  for (int t = tid; t < G; t += kRBThreads) S.L[lc].phi[t] = sm[S.phi[lc] + t];
 }
 
-size_t rb_shared_bytes(const RBShared& S) {
-  size_t n = 0;
-  for (int l = 1; l <= S.lc; ++l) n += 2 * (size_t)S.L[l].G + rb_coefs(S.L[l].X, S.L[l].Y, S.L[l].Z);
-  return n * sizeof(double);
+bool rb_shared_fits(RBShared& S, int l) {
+  // offsets in doubles: coefficients and ghost words (the blob), the
+  // residuals of a visit, phi and f of each level
+  int at = 0;
+  for (int m = 1; m <= l; ++m) {
+    const DevLevel<double>& L = S.L[m];
+    const int64_t hx = (L.nx + 1) / 2, ng = L.G - (int64_t)L.nx * L.ny * L.nz;
+    if (hx * L.ny * L.nz > 2 * kRBThreads || L.G >= 0xffff || (m < l && S.cd[m] == 0)) return false;
+    S.mh[m] = rb_magic((int)hx);
+    S.mx[m] = rb_magic(L.nx);
+    S.my[m] = rb_magic(L.ny);
+    S.coef[m] = at;
+    at += 2 * L.X + 2 * L.Y + 4 * L.Z;
+    S.ghost[m] = at;
+    at += (int)((ng + 1) / 2);
+  }
+  S.nblob = S.res = at;
+  at += (int)S.L[l].G;
+  for (int m = 1; m <= l; ++m) {
+    S.phi[m] = at;
+    at += 2 * (int)S.L[m].G;
+  }
+  S.bytes = (size_t)at * sizeof(double);
+  return S.bytes <= kRBSharedBytes;
 }
 
 void rb_shared_prepare() { set_smem_limit_once((const void*)k_rb_shared, (int)kRBSharedBytes); }
 
 void launch_rb_shared(const RBShared& S, cudaStream_t s) {
-  launch_chained(k_rb_shared, 1, kRBThreads, rb_shared_bytes(S), s, S);
+  launch_chained(k_rb_shared, 1, kRBThreads, S.bytes, s, S);
   count_launch();
 }
 
@@ -255,8 +331,8 @@ void launch_rb_shared(const RBShared& S, cudaStream_t s) {
 // maxima of non-negative doubles by their bit patterns, exact in any order,
 // one atomic pair per block.  256x128x128: 66 us with one value at a time.
 constexpr int kMaxU = 4;
-__global__ void __launch_bounds__(256) k_relmax_copy(DevLevel<double> L, const double* __restrict__ phin,
-                                                     double* __restrict__ phio, unsigned long long* out) {
+__global__ void __launch_bounds__(256) k_relmax_copy(DevLevel<double> L, const double* phin, double* phio,
+                                                     unsigned long long* out) {
   chain_enter();
   __shared__ unsigned long long sh[2][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

@@ -22,20 +22,26 @@ void launch_rb_march(const RBLevel& L, int color, cudaStream_t s);
 
 // Levels 1..lc of the cycle in one block, phi and f in shared memory.
 constexpr int kRBSharedLevels = 10;
-constexpr int kRBSharedCells = 2048;         // most interior cells of level lc
 constexpr size_t kRBSharedBytes = 220 << 10;
 struct RBShared {
   int lc;
   DevLevel<double> L[kRBSharedLevels + 1];   // [1..lc]
-  const int2* gt[kRBSharedLevels + 1];       // their homogeneous ghost tables
   int pre[kRBSharedLevels + 1], post[kRBSharedLevels + 1];
   int cd[kRBSharedLevels + 1];               // directions coarsened from l + 1 to l
+  unsigned mh[kRBSharedLevels + 1], mx[kRBSharedLevels + 1], my[kRBSharedLevels + 1];  // dividers of cell indices
+  int coef[kRBSharedLevels + 1], ghost[kRBSharedLevels + 1], phi[kRBSharedLevels + 1]; // shared-memory offsets
+  int nblob, res;
+  size_t bytes;
+  // the levels' coefficients and homogeneous ghost tables (ghost cell << 16
+  // | interior cell it copies, or 0xffff for zero), as they lie in shared
+  // memory
+  const double* blob;
 };
 // phi += the interpolated correction of the coarse level, ghosts included
 void launch_rb_prolong(const RBLevel& L, const DevLevel<double>& F, const DevLevel<double>& C, int cdir,
                        cudaStream_t s);
-// shared memory of levels 1..lc
-size_t rb_shared_bytes(const RBShared& S);
+// whether levels 1..l fit (their L, cd filled in), and their layout
+bool rb_shared_fits(RBShared& S, int l);
 void rb_shared_prepare();
 // level lc's f from global memory, its corrected phi (ghosts too) to it
 void launch_rb_shared(const RBShared& S, cudaStream_t s);

@@ -378,7 +378,7 @@ MGSolver::~MGSolver() {
     cudaFree(d_colfac_[l]);
   }
   for (double* q : d_rbz_) cudaFree(q);
-  for (int2* q : d_rbtab_) cudaFree(q);
+  cudaFree(d_rbblob_);
   direct_free(dir_);
   direct_free(dirfine_);
   spec_free(spec_);
@@ -1124,7 +1124,10 @@ int MGSolver::upload_coefficients() {
     }
   }
   op_hash_ = h;
-  if (prm_.precision != ANEL_PREC_MIXED && prm_.smoother == ANEL_SMOOTHER_RBPGS) return build_rb_levels();
+  if (prm_.precision != ANEL_PREC_MIXED && prm_.smoother == ANEL_SMOOTHER_RBPGS) {
+    const int st = upload_rb_shared();
+    return st != ANEL_OK ? st : build_rb_levels();
+  }
   return spec_want_ ? build_spec() : ANEL_OK;
 }
 
@@ -1134,23 +1137,49 @@ int MGSolver::build_rb_shared() {
   rbs_.lc = 0;
   const int top = std::min(ngrid_ - 1, kRBSharedLevels);
   for (int l = 1; l <= top; ++l) {
-    const LevelGeom& G = geo_[l];
     rbs_.L[l] = L64(l);
     rbs_.pre[l] = prm_.pre_relax[l - 1];
     rbs_.post[l] = prm_.post_relax[l - 1];
     rbs_.cd[l] = coarsen_dirs(l);
     RBShared t = rbs_;
+    if (!rb_shared_fits(t, l)) break;
     t.lc = l;
-    if ((int64_t)G.n[0] * G.n[1] * G.n[2] > kRBSharedCells || rb_shared_bytes(t) > kRBSharedBytes) break;
-    rbs_.lc = l;
-    const int64_t ngh = G.G - (int64_t)G.n[0] * G.n[1] * G.n[2];
-    ANEL_CUDA_TRY(cudaMalloc(&d_rbtab_[l], (size_t)ngh * sizeof(int2)));
-    launch_ghost_table(L32(l, true), d_rbtab_[l], stream_);
-    rbs_.gt[l] = d_rbtab_[l];
+    rbs_ = t;
   }
+  if (rbs_.lc == 0) return ANEL_OK;
+  rbs_blob_.assign(rbs_.nblob, 0.0);
+  for (int l = 1; l <= rbs_.lc; ++l) {
+    const LevelGeom& G = geo_[l];
+    const int64_t ngh = G.G - (int64_t)G.n[0] * G.n[1] * G.n[2];
+    int2* d_tab = nullptr;
+    ANEL_CUDA_TRY(cudaMalloc(&d_tab, (size_t)ngh * sizeof(int2)));
+    launch_ghost_table(L32(l, true), d_tab, stream_);
+    std::vector<int2> tab(ngh);
+    cudaMemcpyAsync(tab.data(), d_tab, (size_t)ngh * sizeof(int2), cudaMemcpyDeviceToHost, stream_);
+    const cudaError_t e = cudaStreamSynchronize(stream_);
+    cudaFree(d_tab);
+    ANEL_CUDA_TRY(e);
+    unsigned* w = reinterpret_cast<unsigned*>(rbs_blob_.data() + rbs_.ghost[l]);
+    for (int64_t g = 0; g < ngh; ++g)
+      w[g] = (unsigned)tab[g].x << 16 | (tab[g].y >= 0 ? (unsigned)tab[g].y : 0xffffu);
+  }
+  ANEL_CUDA_TRY(cudaMalloc(&d_rbblob_, rbs_blob_.size() * sizeof(double)));
+  rbs_.blob = d_rbblob_;
   rb_shared_prepare();
-  ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
   return check_launch("ghost tables");
+}
+
+// the shared levels' part of the coefficients
+int MGSolver::upload_rb_shared() {
+  if (rbs_.lc == 0) return ANEL_OK;
+  for (int l = 1; l <= rbs_.lc; ++l) {
+    const LevelCoef& c = coef_[l];
+    double* at = rbs_blob_.data() + rbs_.coef[l];
+    for (const std::vector<double>* v : {&c.cx1, &c.cx2, &c.cy3, &c.cy4, &c.cz5, &c.cz6, &c.dz5, &c.dz6})
+      at = std::copy(v->begin(), v->end(), at);
+  }
+  ANEL_CUDA_TRY(cudaMemcpy(d_rbblob_, rbs_blob_.data(), rbs_blob_.size() * sizeof(double), cudaMemcpyHostToDevice));
+  return ANEL_OK;
 }
 
 // Self-ghosting half-sweeps: x and y periodic, even and with one
@@ -1590,8 +1619,7 @@ int MGSolver::build_self_ghosting(int l) {
 double MGSolver::true_resid(const double* d_phi, const double* d_rhs, cudaStream_t s,
                             double* fnorm) {
   const DevLevel<double> F = fine_view(const_cast<double*>(d_phi), d_rhs);
-  launch_resid_norm(F, d_phi, d_rhs, d_part_, d_norm_, s);
-  copy_words(d_norm_, h_pin_, 2, s);
+  launch_resid_norm(F, d_phi, d_rhs, d_part_, h_pin_, s);  // the fold writes the mapped words itself
   cudaStreamSynchronize(s);
   if (fnorm) *fnorm = std::sqrt(h_pin_[1]);
   return h_pin_[1] > 0.0 ? std::sqrt(h_pin_[0] / h_pin_[1]) : std::sqrt(h_pin_[0]);

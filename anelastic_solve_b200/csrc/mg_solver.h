@@ -75,8 +75,10 @@ class MGSolver {
   RBLevel rb_[ANEL_MAX_LEVELS + 1];
   double* d_rbz_[ANEL_MAX_LEVELS + 1] = {nullptr};
   RBShared rbs_{};
-  int2* d_rbtab_[kRBSharedLevels + 1] = {nullptr};
+  std::vector<double> rbs_blob_;
+  double* d_rbblob_ = nullptr;
   int build_rb_shared();
+  int upload_rb_shared();
   int build_rb_levels();
   template <class F>
   void run_captured(cudaStream_t s, F cycle);

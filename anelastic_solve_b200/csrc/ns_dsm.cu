@@ -34,8 +34,7 @@ dim3 interior_grid(const NSDev& D) {
   if (i > D.nx + 1) return;                              \
   const int64_t o = NS_IX(i, j, k)
 
-__global__ void k_dyn_modS(NSDev D, const double* __restrict__ l1, const double* __restrict__ l2,
-                           const double* __restrict__ l3, double* __restrict__ out) {
+__global__ void k_dyn_modS(NSDev D, const double* l1, const double* l2, const double* l3, double* out) {
   chain_enter();
   DYN_CELL();
   out[o] = strain_mag(D, l1, l2, l3, i, j, k);
@@ -44,7 +43,7 @@ __global__ void k_dyn_modS(NSDev D, const double* __restrict__ l1, const double*
 // DSM's lestmp1 of component ij (DSM.F90:38-86): the diagonal strain, and
 // for ij = 4..6 half the difference of the two cross derivatives (the
 // source subtracts where straincal adds).
-__global__ void k_dyn_comp(NSDev D, int ij, double* __restrict__ out) {
+__global__ void k_dyn_comp(NSDev D, int ij, double* out) {
   chain_enter();
   DYN_CELL();
   const double *l1 = D.u, *l2 = D.v, *l3 = D.w;
@@ -453,9 +452,8 @@ __global__ void k_dyn_column(NSDev D, const double* __restrict__ a, double* __re
 // then filterHF (DSM.F90:196-256).  Everything after the averages is
 // constant on planes, where filterHF's x and y passes change nothing, so it
 // is a computation on profiles; prof(k), k = 2..nz+1.
-__global__ void __launch_bounds__(256) k_dyn_ratio(NSDev D, const double* __restrict__ pn,
-                                                   const double* __restrict__ pd, int nb, double area, DynZ R,
-                                                   double* __restrict__ prof) {
+__global__ void __launch_bounds__(256) k_dyn_ratio(NSDev D, const double* pn, const double* pd, int nb, double area,
+                                                   DynZ R, double* prof) {
   chain_enter();
   extern __shared__ double sr[];
   const int nz = D.nz;

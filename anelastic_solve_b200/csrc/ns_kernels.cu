@@ -1568,10 +1568,8 @@ __global__ void k_fluct_sq(NSDev D, const double* __restrict__ a, const double* 
 // given grid; the order differs from the reference's single running sum.
 constexpr int kPlaneBlocks = 32;
 constexpr int kPlaneThreads = 256;
-__global__ void __launch_bounds__(kPlaneThreads) k_plane_part(NSDev D, const double* __restrict__ a,
-                                                             const double* __restrict__ wx,
-                                                             const double* __restrict__ wy,
-                                                             double* __restrict__ part) {
+__global__ void __launch_bounds__(kPlaneThreads) k_plane_part(NSDev D, const double* a, const double* wx,
+                                                             const double* wy, double* part) {
   chain_enter();
   __shared__ double sh[kPlaneThreads / 32];
   const int k = 1 + blockIdx.y;

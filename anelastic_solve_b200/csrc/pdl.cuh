@@ -6,7 +6,9 @@
 // visible.  What overlaps is the launch itself (about 1 us per kernel on the
 // small grids, whose sub-step is a chain of some 13 kernels of 3-10 us), so
 // the results and the order of all memory accesses are those of plain
-// launches.
+// launches.  No kernel launched this way has a __restrict__ pointer to const
+// among its parameters: loads through one count as loads of constant memory
+// and need not stay behind the wait.
 #pragma once
 
 #include <cuda_runtime.h>
