@@ -277,28 +277,38 @@ __device__ __forceinline__ double rhs_scalar(const NSDev& D, const Acc& A_, int 
 //
 // Tiled: a block owns 32 (i) x 8 (j) columns and marches `per` planes in z
 // (kRT_K = 32, fewer on grids that would not fill the GPU: 64x32x64 has 16
-// tiles of 32 planes, 59 us; 4 planes still repay the two halo planes).  u, v, w and rho are staged in shared memory plane by plane (the
-// tile plus a one-cell halo), four planes per field in a ring: the
-// functions read planes k-1, k, k+1 while the block brings plane k+2 in
-// with asynchronous copies, so every field value is read from global memory once
-// per tile instead of once per use.  kL (the eddy coefficients exist):
-// nuT and kappaT are staged in the same ring; scal1 and nappaT are read
-// from global memory.
+// tiles of 32 planes, 59 us; 4 planes still repay the two halo planes).  u,
+// v, w and rho are staged in shared memory plane by plane (the tile plus a
+// one-cell halo) in a ring: the functions read planes k-1, k, k+1 while
+// asynchronous copies bring the next kRhsAhead planes in, so every field
+// value is read from global memory once per tile instead of once per use,
+// and the accumulators q arrive the same way.  kL (the eddy coefficients
+// exist): nuT and kappaT are staged in the same ring; scal1 and nappaT are
+// read from global memory.  With one plane ahead and q loaded by the step
+// that uses it, a step of 1.6 us (2.2 with q) was mostly the copies' latency:
+// 256x128x256 303 us with q, 245 so.  The six fields of kL have no room for
+// it (711 us instead of 523 at 384x192x192), and over members it spills
+// registers (8 x 64^3: 150 us instead of 63).
 constexpr int kRT_I = 32, kRT_J = 8, kRT_K = 32;
 constexpr int kRT_W = kRT_I + 2, kRT_PL = kRT_W * (kRT_J + 2);
 constexpr int kRT_PER = (kRT_PL + kRT_I * kRT_J - 1) / (kRT_I * kRT_J);  // plane elements per thread
 
-// u, v, w, rho (and with kL nuT and kappaT) from the ring of shared planes
-// (slot of plane k = k & 3), the rest from global memory around c0.
-template <bool kL>
+// planes in flight beyond k + 1, planes of the ring, and whether the
+// accumulators are staged
+constexpr int rhs_ahead(bool les, int N) { return les || N > 1 ? 1 : 3; }
+constexpr int rhs_ring(bool les, int N) { return 3 + rhs_ahead(les, N); }
+constexpr bool rhs_stage_q(bool first, int N, bool les) { return !first && N == 1 && !les; }
+
+// u, v, w, rho (and with kL nuT and kappaT) from the ring of shared planes,
+// the rest from global memory around c0.
+template <bool kL, int kRing>
 struct TileAcc {
-  const double* sm;  // [field u v w rho (nuT kappaT)][slot][j + 1][i + 1]
-  int idx;           // (ty + 1) * kRT_W + tx + 1
-  int k;
+  const double* sm;  // [field u v w rho (nuT kappaT)][slot][j + 1][i + 1], at (ty + 1, tx + 1)
+  int so[3];         // offsets of the slots of planes k - 1, k, k + 1
   const NSDev& D;
   int64_t c0;
   __device__ __forceinline__ double f(int fi, int a, int b, int c) const {
-    return sm[(fi * 4 + ((k + c) & 3)) * kRT_PL + idx + b * kRT_W + a];
+    return sm[fi * kRing * kRT_PL + so[c + 1] + b * kRT_W + a];
   }
   __device__ __forceinline__ double u(int a, int b, int c) const { return f(0, a, b, c); }
   __device__ __forceinline__ double v(int a, int b, int c) const { return f(1, a, b, c); }
@@ -317,8 +327,13 @@ struct TileAcc {
   }
 };
 
-// shared-memory bytes of k_rhs_accum: four planes of 4 (6 with kL) fields
-constexpr size_t rhs_smem_bytes(bool les) { return (size_t)(les ? 6 : 4) * 4 * kRT_PL * sizeof(double); }
+// shared-memory bytes of k_rhs_accum: the ring of 4 (6 with kL) fields, and
+// of the four accumulators where they are staged
+constexpr size_t rhs_smem_bytes(bool first, bool les, int N) {
+  return ((size_t)(les ? 6 : 4) * rhs_ring(les, N) * kRT_PL +
+          (rhs_stage_q(first, N, les) ? 4 * (rhs_ahead(les, N) + 1) * kRT_I * kRT_J : 0)) *
+         sizeof(double);
+}
 
 template <bool kFirst, bool kU, bool kL, int N>
 __global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(const __grid_constant__ NSMany<N> P, double a1,
@@ -329,7 +344,8 @@ __global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(const __grid_con
   const int m_ = N > 1 ? blockIdx.z / zb : 0;
   const NSDev& D = P.d[m_];
   const double dt = dts.v[m_];
-  constexpr int NF = kL ? 6 : 4;
+  constexpr int NF = kL ? 6 : 4, R = rhs_ring(kL, N), RQ = rhs_ahead(kL, N) + 1, NT = kRT_I * kRT_J;
+  constexpr bool kQ = rhs_stage_q(kFirst, N, kL);
   const int t = threadIdx.x;
   const int tx = t & 31, ty = t >> 5;
   const int i0 = 2 + blockIdx.x * kRT_I, j0 = 2 + blockIdx.y * kRT_J, k0 = 2 + (blockIdx.z - m_ * zb) * per;
@@ -344,54 +360,82 @@ __global__ void __launch_bounds__(kRT_I * kRT_J, 2) k_rhs_accum(const __grid_con
     const int gi = i0 - 1 + e % kRT_W, gj = j0 - 1 + e / kRT_W;
     off[q] = (e < kRT_PL && gi <= D.X && gj <= D.Y) ? NS_IX(gi, gj, 1) : -1;
   }
-  // plane p of the four fields into its ring slot, by asynchronous copies
-  // (elements outside the array are never read and are skipped)
-  auto fetch = [&](int p) {
+  const bool in = i <= D.nx + 1 && j <= D.ny + 1;
+  double* const sq = sm + NF * R * kRT_PL + t;  // [slot][q][thread]
+  auto copy = [](const double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+  };
+  // plane p of the fields into ring slot `slot`, and plane p - 1 of the
+  // accumulators, by asynchronous copies (elements outside the array are
+  // never read and are skipped)
+  auto fetch = [&](int p, int slot, int qslot) {
+    if (p <= kend) {
 #pragma unroll
-    for (int q = 0; q < kRT_PER; ++q) {
-      if (off[q] < 0) continue;
-      const int e = t + q * kRT_I * kRT_J;
+      for (int q = 0; q < kRT_PER; ++q) {
+        if (off[q] < 0) continue;
 #pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const unsigned dst =
-            (unsigned)__cvta_generic_to_shared(&sm[(f * 4 + (p & 3)) * kRT_PL + e]);
-        const double* src = fld[f] + off[q] + D.XY * (p - 1);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
+        for (int f = 0; f < NF; ++f)
+          copy(&sm[(f * R + slot) * kRT_PL + t + q * NT], fld[f] + off[q] + D.XY * (p - 1));
+      }
+      if (kQ && in && p > k0) {
+        const int64_t c = NS_IX(i, j, p - 1);
+        double* const s = sq + qslot * 4 * NT;
+        copy(s, D.qu + c);
+        copy(s + NT, D.qv + c);
+        copy(s + 2 * NT, D.qw + c);
+        copy(s + 3 * NT, D.qr + c);
       }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
-  for (int p = k0 - 1; p <= k0 + 1; ++p) fetch(p);
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-  const bool in = i <= D.nx + 1 && j <= D.ny + 1;
+  // plane p is in slot (p - (k0 - 1)) % R, q of plane p in (p - k0) % RQ
+#pragma unroll
+  for (int p = 0; p < R - 1; ++p) fetch(k0 - 1 + p, p, p >= 2 ? p - 2 : 0);
+  int s0 = 0, s1 = 1, s2 = 2, sf = R - 1, sc = 0, sn = RQ - 1;
   for (int k = k0; k < kend; ++k) {
-    const bool pre = k + 1 < kend;  // the next plane's neighbour k+2 is needed
-    if (pre) fetch(k + 2);
+    // plane k + 1 and q of plane k have arrived; everyone is done with k - 2
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(R - 4) : "memory");
+    __syncthreads();
+    fetch(k + R - 2, sf, sn);
     if (in) {
       const int64_t c = NS_IX(i, j, k);
-      // the accumulators' loads first: their latency overlaps the RHS
-      const double q0u = kFirst ? 0.0 : D.qu[c];
-      const double q0v = kFirst ? 0.0 : D.qv[c];
-      const double q0w = kFirst ? 0.0 : D.qw[c];
-      const double q0r = kFirst ? 0.0 : D.qr[c];
-      const TileAcc<kL> A{sm, (ty + 1) * kRT_W + tx + 1, k, D, c};
+      // accumulators that are not staged: their latency overlaps the RHS
+      double qu = 0.0, qv = 0.0, qw = 0.0, qr = 0.0;
+      if (!kFirst && !kQ) {
+        qu = D.qu[c];
+        qv = D.qv[c];
+        qw = D.qw[c];
+        qr = D.qr[c];
+      }
+      const TileAcc<kL, R> A{sm + (ty + 1) * kRT_W + tx + 1, {s0 * kRT_PL, s1 * kRT_PL, s2 * kRT_PL}, D, c};
       const double fu = rhs_u<kU>(D, A, i, j, k);
       const double fv = rhs_v<kU>(D, A, i, j, k);
       const double fw = rhs_w<kU>(D, A, i, j, k);
       const double fr = rhs_scalar<true, kU>(D, A, i, j, k);
-      D.qu[c] = a1 * q0u + a2 * fu * dt;
-      D.qv[c] = a1 * q0v + a2 * fv * dt;
-      D.qw[c] = a1 * q0w + a2 * fw * dt;
-      D.qr[c] = a1 * q0r + a2 * fr * dt;
+      if (kQ) {
+        const double* const q = sq + sc * 4 * NT;
+        qu = q[0];
+        qv = q[NT];
+        qw = q[2 * NT];
+        qr = q[3 * NT];
+      }
+      D.qu[c] = a1 * qu + a2 * fu * dt;
+      D.qv[c] = a1 * qv + a2 * fv * dt;
+      D.qw[c] = a1 * qw + a2 * fw * dt;
+      D.qr[c] = a1 * qr + a2 * fr * dt;
       if (D.scal1_on) {
         const double fs = rhs_scalar<false, kU>(D, A, i, j, k);
         const double q0s = kFirst ? 0.0 : D.qs[c];
         D.qs[c] = a1 * q0s + a2 * fs * dt;
       }
     }
-    if (pre) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
+    s0 = s1;
+    s1 = s2;
+    s2 = s2 + 1 == R ? 0 : s2 + 1;
+    sf = sf + 1 == R ? 0 : sf + 1;
+    sc = sc + 1 == RQ ? 0 : sc + 1;
+    sn = sn + 1 == RQ ? 0 : sn + 1;
   }
 }
 
@@ -994,6 +1038,9 @@ __global__ void k_clip(NSDev D, double* a, double vmin, double vmax) {
 // ------------------------------------------------------------ Psource
 // NSsolver.F90:2167-2223 (its ghost pass is not needed: the multigrid
 // reads the interior of the right-hand side only).
+// Bound by DRAM; one plane at a time kept too few loads in flight (57 % of
+// its rate at 256x128x256, 55 us).
+constexpr int kCellU = 4;
 template <int N>
 __global__ void __launch_bounds__(kCellCols) k_psource(const __grid_constant__ NSMany<N> P,
                                                        const __grid_constant__ NSScal<N> rdts, int per) {
@@ -1001,16 +1048,32 @@ __global__ void __launch_bounds__(kCellCols) k_psource(const __grid_constant__ N
   const NSDev& D = P.d[N > 1 ? blockIdx.z : 0];
   const double rdt = rdts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
-  for (int k = k0; k < kend; ++k) {
-    const double rk = D.rz[k - 1];
-    const double H = 0.5;
-    const double v = ((rk * FA(D.u, i, j, k) - rk * FA(D.u, i - 1, j, k)) * MT(D.rdxc, i) +
-                      (rk * FA(D.v, i, j, k) - rk * FA(D.v, i, j - 1, k)) * MT(D.rdyc, j) +
-                      (H * (D.rz[k] + rk) * FA(D.w, i, j, k) - H * (rk + D.rz[k - 2]) * FA(D.w, i, j, k - 1)) *
-                          MT(D.rdzc, k)) *
-                     rdt;
-    FA(D.psrc, i, j, k) = 0.0 + v;
-  }
+  const double dxi = MT(D.rdxc, i), dyj = MT(D.rdyc, j), H = 0.5;
+  // U planes, their loads before the first store
+  auto planes = [&](auto U, int k1) {
+    double u0[U.value], u1[U.value], v0[U.value], v1[U.value], w[U.value + 1];
+    w[0] = FA(D.w, i, j, k1 - 1);
+#pragma unroll
+    for (int q = 0; q < U.value; ++q) {
+      u0[q] = FA(D.u, i, j, k1 + q);
+      u1[q] = FA(D.u, i - 1, j, k1 + q);
+      v0[q] = FA(D.v, i, j, k1 + q);
+      v1[q] = FA(D.v, i, j - 1, k1 + q);
+      w[q + 1] = FA(D.w, i, j, k1 + q);
+    }
+#pragma unroll
+    for (int q = 0; q < U.value; ++q) {
+      const int k = k1 + q;
+      const double rk = D.rz[k - 1];
+      const double v = ((rk * u0[q] - rk * u1[q]) * dxi + (rk * v0[q] - rk * v1[q]) * dyj +
+                        (H * (D.rz[k] + rk) * w[q + 1] - H * (rk + D.rz[k - 2]) * w[q]) * MT(D.rdzc, k)) *
+                       rdt;
+      FA(D.psrc, i, j, k) = 0.0 + v;
+    }
+  };
+  int k = k0;
+  for (; k + kCellU <= kend; k += kCellU) planes(std::integral_constant<int, kCellU>{}, k);
+  for (; k < kend; ++k) planes(std::integral_constant<int, 1>{}, k);
 }
 
 // ------------------------------------------------------ Pgrad + ghosts
@@ -1020,6 +1083,7 @@ __global__ void __launch_bounds__(kCellCols) k_psource(const __grid_constant__ N
 // hist (may be null): the interior of p is also copied there (the history
 // of the pressure initial guess).  kU: r is 1 on every plane, so the
 // divisions by r are left out (x / 1.0 == x exactly in IEEE arithmetic).
+// Bound by DRAM, like k_psource (one plane at a time: 56 % of its rate, 91 us).
 template <bool kU, int N>
 __global__ void __launch_bounds__(kCellCols) k_pgrad(const __grid_constant__ NSMany<N> P,
                                                      const __grid_constant__ NSScal<N> dts,
@@ -1029,21 +1093,40 @@ __global__ void __launch_bounds__(kCellCols) k_pgrad(const __grid_constant__ NSM
   const double dt = dts.v[N > 1 ? blockIdx.z : 0];
   CELL_COLUMN();
   const int kend_w = D.nz + 1 - D.ew;
-  const double* __restrict__ p = D.p;
-  for (int k = k0; k < kend; ++k) {
-    const double rk = kU ? 1.0 : D.rz[k - 1];
-    const double pk = FA(p, i, j, k);
-    if (hist) FA(hist, i, j, k) = pk;
-    const double pr = kU ? pk : pk / rk;
-    const double pe = kU ? FA(p, i + 1, j, k) : FA(p, i + 1, j, k) / rk;
-    const double pn = kU ? FA(p, i, j + 1, k) : FA(p, i, j + 1, k) / rk;
-    FA(D.u, i, j, k) = FA(D.u, i, j, k) - (pe - pr) * MT(D.rdxe, i) * dt;
-    FA(D.v, i, j, k) = FA(D.v, i, j, k) - (pn - pr) * MT(D.rdye, j) * dt;
-    if (k <= kend_w) {
-      const double pt = kU ? FA(p, i, j, k + 1) : FA(p, i, j, k + 1) / D.rz[k];
-      FA(D.w, i, j, k) = FA(D.w, i, j, k) - (pt - pr) * MT(D.rdze, k) * dt;
+  const double* p = D.p;
+  const double dxi = MT(D.rdxe, i), dyj = MT(D.rdye, j);
+  // U planes, their loads before the first store
+  auto planes = [&](auto U, int k1) {
+    double pk[U.value + 1], pe[U.value], pn[U.value], u[U.value], v[U.value], w[U.value];
+    pk[0] = FA(p, i, j, k1);
+#pragma unroll
+    for (int q = 0; q < U.value; ++q) {
+      pk[q + 1] = FA(p, i, j, k1 + q + 1);
+      pe[q] = FA(p, i + 1, j, k1 + q);
+      pn[q] = FA(p, i, j + 1, k1 + q);
+      u[q] = FA(D.u, i, j, k1 + q);
+      v[q] = FA(D.v, i, j, k1 + q);
+      w[q] = FA(D.w, i, j, k1 + q);
     }
-  }
+#pragma unroll
+    for (int q = 0; q < U.value; ++q) {
+      const int k = k1 + q;
+      const double rk = kU ? 1.0 : D.rz[k - 1];
+      if (hist) FA(hist, i, j, k) = pk[q];
+      const double pr = kU ? pk[q] : pk[q] / rk;
+      const double xe = kU ? pe[q] : pe[q] / rk;
+      const double yn = kU ? pn[q] : pn[q] / rk;
+      FA(D.u, i, j, k) = u[q] - (xe - pr) * dxi * dt;
+      FA(D.v, i, j, k) = v[q] - (yn - pr) * dyj * dt;
+      if (k <= kend_w) {
+        const double zt = kU ? pk[q + 1] : pk[q + 1] / D.rz[k];
+        FA(D.w, i, j, k) = w[q] - (zt - pr) * MT(D.rdze, k) * dt;
+      }
+    }
+  };
+  int k = k0;
+  for (; k + kCellU <= kend; k += kCellU) planes(std::integral_constant<int, kCellU>{}, k);
+  for (; k < kend; ++k) planes(std::integral_constant<int, 1>{}, k);
 }
 
 // -------------------------------------------------------------- calcdt
@@ -1384,8 +1467,8 @@ static void rhs_launch(const NSMany<N>& P, const NSScal<N>& dt, int members, dou
   const int per = fill_planes(D, (int64_t)g.x * g.y * members, kRT_K, 4);
   const int zb = (D.nz + per - 1) / per;
   g.z = (unsigned)(zb * members);
-  const size_t sm = rhs_smem_bytes(kL);
-  if (kL) set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL, N>, (int)sm);
+  const size_t sm = rhs_smem_bytes(kFirst, kL, N);
+  set_smem_limit_once((const void*)k_rhs_accum<kFirst, kU, kL, N>, (int)sm);
   launch_chained(k_rhs_accum<kFirst, kU, kL, N>, g, kRT_I * kRT_J, sm, s, P, a1, a2, dt, per, zb);
 }
 
