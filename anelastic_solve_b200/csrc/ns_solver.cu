@@ -183,10 +183,11 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
     ANEL_CUDA_TRY(cudaMemset(d_les_, 0, 4 * (size_t)Z * sizeof(double)));
   }
   if (ns->vmodel != ANEL_MODEL_DNS) {
-    // per-column eliminated diagonal of the LES CN solve: one array per
-    // variable up to kCNSharedCells cells
-    cnb_n_ = (int64_t)nx_ * ny_ * nz_ <= kCNSharedCells ? 5 : 1;
-    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, cnb_n_ * G_ * sizeof(double)));
+    // per-column eliminated diagonal of the LES CN solve: four variables'
+    // up to kCNSharedCells cells, the fourth in the pressure source, which is
+    // formed after the column solves (the multigrid reads its interior only)
+    cnb_n_ = (int64_t)nx_ * ny_ * nz_ <= kCNSharedCells ? 4 : 1;
+    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, (cnb_n_ > 1 ? 3 : 1) * G_ * sizeof(double)));
   }
   // metrics
   std::vector<double> met;
@@ -355,14 +356,14 @@ int NSSolver::cn_set(int slot, CNSet* set) const {
 }
 
 // LES: as many variables per launch as there are scratch arrays for their
-// eliminated diagonals (five on grids that one variable does not fill the
+// eliminated diagonals (four on grids that one variable does not fill the
 // GPU with, else one).
 void NSSolver::cn_solve_les(int slot, double a3, double dt_rk, int variant, cudaStream_t s) {
   CNSet set[5];
   const int n = cn_set(slot, set);
   for (int v = 0; v < n; v += cnb_n_) {
     const int m = n - v < cnb_n_ ? n - v : cnb_n_;
-    for (int q = 0; q < m; ++q) set[v + q].b = d_cnb_ + (size_t)q * G_;
+    for (int q = 0; q < m; ++q) set[v + q].b = q < 3 ? d_cnb_ + (size_t)q * G_ : D_.psrc;
     launch_cn_les(D_, set + v, m, a3, dt_rk, variant, s);
   }
 }
