@@ -81,6 +81,28 @@ __device__ __forceinline__ void spec_norm_finish(SpecNorm& N, const SpecDev& D, 
   }
 }
 
+// The passes wait for DRAM with 16 to 24 warps per SM (the transforms' stages
+// fill the registers), so each block asks L2 for what the block that will
+// take its place reads: the block `resident` further on, in launch order.
+// 512x256x512: forward 539 -> 515 us, y 260 -> 219, update 411 -> 361, check
+// 326 -> 314, the whole solve 2.79 -> 2.58 ms; twice the distance gives
+// nothing.
+__device__ __forceinline__ void spec_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ bool spec_next_block(int resident, int& bx, int& by) {
+  const int at = blockIdx.x + gridDim.x * blockIdx.y + resident;
+  by = at / gridDim.x;
+  bx = at - by * gridDim.x;
+  return by < (int)gridDim.y;
+}
+// rows of n elements of esize bytes, `stride` elements apart, by lines
+__device__ __forceinline__ void spec_prefetch_rows(const void* p, int rows, int n, int64_t stride, int esize) {
+  const int per = 128 / esize, lines = (n + per - 1) / per;
+  for (int t = threadIdx.x; t < rows * lines; t += blockDim.x) {
+    const int r = t / lines;
+    spec_prefetch(static_cast<const char*>(p) + (r * stride + (int64_t)(t - r * lines) * per) * esize);
+  }
+}
+
 // f - A phi at interior cell offset c of plane k (1-based), whose
 // coefficients are (c5, c6, dg)
 __device__ __forceinline__ double spec_resid(const SpecDev& D, const double* __restrict__ p, int64_t c, double f,
@@ -108,6 +130,13 @@ __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
   const double c5 = D.coef[k - 1], c6 = D.coef[D.Z + k - 1];
   const double dg = -(2.0 * D.a1 + 2.0 * D.a3 + D.coef[2 * D.Z + k - 1] + D.coef[3 * D.Z + k - 1]);
   const int64_t base = cidx(2, 2 + 2 * pair0, k, D.X, D.XY);
+  int bx, by;
+  if (spec_next_block(148 * 2, bx, by)) {
+    const int64_t c = cidx(2, 2 + 2 * bx * D.pairs, 2 + by, D.X, D.XY);
+    const int rows = min(2 * D.pairs, D.ny - 2 * bx * D.pairs);
+    spec_prefetch_rows(phi + c, rows, n, D.X, 8);
+    spec_prefetch_rows(rhs + c, rows, n, D.X, 8);
+  }
   double rr = 0.0, ff = 0.0;
   auto in = [&](int q, int i) {
     const int64_t c = base + (int64_t)(2 * q) * D.X + i;
@@ -158,6 +187,11 @@ __global__ void __launch_bounds__(256, 3) k_spec_update(SpecDev D) {
   const int64_t base = cidx(2, 2 + 2 * pair0, k, D.X, D.XY);
   const double2* __restrict__ w =
       D.work + (int64_t)b * D.nz * D.nu + (int64_t)(k - 2) * D.nu + (int64_t)(2 * pair0) * h;
+  spec_prefetch_rows(phi + base, 2 * nb, n, D.X, 8);
+  int bx, by;
+  if (spec_next_block(148 * 3, bx, by))
+    spec_prefetch_rows(D.work + ((int64_t)b * D.nz + by) * D.nu + (int64_t)(2 * bx * D.pairs) * h,
+                       min(2 * D.pairs, D.ny - 2 * bx * D.pairs), h, h, 16);
   auto in = [&](int q, int i) {
     const bool up = i > h;
     const int c = i == h ? 0 : (up ? n - i : i);
@@ -211,6 +245,9 @@ __global__ void __launch_bounds__(256, 3) k_spec_y(SpecDev D) {
   const int nb = min(W, h - c0);
   double2* w = D.work + (int64_t)b * D.nz * D.nu + (int64_t)blockIdx.y * D.nu + c0;
   double2* col = xsm + 2 * W * n;  // column 0 of the forward transform
+  int bx, by;
+  if (spec_next_block(148 * 3, bx, by))
+    spec_prefetch_rows(D.work + ((int64_t)b * D.nz + by) * D.nu + bx * W, n, min(W, h - bx * W), h, 16);
   const bool zero = c0 == 0;
   auto in = [&](int q, int i) {
     if (kInv) {
@@ -305,6 +342,9 @@ __global__ void __launch_bounds__(512) k_spec_z(SpecDev D, int ntiles) {
       sh = c == 0 ? D.l0[l] : D.lx[c] + D.ly[l];
       if (c == 0 && (l == 0 || l == D.ny / 2)) live = false;
     }
+    if (tile + (int)gridDim.x < ntiles - 1)
+      for (int q = w; q < M; q += 8)
+        if (r0 + q < D.nz) spec_prefetch(work + (int64_t)(r0 + q) * D.nu + (int64_t)(tile + gridDim.x) * 8);
     double2 v[M];
 #pragma unroll
     for (int q = 0; q < M; ++q)
@@ -457,7 +497,17 @@ __global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int per, int nzb)
       pc = pp;
     };
     int k = k0;
+    const int lane = threadIdx.x & 31;
+    const bool ahead = lane == 0 || lane == 16 || lane == 31;
     for (; k + kCheckK <= kend; k += kCheckK) {
+      if (ahead) {
+#pragma unroll
+        for (int q = 0; q < kCheckK; ++q)
+          if (k + 2 * kCheckK + q < kend) {
+            spec_prefetch(rhs + c + (2 * kCheckK + q) * D.XY);
+            spec_prefetch(phi + c + (2 * kCheckK + q + 1) * D.XY);
+          }
+      }
       double v[kCheckK][6];
 #pragma unroll
       for (int q = 0; q < kCheckK; ++q) {
