@@ -16,10 +16,13 @@ namespace anel {
 void set_error(const char* fmt, ...);
 const char* last_error();
 
+// A failed call's error is taken out of the runtime too, or the next call's
+// check_launch would report it again (a failed allocation is not sticky).
 #define ANEL_CUDA_TRY(expr)                                                              \
   do {                                                                                   \
     cudaError_t _e = (expr);                                                             \
     if (_e != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       ::anel::set_error("%s failed: %s (%s:%d)", #expr, cudaGetErrorString(_e), __FILE__, \
                         __LINE__);                                                       \
       return ANEL_ERR_CUDA;                                                              \

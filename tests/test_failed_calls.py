@@ -1,0 +1,44 @@
+"""What a context does after a call that failed: an allocation that the
+device cannot meet is an error of that call alone, and leaves no state that
+later calls would take for that of a call that succeeded."""
+import numpy as np
+import pytest
+
+from anelastic_solve_b200 import abi
+from anelastic_solve_b200 import grid as G
+from anelastic_solve_b200._lib import AnelError
+from anelastic_solve_b200.mg import MGSolver
+
+from .helpers import compatible, field, levels_for, mg_params
+from .test_mg_batch import to_dev, to_host
+
+pytestmark = pytest.mark.gpu
+
+
+def zline(g, tol):
+    return mg_params(g, levels=levels_for(g)[:2] + (1,), mode=abi.MODE_METRIC, smoother=abi.SMOOTHER_ZLINE,
+                     maxcy=60, tolmax=tol, stop=abi.STOP_RESID, precision=abi.PREC_MIXED)
+
+
+def refused_batch(s, phi, rhs, members):
+    """A batch of more members than the device has memory for (every member
+    the same two arrays: the call fails before its first launch)."""
+    with pytest.raises(AnelError) as e:
+        s.solve_batch([phi] * members, [rhs] * members)
+    assert e.value.code == abi.ERR_CUDA
+
+
+def test_solve_after_a_batch_without_memory():
+    """64^3 by V-cycles: 2 MB of FP32 levels a member."""
+    g = G.shear_layer_grid(64, 64, 64, stretched=True)
+    rhs = to_dev(compatible(field(g, np.random.default_rng(1)), g, abi.MODE_METRIC))
+    s = MGSolver(g, zline(g, 1e-10))
+    want, got = rhs * 0.0, rhs * 0.0
+    s.solve(want, rhs)
+    refused_batch(s, got, rhs, 200_000)
+    s.solve(got, rhs)
+    assert s.last_report.status == abi.OK
+    np.testing.assert_array_equal(to_host(got), to_host(want))
+    (rep,) = s.solve_batch([got], [rhs])
+    assert rep.status == abi.OK and rep.iter == 0
+    s.close()
