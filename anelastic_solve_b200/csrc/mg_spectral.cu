@@ -730,24 +730,33 @@ int spec_build(SpecHost& H, SpecState* h_one, int nx, int ny, int nz, double a1,
 int spec_reserve(SpecHost& H, int n) {
   SpecDev& D = H.d;
   if (n <= H.cap) return ANEL_OK;
-  cudaFree(H.d_buf);
-  H.d_buf = nullptr;
-  if (H.h_st && H.h_st != H.h_one) cudaFreeHost(H.h_st);
-  H.h_st = nullptr;
-  H.cap = 0;
   const int64_t fwd = (int64_t)((D.ny / 2 + D.pairs - 1) / D.pairs) * D.nz;
-  D.pstride = 2 * std::max<int64_t>(fwd, (int64_t)check_cols(D) * check_zblocks(D));
+  const int64_t pstride = 2 * std::max<int64_t>(fwd, (int64_t)check_cols(D) * check_zblocks(D));
   const size_t st = (size_t)n * sizeof(SpecState), cnt = ((size_t)n * sizeof(unsigned) + 15) / 16 * 16;
-  ANEL_CUDA_TRY(cudaMalloc(&H.d_buf, st + cnt + (size_t)n * D.pstride * sizeof(double)));
-  ANEL_CUDA_TRY(cudaMemset(H.d_buf, 0, st + cnt));
-  if (n == 1) H.h_st = H.h_one;
-  else ANEL_CUDA_TRY(cudaHostAlloc(&H.h_st, (size_t)n * sizeof(SpecState), cudaHostAllocMapped));
-  D.hst = H.h_st;
-  char* p = reinterpret_cast<char*>(H.d_buf);
+  // the new buffers first: where one of them cannot be had, the old ones
+  // stay and solves within their room go on
+  double* buf = nullptr;
+  SpecState* host = H.h_one;
+  cudaError_t e = cudaMalloc(&buf, st + cnt + (size_t)n * pstride * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemset(buf, 0, st + cnt);
+  if (e == cudaSuccess && n > 1) e = cudaHostAlloc(&host, (size_t)n * sizeof(SpecState), cudaHostAllocMapped);
+  if (e != cudaSuccess) {
+    cudaFree(buf);
+    cudaGetLastError();
+    set_error("direct solve: no memory for %d members: %s", n, cudaGetErrorString(e));
+    return ANEL_ERR_CUDA;
+  }
+  cudaFree(H.d_buf);
+  if (H.h_st && H.h_st != H.h_one) cudaFreeHost(H.h_st);
+  H.d_buf = buf;
+  H.h_st = host;
+  H.cap = n;
+  char* p = reinterpret_cast<char*>(buf);
+  D.pstride = pstride;
+  D.hst = host;
   D.st = reinterpret_cast<SpecState*>(p);
   D.count = reinterpret_cast<unsigned*>(p + st);
   D.part = reinterpret_cast<double*>(p + st + cnt);
-  H.cap = n;
   return ANEL_OK;
 }
 

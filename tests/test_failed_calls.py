@@ -42,3 +42,35 @@ def test_solve_after_a_batch_without_memory():
     (rep,) = s.solve_batch([got], [rhs])
     assert rep.status == abi.OK and rep.iter == 0
     s.close()
+
+
+def test_direct_solve_after_a_batch_without_memory():
+    """512x256x512: 0.26 MB of partial sums a member, so a batch of 800 000
+    fails at the direct solve's first buffer; the buffers that it had before,
+    for one member and for two, go on."""
+    import torch
+
+    g = G.shear_layer_grid(512, 256, 512, stretched=True)
+    gen = torch.Generator("cuda").manual_seed(1)
+    rhs = torch.zeros(g.ghosted[::-1], dtype=torch.float64, device="cuda")
+    f = torch.randn(g.shape[::-1], generator=gen, dtype=torch.float64, device="cuda")
+    dz = torch.from_numpy(g.z.dxc[1:-1].copy()).cuda()
+    rhs[1:-1, 1:-1, 1:-1] = f - (f.mean(dim=(1, 2)) * dz).sum() / dz.sum()
+    s = MGSolver(g, zline(g, 1e-11))
+    want = torch.zeros_like(rhs)
+    s.solve(want, rhs)
+    assert s.last_report.reserved == 1
+    for reserved in (1, 2):
+        if reserved == 2:
+            two = [torch.zeros_like(rhs) for _ in range(2)]
+            s.solve_batch(two, [rhs, rhs])
+        got = torch.zeros_like(rhs)
+        refused_batch(s, got, rhs, 800_000)
+        s.solve(got, rhs)
+        assert s.last_report.status == abi.OK and s.last_report.reserved == 1
+        assert torch.equal(got, want)
+    got = [torch.zeros_like(rhs) for _ in range(2)]
+    for rep in s.solve_batch(got, [rhs, rhs]):
+        assert rep.status == abi.OK
+    assert torch.equal(got[0], want) and torch.equal(got[1], want)
+    s.close()
