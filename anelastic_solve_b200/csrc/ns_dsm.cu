@@ -498,9 +498,9 @@ enum { DY_MODS, DY_FMODS, DY_C0, DY_FC0 = DY_C0 + 3, DY_L1 = DY_FC0 + 3, DY_L2, 
        DY_TMP, DY_N };
 
 int NSSolver::ensure_dyn() {
-  if (d_dyn_) return ANEL_OK;
+  if (dyn_area_ > 0.0) return ANEL_OK;  // set last: a call that ran out of memory is taken up again
   const int X = nx_ + 2, Y = ny_ + 2, Z = nz_ + 2;
-  ANEL_CUDA_TRY(cudaMalloc(&d_dyn_, (size_t)DY_N * G_ * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_dyn_, (size_t)DY_N * G_));
   ANEL_CUDA_TRY(cudaMemset(d_dyn_, 0, (size_t)DY_N * G_ * sizeof(double)));
   // dxc[X] dyc[Y] delg[Z] profiles[2Z], then the plane partial sums
   std::vector<double> h;
@@ -516,14 +516,14 @@ int NSSolver::ensure_dyn() {
   h.insert(h.end(), dg.begin(), dg.end());
   h.resize(h.size() + 2 * (size_t)Z, 0.0);
   const size_t nm = h.size();
-  ANEL_CUDA_TRY(cudaMalloc(&d_dyn_m_, (nm + 2 * (size_t)plane_part_doubles(D_)) * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_dyn_m_, nm + 2 * (size_t)plane_part_doubles(D_)));
   ANEL_CUDA_TRY(cudaMemcpy(d_dyn_m_, h.data(), nm * sizeof(double), cudaMemcpyHostToDevice));
   dyn_part_ = d_dyn_m_ + nm;
   // coordinates for center_velocity: xe xc ye yc ze zc
   std::vector<double> ax;
   for (int d = 0; d < 3; ++d)
     for (int q = 0; q < 2; ++q) ax.insert(ax.end(), m_[d][q].begin(), m_[d][q].end());
-  ANEL_CUDA_TRY(cudaMalloc(&d_dyn_axes_, ax.size() * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_dyn_axes_, ax.size()));
   ANEL_CUDA_TRY(cudaMemcpy(d_dyn_axes_, ax.data(), ax.size() * sizeof(double), cudaMemcpyHostToDevice));
   {
     const int len[3] = {X, Y, Z};

@@ -512,10 +512,10 @@ int NSSolver::get_fields(const anel_fields* f, int mem, cudaStream_t s) {
 }
 
 int NSSolver::ensure_hist() {
-  if (hist_[0][0]) return ANEL_OK;
+  if (hist_[2][1]) return ANEL_OK;  // the last of them
   for (auto& h : hist_)
     for (double*& a : h) {
-      ANEL_CUDA_TRY(cudaMalloc(&a, G_ * sizeof(double)));
+      ANEL_CUDA_TRY(need_doubles(&a, G_));
       ANEL_CUDA_TRY(cudaMemset(a, 0, G_ * sizeof(double)));
     }
   return ANEL_OK;
@@ -1102,27 +1102,27 @@ int NSSolver::set_diagnostics(int on, int mode, const int* stretched) {
 }
 
 int NSSolver::ensure_diag() {
-  if (d_diag_) return ANEL_OK;
+  if (dev1_) return ANEL_OK;  // made last: an earlier call that ran out of memory is taken up again
   ANEL_CUDA_TRY(cudaSetDevice(device_));
   const int X = nx_ + 2, Y = ny_ + 2, Z = nz_ + 2;
-  ANEL_CUDA_TRY(cudaMalloc(&d_diag_, 26 * (size_t)Z * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_diag_, 26 * (size_t)Z));
   ANEL_CUDA_TRY(cudaMemset(d_diag_, 0, 26 * (size_t)Z * sizeof(double)));
-  ANEL_CUDA_TRY(cudaMalloc(&d_dgA_, G_ * sizeof(double)));
-  ANEL_CUDA_TRY(cudaMalloc(&d_dgB_, G_ * sizeof(double)));
-  ANEL_CUDA_TRY(cudaMalloc(&d_dgpart_, (size_t)plane_part_doubles(D_) * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_dgA_, G_));
+  ANEL_CUDA_TRY(need_doubles(&d_dgB_, G_));
+  ANEL_CUDA_TRY(need_doubles(&d_dgpart_, (size_t)plane_part_doubles(D_)));
   // dxc[X] dyc[Y] xe[X] xc[X] ye[Y] yc[Y] ze[Z] zc[Z] (m_[d] = xe xc dxe dxc rdxe rdxc)
   std::vector<double> h;
   for (const std::vector<double>* v : {&m_[0][3], &m_[1][3], &m_[0][0], &m_[0][1], &m_[1][0], &m_[1][1],
                                        &m_[2][0], &m_[2][1]})
     h.insert(h.end(), v->begin(), v->end());
-  ANEL_CUDA_TRY(cudaMalloc(&d_dgm_, h.size() * sizeof(double)));
+  ANEL_CUDA_TRY(need_doubles(&d_dgm_, h.size()));
   ANEL_CUDA_TRY(cudaMemcpy(d_dgm_, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
   // Area of avgX1X2 (Average.F90:351-356), summed in its order
   double area = 0.0;
   for (int j = 2; j <= ny_ + 1; ++j)
     for (int i = 2; i <= nx_ + 1; ++i) area = area + m_[0][3][i - 1] * m_[1][3][j - 1];
   diag_area_ = area;
-  ANEL_CUDA_TRY(cudaEventCreate(&dev0_));
+  if (!dev0_) ANEL_CUDA_TRY(cudaEventCreate(&dev0_));
   ANEL_CUDA_TRY(cudaEventCreate(&dev1_));
   (void)X;
   (void)Y;

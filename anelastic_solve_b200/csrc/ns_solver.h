@@ -10,6 +10,11 @@ namespace anel {
 
 // One shear-layer member: device-resident fields, its multigrid context
 // and the sub-step schedule of NSsolver/rk_ss (NSsolver.F90:63-583).
+// n doubles of device memory at *p, unless they are there already
+inline cudaError_t need_doubles(double** p, size_t n) {
+  return *p ? cudaSuccess : cudaMalloc(p, n * sizeof(double));
+}
+
 class NSSolver {
  public:
   static NSSolver* create(const anel_grid_desc* g, const anel_mg_params* mg, const anel_ns_params* ns,

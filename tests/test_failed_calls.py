@@ -1,13 +1,16 @@
 """What a context does after a call that failed: an allocation that the
 device cannot meet is an error of that call alone, and leaves no state that
 later calls would take for that of a call that succeeded."""
+import contextlib
+
 import numpy as np
 import pytest
 
-from anelastic_solve_b200 import abi
+from anelastic_solve_b200 import abi, shear
 from anelastic_solve_b200 import grid as G
 from anelastic_solve_b200._lib import AnelError
 from anelastic_solve_b200.mg import MGSolver
+from anelastic_solve_b200.ns import NSSolver
 
 from .helpers import compatible, field, levels_for, mg_params
 from .test_mg_batch import to_dev, to_host
@@ -74,3 +77,56 @@ def test_direct_solve_after_a_batch_without_memory():
         assert rep.status == abi.OK
     assert torch.equal(got[0], want) and torch.equal(got[1], want)
     s.close()
+
+
+@contextlib.contextmanager
+def memory_left(nbytes):
+    """All device memory but nbytes is taken."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - nbytes, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        hog.untyped_storage().resize_(0)
+        torch.cuda.empty_cache()
+
+
+def stepper(g, seed, **phys):
+    f = shear.shear_layer_fields(g, amp=1e-2, seed=seed)
+    kw = dict(Re=1000.0, Pr=1.0, g=-0.1, cfl=0.5, dtmax=1e9, ew=1, scal1_on=0)
+    s = NSSolver(g, zline(g, 1e-11), abi.make_ns_params(**{**kw, **phys}))
+    s.set_fields({k: f[k] for k in ("u", "v", "w", "p", "rho", "scal1", "r", "densityBG")})
+    s.project()
+    return s
+
+
+FIELDS = ("u", "v", "w", "p", "rho")
+# 256x128x128: a field of 36 MB; less than one is left free where a call is
+# to fail, and the kernels that it launches have been loaded by then
+GRID, LEFT = (256, 128, 128), 24 << 20
+
+
+def test_a_set_up_that_ran_out_of_memory_is_taken_up_again():
+    """The plane statistics' arrays, a small one and then two of the size of
+    a field: a call that could not have them all fails, and a step with
+    memory back equals that of a context that never lacked any."""
+    g = G.shear_layer_grid(*GRID, stretched=True)
+    a, b = stepper(g, 1), stepper(g, 1)
+    for s in (a, b):
+        s.set_diagnostics(True)
+    a.step(1)
+    with memory_left(LEFT), pytest.raises(AnelError) as e:
+        b.compute_diagnostics()
+    assert e.value.code == abi.ERR_CUDA
+    b.step(1)
+    want, got = a.get_fields(FIELDS), b.get_fields(FIELDS)
+    for k in FIELDS:
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    want, got = a.diagnostics(), b.diagnostics()
+    for k, v in want.items():
+        np.testing.assert_array_equal(got[k], v, err_msg=k)
+    a.close()
+    b.close()
