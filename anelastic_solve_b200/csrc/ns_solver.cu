@@ -849,12 +849,12 @@ int NSSolver::step_end(double delt, cudaStream_t s, anel_step_report* r, bool di
   r->time = time_;
   nstep_ += 1;
   // divergence of the step's result and the next step's CFL maximum (a
-  // cohort takes its members' together)
+  // cohort takes its members' together, and calls divergence_taken then)
   if (div) {
     const int st = divergence_pass(s, true);
     if (st != ANEL_OK) return st;
+    divergence_taken();
   }
-  cfl_ready_ = div_ready_ = true;
   return ANEL_OK;
 }
 
@@ -1037,6 +1037,7 @@ int NSSolver::step_cohort(NSSolver* const* ms, int n, int nsteps, MGSolver* bmg,
       if (st != ANEL_OK) return st;
     }
     launch_divergence(devs.data(), divs.data(), n, true, s);
+    for (int b = 0; b < n; ++b) ms[b]->divergence_taken();
   }
   ANEL_CUDA_TRY(cudaEventRecord(ms[0]->ev1_, s));
   ANEL_CUDA_TRY(cudaEventSynchronize(ms[0]->ev1_));

@@ -114,6 +114,7 @@ class NSSolver {
   int divergence_pass(cudaStream_t s, bool with_cfl);
   int divergence_read(cudaStream_t s, double* out);
   int divergence_prepare();
+  void divergence_taken() { cfl_ready_ = div_ready_ = true; }  // the pass that step_end wants is on the stream
   DivSet divergence_set() const;
   CNFactorSet cn_factor_set() const;
   bool cn_step_slots(double delt);

@@ -130,3 +130,28 @@ def test_a_set_up_that_ran_out_of_memory_is_taken_up_again():
         np.testing.assert_array_equal(got[k], v, err_msg=k)
     a.close()
     b.close()
+
+
+def failed_cohort(members):
+    with memory_left(LEFT), pytest.raises(AnelError) as e:
+        NSSolver.step_cohort(members, 1)
+    assert e.value.code == abi.ERR_CUDA
+
+
+def test_time_step_after_a_cohort_step_that_failed_at_its_end():
+    """The second member's statistics find no memory after the fields have
+    been advanced and before the cohort's divergence pass: the first member's
+    next time step comes from the fields it has now."""
+    g = G.shear_layer_grid(*GRID, stretched=True)
+    ms = [stepper(g, seed) for seed in (1, 2)]
+    ms[0].set_diagnostics(True)
+    before = NSSolver.step_cohort(ms, 2)[0]
+    ms[1].set_diagnostics(True)
+    failed_cohort(ms)
+    ref = stepper(g, 1)
+    ref.set_fields(ms[0].get_fields(FIELDS + ("scal1",)))
+    want = ref.step(1)
+    got = ms[0].step(1)
+    assert got.nstep == before.nstep + 2 and got.dt == want.dt != before.dt
+    for s in (*ms, ref):
+        s.close()
