@@ -411,12 +411,11 @@ ZRule NSSolver::zrule(int vt) const {
   return R;
 }
 
-// The CN factors of slots slot0 .. slot0 + n - 1 for their rkdt (cn_rkdt_):
-// what launch_cn_factors needs of this member.
-CNFactorSet NSSolver::cn_factor_set() const {
+// What launch_cn_factors needs of this member for the slots' rkdt.
+CNFactorSet NSSolver::cn_factor_set(const double* rkdt) const {
   CNFactorSet c{};
   c.dst = d_cn_;
-  for (int q = 0; q < 3; ++q) c.rkdt[q] = cn_rkdt_[q];
+  for (int q = 0; q < 3; ++q) c.rkdt[q] = rkdt[q];
   for (int vi = 0; vi < 5; ++vi)
     for (int f = 0; f < 2; ++f) {
       c.type[vi][f] = prm_.tb[2][f][kVarCode[vi] - 1];
@@ -427,22 +426,25 @@ CNFactorSet NSSolver::cn_factor_set() const {
 
 int NSSolver::cn_factors(int slot, double rkdt, cudaStream_t s) {
   if (cn_rkdt_[slot] == rkdt) return ANEL_OK;
-  cn_rkdt_[slot] = rkdt;
   const NSDev* d = &D_;
-  const CNFactorSet c = cn_factor_set();
+  double want[3] = {cn_rkdt_[0], cn_rkdt_[1], cn_rkdt_[2]};
+  want[slot] = rkdt;
+  const CNFactorSet c = cn_factor_set(want);
   launch_cn_factors(&d, &c, 1, slot, 1, s);
+  cn_rkdt_[slot] = rkdt;
   return ANEL_OK;
 }
 
-// A step's three factor sets; false when they are there already.
-bool NSSolver::cn_step_slots(double delt) {
+// A step's three factor sets; false when they are there already.  The slots
+// count as made (cn_made) once the launch that makes them is on the stream.
+bool NSSolver::cn_step_slots(double delt, CNFactorSet* set) const {
   const double dtr[3] = {1.0 / 3.0 * delt, 5.0 / 12.0 * delt, 1.0 / 4.0 * delt};
-  bool make = false;
-  for (int q = 0; q < 3; ++q) {
-    make = make || cn_rkdt_[q] != dtr[q];
-    cn_rkdt_[q] = dtr[q];
-  }
-  return make;
+  *set = cn_factor_set(dtr);
+  return cn_rkdt_[0] != dtr[0] || cn_rkdt_[1] != dtr[1] || cn_rkdt_[2] != dtr[2];
+}
+
+void NSSolver::cn_made(const CNFactorSet& set) {
+  for (int q = 0; q < 3; ++q) cn_rkdt_[q] = set.rkdt[q];
 }
 
 CNFacHost NSSolver::fac(int slot, int vi) const {
@@ -781,10 +783,11 @@ int NSSolver::step_begin(cudaStream_t s, double* delt_out) {
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
   const int st = step_begin_finish(s, delt_out);
   if (st != ANEL_OK) return st;
-  if (cn_step_slots(*delt_out)) {
+  CNFactorSet c;
+  if (cn_step_slots(*delt_out, &c)) {
     const NSDev* d = &D_;
-    const CNFactorSet c = cn_factor_set();
     launch_cn_factors(&d, &c, 1, 0, 3, s);
+    cn_made(c);
   }
   return ANEL_OK;
 }
@@ -988,13 +991,13 @@ int NSSolver::step_cohort(NSSolver* const* ms, int n, int nsteps, MGSolver* bmg,
     for (int b = 0; b < n; ++b) {
       const int st = ms[b]->step_begin_finish(s, &delt[b]);
       if (st != ANEL_OK) return st;
-      make = ms[b]->cn_step_slots(delt[b]) || make;
-      facs[b] = ms[b]->cn_factor_set();
+      make = ms[b]->cn_step_slots(delt[b], &facs[b]) || make;
     }
     if (make) {
       if (together) launch_cn_factors(devs.data(), facs.data(), n, 0, 3, s);
       else
         for (int b = 0; b < n; ++b) launch_cn_factors(&devs[b], &facs[b], 1, 0, 3, s);
+      for (int b = 0; b < n; ++b) ms[b]->cn_made(facs[b]);
     }
     for (int q = 0; q < 3; ++q) {
       if (together) {

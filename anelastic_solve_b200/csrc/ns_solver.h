@@ -116,8 +116,9 @@ class NSSolver {
   int divergence_prepare();
   void divergence_taken() { cfl_ready_ = div_ready_ = true; }  // the pass that step_end wants is on the stream
   DivSet divergence_set() const;
-  CNFactorSet cn_factor_set() const;
-  bool cn_step_slots(double delt);
+  CNFactorSet cn_factor_set(const double* rkdt) const;
+  bool cn_step_slots(double delt, CNFactorSet* set) const;
+  void cn_made(const CNFactorSet& set);
   int cfl_word_ = 0;  // of h_red_: where calcdt_take finds the CFL maximum
   int divergence_take(double* out);
   int les_coeffs(cudaStream_t s);

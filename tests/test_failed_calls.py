@@ -155,3 +155,22 @@ def test_time_step_after_a_cohort_step_that_failed_at_its_end():
     assert got.nstep == before.nstep + 2 and got.dt == want.dt != before.dt
     for s in (*ms, ref):
         s.close()
+
+
+def test_column_factors_after_a_cohort_step_that_failed_at_its_start():
+    """The second member's dynamic model finds no memory before the members'
+    Crank-Nicolson factors are made for their new time steps: the first
+    member's next step makes them."""
+    g = G.shear_layer_grid(*GRID, stretched=True)
+    kw = dict(les=True, Re=5e4, models=(abi.MODEL_DSM,) * 3)
+    ref, *ms = (stepper(g, seed, **kw) for seed in (1, 1, 2))
+    for s in (ref, ms[0]):
+        s.step(1)
+    failed_cohort(ms)
+    ref.step(1)
+    ms[0].step(1)
+    want, got = ref.get_fields(FIELDS), ms[0].get_fields(FIELDS)
+    for k in FIELDS:
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    for s in (*ms, ref):
+        s.close()
