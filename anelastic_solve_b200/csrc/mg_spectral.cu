@@ -803,10 +803,21 @@ void launch_spec_update(const SpecDev& D, int nm, cudaStream_t s) {
 }
 
 void launch_spec_check(const SpecDev& D, int nm, cudaStream_t s) {
-  const int nzb = check_zblocks(D);
-  const dim3 g((unsigned)((D.nx + 31) / 32), (unsigned)((D.ny + 7) / 8), (unsigned)(nzb * nm));
-  launch_chained(k_spec_check, g, 256, 0, s, D, check_planes(D), nzb);
-  count_launch();
+  // member and z-block share blockIdx.z, 65535 at most: more members take
+  // more launches (two z-planes per block of a 16x16x64 member: 2047 fit)
+  const int nzb = check_zblocks(D), most = 65535 / nzb;
+  for (int b = 0; b < nm; b += most) {
+    const int m = std::min(most, nm - b);
+    SpecDev P = D;
+    if (P.mt) P.mt += b;
+    P.st += b;
+    P.hst += b;
+    P.count += b;
+    P.part += b * P.pstride;
+    const dim3 g((unsigned)((D.nx + 31) / 32), (unsigned)((D.ny + 7) / 8), (unsigned)(nzb * m));
+    launch_chained(k_spec_check, g, 256, 0, s, P, check_planes(D), nzb);
+    count_launch();
+  }
 }
 
 }  // namespace anel
