@@ -29,6 +29,12 @@ const char* last_error();
     }                                                                                    \
   } while (0)
 
+// Clears (cudaMemset) and uploads from pageable memory may still be under way
+// when they return, on the legacy default stream; the contexts' own streams
+// are non-blocking and not ordered after it.  Every set-up that made some
+// ends with this wait.
+inline cudaError_t setup_wait() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // Every kernel launch of this library goes through count_launch() so the
 // total is observable through anel_kernel_launch_count().
 // The thread-local count gives per-call reports (solve, step) that are

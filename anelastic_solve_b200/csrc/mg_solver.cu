@@ -1124,11 +1124,16 @@ int MGSolver::upload_coefficients() {
     }
   }
   op_hash_ = h;
+  int st = ANEL_OK;
   if (prm_.precision != ANEL_PREC_MIXED && prm_.smoother == ANEL_SMOOTHER_RBPGS) {
-    const int st = upload_rb_shared();
-    return st != ANEL_OK ? st : build_rb_levels();
+    st = upload_rb_shared();
+    if (st == ANEL_OK) st = build_rb_levels();
+  } else if (spec_want_) {
+    st = build_spec();
   }
-  return spec_want_ ? build_spec() : ANEL_OK;
+  if (st != ANEL_OK) return st;
+  ANEL_CUDA_TRY(setup_wait());
+  return ANEL_OK;
 }
 
 // The coarse levels the FP64 red-black cycle does in one block: from the
@@ -2105,6 +2110,7 @@ int MGSolver::batch_reserve(int n) {
   ANEL_CUDA_TRY(cudaMalloc(&d_bconv_, (size_t)n * sizeof(BatchConv)));
   ANEL_CUDA_TRY(cudaHostAlloc(&h_bmt_, (size_t)n * sizeof(MemberIO), cudaHostAllocDefault));
   ANEL_CUDA_TRY(cudaHostAlloc(&h_bconv_, (size_t)n * sizeof(BatchConv), cudaHostAllocDefault));
+  ANEL_CUDA_TRY(setup_wait());
   bcap_ = n;
   return ANEL_OK;
 }

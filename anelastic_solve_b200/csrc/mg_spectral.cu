@@ -739,6 +739,8 @@ int spec_reserve(SpecHost& H, int n) {
   SpecState* host = H.h_one;
   cudaError_t e = cudaMalloc(&buf, st + cnt + (size_t)n * pstride * sizeof(double));
   if (e == cudaSuccess) e = cudaMemset(buf, 0, st + cnt);
+  // the kernels count on counters that start at zero
+  if (e == cudaSuccess) e = setup_wait();
   if (e == cudaSuccess && n > 1) e = cudaHostAlloc(&host, (size_t)n * sizeof(SpecState), cudaHostAllocMapped);
   if (e != cudaSuccess) {
     cudaFree(buf);

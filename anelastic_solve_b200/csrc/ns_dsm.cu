@@ -537,6 +537,7 @@ int NSSolver::ensure_dyn() {
   double area = 0.0;
   for (int j = 2; j <= ny_ + 1; ++j)
     for (int i = 2; i <= nx_ + 1; ++i) area = area + m_[0][3][i - 1] * m_[1][3][j - 1];
+  ANEL_CUDA_TRY(setup_wait());
   dyn_area_ = area;
   (void)X;
   (void)Y;

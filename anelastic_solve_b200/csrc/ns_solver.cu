@@ -375,6 +375,7 @@ int NSSolver::upload_profiles() {
   std::vector<double> pr(rz_);
   pr.insert(pr.end(), bgz_.begin(), bgz_.end());
   ANEL_CUDA_TRY(cudaMemcpy(d_prof_, pr.data(), pr.size() * sizeof(double), cudaMemcpyHostToDevice));
+  ANEL_CUDA_TRY(setup_wait());  // init's clears too
   for (double& v : cn_rkdt_) v = -1.0;  // factors depend on r
   return ANEL_OK;
 }
@@ -520,6 +521,7 @@ int NSSolver::ensure_hist() {
       ANEL_CUDA_TRY(need_doubles(&a, G_));
       ANEL_CUDA_TRY(cudaMemset(a, 0, G_ * sizeof(double)));
     }
+  ANEL_CUDA_TRY(setup_wait());
   return ANEL_OK;
 }
 
@@ -1126,6 +1128,7 @@ int NSSolver::ensure_diag() {
   for (int j = 2; j <= ny_ + 1; ++j)
     for (int i = 2; i <= nx_ + 1; ++i) area = area + m_[0][3][i - 1] * m_[1][3][j - 1];
   diag_area_ = area;
+  ANEL_CUDA_TRY(setup_wait());
   if (!dev0_) ANEL_CUDA_TRY(cudaEventCreate(&dev0_));
   ANEL_CUDA_TRY(cudaEventCreate(&dev1_));
   (void)X;
