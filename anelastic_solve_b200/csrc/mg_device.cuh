@@ -870,7 +870,7 @@ __device__ __forceinline__ T prolong_corr(const DevLevel<T>& Cl, int i, int j, i
   const T wx0 = cx ? ((i & 1) ? T(3) : T(1)) : T(1), wx1 = cx ? ((i & 1) ? T(1) : T(3)) : T(0);
   const T wy0 = cy ? ((j & 1) ? T(3) : T(1)) : T(1), wy1 = cy ? ((j & 1) ? T(1) : T(3)) : T(0);
   const T wz0 = cz ? ((k & 1) ? T(3) : T(1)) : T(1), wz1 = cz ? ((k & 1) ? T(1) : T(3)) : T(0);
-  const T* __restrict__ pc = Cl.phi + cidx(ic, jc, kc, Cl.X, Cl.XY);
+  const T* pc = Cl.phi + cidx(ic, jc, kc, Cl.X, Cl.XY);
   const int64_t ox = 1, oy = Cl.X, oz = Cl.XY;
   if constexpr (cx && cy && cz) {
     // order (x,y,z) offsets: 000 010 001 011 100 110 101 111

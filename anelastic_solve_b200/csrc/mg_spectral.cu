@@ -105,7 +105,7 @@ __device__ __forceinline__ void spec_prefetch_rows(const void* p, int rows, int 
 
 // f - A phi at interior cell offset c of plane k (1-based), whose
 // coefficients are (c5, c6, dg)
-__device__ __forceinline__ double spec_resid(const SpecDev& D, const double* __restrict__ p, int64_t c, double f,
+__device__ __forceinline__ double spec_resid(const SpecDev& D, const double* p, int64_t c, double f,
                                              double c5, double c6, double dg) {
   double acc = D.a1 * (p[c - 1] + p[c + 1]);
   acc += D.a3 * (p[c - D.X] + p[c + D.X]);
@@ -122,8 +122,8 @@ __global__ void __launch_bounds__(256, 2) k_spec_forward(SpecDev D, int test) {
   extern __shared__ double2 xsm[];
   const int b = blockIdx.z;
   if (!test && !D.st[b].act) return;  // the whole block
-  const double* __restrict__ phi = D.mt ? D.mt[b].phi : D.phi;
-  const double* __restrict__ rhs = D.mt ? D.mt[b].rhs : D.rhs;
+  const double* phi = D.mt ? D.mt[b].phi : D.phi;
+  const double* rhs = D.mt ? D.mt[b].rhs : D.rhs;
   const int n = D.nx, row = spec_row(n), k = 2 + blockIdx.y;
   const int pair0 = blockIdx.x * D.pairs;
   const int nb = min(D.pairs, D.ny / 2 - pair0);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, 3) k_spec_update(SpecDev D) {
   const int pair0 = blockIdx.x * D.pairs;
   const int nb = min(D.pairs, D.ny / 2 - pair0);
   const int64_t base = cidx(2, 2 + 2 * pair0, k, D.X, D.XY);
-  const double2* __restrict__ w =
+  const double2* w =
       D.work + (int64_t)b * D.nz * D.nu + (int64_t)(k - 2) * D.nu + (int64_t)(2 * pair0) * h;
   spec_prefetch_rows(phi + base, 2 * nb, n, D.X, 8);
   int bx, by;
@@ -473,8 +473,8 @@ __global__ void __launch_bounds__(256) k_spec_check(SpecDev D, int per, int nzb)
   chain_enter();
   const int b = blockIdx.z / nzb;
   if (!D.st[b].act) return;
-  const double* __restrict__ phi = D.mt ? D.mt[b].phi : D.phi;
-  const double* __restrict__ rhs = D.mt ? D.mt[b].rhs : D.rhs;
+  const double* phi = D.mt ? D.mt[b].phi : D.phi;
+  const double* rhs = D.mt ? D.mt[b].rhs : D.rhs;
   const int i = 2 + blockIdx.x * 32 + (threadIdx.x & 31), j = 2 + blockIdx.y * 8 + (threadIdx.x >> 5);
   const int zb = blockIdx.z - b * nzb;
   const int k0 = 2 + zb * per, kend = min(k0 + per, D.nz + 2);  // exclusive

@@ -258,13 +258,13 @@ __global__ void __launch_bounds__(kDynI * kDynJ) k_dyn_filter(const __grid_const
 
 // a field to a field
 struct DynFieldIn {
-  const double* __restrict__ a;
+  const double* a;
   __device__ __forceinline__ void operator()(const NSDev& D, int i, int j, int k, double (&v)[1]) const {
     v[0] = a[NS_IX(i, j, k)];
   }
 };
 struct DynFieldOut {
-  double* __restrict__ a;
+  double* a;
   __device__ __forceinline__ void operator()(const NSDev&, int64_t o, int, const double (&v)[1]) const { a[o] = v[0]; }
 };
 

@@ -626,7 +626,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
 // autotuner chooses from (launch_cn); the arithmetic does not depend on
 // them.
 template <int kVar, int U>
-__device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ fld, const double* __restrict__ q,
+__device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ fld, const double* q,
                                           const CNFac& F, double a3, double rkdt, const ZRule& R) {
   extern __shared__ double cn_sm[];
   const int n = D.nz + 2;
@@ -833,8 +833,8 @@ __device__ __forceinline__ double les_sup(const double* s_c, const double* s_re,
 
 template <int kVar, bool kU, int U>
 __device__ __forceinline__ void cn_column_les(const NSDev& D, double* __restrict__ fld,
-                                              const double* __restrict__ q, const CNFac& F, double a3, double rkdt,
-                                              const ZRule& R, const double* __restrict__ kT,
+                                              const double* q, const CNFac& F, double a3, double rkdt,
+                                              const ZRule& R, const double* kT,
                                               double* __restrict__ bb) {
   extern __shared__ double cn_sm[];
   const int n = D.nz + 2;

@@ -6,9 +6,10 @@
 // visible.  What overlaps is the launch itself (about 1 us per kernel on the
 // small grids, whose sub-step is a chain of some 13 kernels of 3-10 us), so
 // the results and the order of all memory accesses are those of plain
-// launches.  No kernel launched this way has a __restrict__ pointer to const
-// among its parameters: loads through one count as loads of constant memory
-// and need not stay behind the wait.
+// launches.  No kernel launched this way reads through a __restrict__ pointer
+// to const, be it a parameter, a member of one, a local or a parameter of a
+// function that it calls: such loads count as loads of constant memory and
+// need not stay behind the wait.
 #pragma once
 
 #include <cuda_runtime.h>
