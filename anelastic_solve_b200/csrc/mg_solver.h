@@ -27,8 +27,9 @@ class MGSolver {
   int set_density_device(const double* r, cudaStream_t s);
 
   // mg_solver on device arrays: d_phi inout (ghosted FP64), d_rhs in.
-  // FP64 scratch of the fine level's ghosted size, free between solves
-  double* work_array() const { return d_phi64_[ngrid_]; }
+  // two FP64 scratch arrays of the fine level's ghosted size, free between
+  // solves (every solve fills them before it reads them)
+  double* work_array(int q) const { return q ? d_src64_[ngrid_] : d_phi64_[ngrid_]; }
   int solve_device(double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);
   // Same with host arrays (copies in and out through pinned staging).
   int solve_host(double* phi, const double* rhs, cudaStream_t s, anel_mg_report* rep);

@@ -184,9 +184,9 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
   }
   if (ns->vmodel != ANEL_MODEL_DNS) {
     // per-column eliminated diagonal of the LES CN solve: four variables'
-    // up to kCNSharedCells cells, the fourth in the multigrid's work array
+    // up to kCNSharedCells cells, two of them in the multigrid's work arrays
     cnb_n_ = (int64_t)nx_ * ny_ * nz_ <= kCNSharedCells ? 4 : 1;
-    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, (cnb_n_ > 1 ? 3 : 1) * G_ * sizeof(double)));
+    ANEL_CUDA_TRY(cudaMalloc(&d_cnb_, (cnb_n_ > 1 ? 2 : 1) * G_ * sizeof(double)));
   }
   // metrics
   std::vector<double> met;
@@ -362,7 +362,7 @@ void NSSolver::cn_solve_les(int slot, double a3, double dt_rk, int variant, cuda
   const int n = cn_set(slot, set);
   for (int v = 0; v < n; v += cnb_n_) {
     const int m = n - v < cnb_n_ ? n - v : cnb_n_;
-    for (int q = 0; q < m; ++q) set[v + q].b = q < 3 ? d_cnb_ + (size_t)q * G_ : mg_->work_array();
+    for (int q = 0; q < m; ++q) set[v + q].b = q < 2 ? d_cnb_ + (size_t)q * G_ : mg_->work_array(q - 2);
     launch_cn_les(D_, set + v, m, a3, dt_rk, variant, s);
   }
 }

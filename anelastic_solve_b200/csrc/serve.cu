@@ -199,8 +199,7 @@ class ServeEngine {
     job->key = std::to_string(g.nx) + "x" + std::to_string(g.ny) + "x" + std::to_string(g.nz) + ":" +
                std::to_string(h);
     // device memory of a context: FP64 fields (14, +3 eddy fields, +2 for the
-    // LES-CN scratch, which is 3 fields up to 16 Mi cells and fits with the
-    // slack), multigrid (FP64 fine pair, FP32 levels) and slack
+    // LES-CN scratch), multigrid (FP64 fine pair, FP32 levels) and slack
     const int64_t G = (int64_t)(g.nx + 2) * (g.ny + 2) * (g.nz + 2);
     const bool les_any = nk.vmodel != ANEL_MODEL_DNS || nk.rmodel != ANEL_MODEL_DNS ||
                          nk.smodel != ANEL_MODEL_DNS;

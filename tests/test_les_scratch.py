@@ -34,3 +34,19 @@ def test_pressure_source_is_no_scratch(scal1_on):
         psrc[1:-1, 1:-1, 1:-1] = 0.0
         assert not psrc.any()
     s.close()
+
+
+@pytest.mark.parametrize("n", [(64, 64, 64), (256, 128, 264), (384, 192, 192), (256, 256, 256)])
+def test_les_context_within_what_a_serving_job_is_charged(n):
+    """Device memory of an LES context after a step, against the serving
+    engine's estimate: 14 fields, 3 eddy fields, 2 of scratch, 32 bytes a cell
+    for the multigrid and 64 MB."""
+    import torch
+
+    g = G.shear_layer_grid(*n, stretched=True)
+    before = torch.cuda.mem_get_info()[0]
+    s = les(g)
+    s.step(1)
+    used = before - torch.cuda.mem_get_info()[0]
+    s.close()
+    assert used <= np.prod(g.ghosted) * (8 * 19 + 32) + (64 << 20)
