@@ -1690,7 +1690,6 @@ int MGSolver::solve_vcycle(double* d_phi, const double* d_rhs, cudaStream_t s, a
 // Up to kSpecCorrections direct corrections of n members on the stream,
 // one host synchronisation per correction; the members' states are then in
 // spec_.h_st and ev1_ marks the end.
-constexpr int kSpecCorrections = 2;
 void MGSolver::solve_spec(int n, const SpecDev& D0, const DevLevel<double>& F, cudaStream_t s) {
   SpecDev D = D0;
   D.tol = prm_.tolmax;
@@ -1732,7 +1731,7 @@ int MGSolver::spec_report(const SpecState& st, double* d_phi, const double* d_rh
   const int done = st.iter;
   if (!st.conv && st.act && std::isfinite(st.rel)) {
     const int rc = solve_vcycle(d_phi, d_rhs, s, rep);
-    if (rc == ANEL_OK) rep->iter = std::min(rep->iter + done, prm_.maxcy);
+    if (rc == ANEL_OK) rep->iter += done;
     return rc;
   }
   rep->iter = st.conv ? done : prm_.maxcy + 1;
@@ -1902,7 +1901,7 @@ int MGSolver::build_solve_graph(double* d_phi, const double* d_rhs, cudaStream_t
   const ColLevel Ec = C32(ng);
   ConvState* cs = static_cast<ConvState*>(d_conv_);
   const double tol = prm_.tolmax;
-  const int maxcy = prm_.maxcy;
+  const int maxcy = vcycle_limit();
   cudaGraph_t g = nullptr;
   bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
   cudaGraphConditionalHandle h{};
@@ -2127,7 +2126,7 @@ int MGSolver::build_batch_graph(int n, cudaStream_t s) {
   const ColLevel Ec = C32b(ng, n);
   BatchConv* cs = static_cast<BatchConv*>(d_bconv_);
   const double tol = prm_.tolmax;
-  const int maxcy = prm_.maxcy;
+  const int maxcy = vcycle_limit();
   cudaGraph_t g = nullptr;
   bool ok = cudaGraphCreate(&g, 0) == cudaSuccess;
   cudaGraphConditionalHandle h{};
@@ -2281,7 +2280,7 @@ int MGSolver::solve_mixed(double* d_phi, const double* d_rhs, cudaStream_t s,
   int iter = 0;
   bool conv = false;
   const ColLevel Ec = col_ ? C32(ng) : ColLevel{};
-  for (iter = 0; iter <= prm_.maxcy; ++iter) {
+  for (iter = 0; iter <= vcycle_limit(); ++iter) {
     if (col_) launch_col_resid_store(Fu, d_phi, d_rhs, Ec, d_part_, d_norm_, s);
     else launch_resid_store(Fu, d_phi, d_rhs, E.src, d_part_, d_norm_, s);
     copy_words(d_norm_, h_pin_, 2, s);
@@ -2292,7 +2291,7 @@ int MGSolver::solve_mixed(double* d_phi, const double* d_rhs, cudaStream_t s,
       conv = true;
       break;
     }
-    if (iter == prm_.maxcy) break;
+    if (iter == vcycle_limit()) break;
     run_cycle32(s);
     if (col_) launch_col_add_correction(Fu, d_phi, Ec, s);
     else launch_add_correction(Fu, d_phi, E.phi, s);

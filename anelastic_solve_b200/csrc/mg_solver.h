@@ -123,6 +123,9 @@ class MGSolver {
   double* d_bspec_ = nullptr;  // spectral work space of a batch
   int build_spec();
   void solve_spec(int n, const SpecDev& D, const DevLevel<double>& F, cudaStream_t s);
+  // a solve's V-cycles: what maxcy leaves after the direct corrections
+  static constexpr int kSpecCorrections = 2;
+  int vcycle_limit() const { return prm_.maxcy - (spec_.ok ? kSpecCorrections : 0); }
   int solve_vcycle(double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);
   int spec_report(const SpecState& st, double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);
   ColLevel C32(int l) const;
