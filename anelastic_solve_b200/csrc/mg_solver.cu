@@ -2227,19 +2227,24 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
     D.work = reinterpret_cast<double2*>(d_bspec_);
     solve_spec(n, D, L64(ngrid_), s);
     ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
-    float ms = 0.f;
-    ANEL_CUDA_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
     const std::vector<SpecState> fin(spec_.h_st, spec_.h_st + n);
     int rc = ANEL_OK;
+    bool more = false;
     for (int b = 0; b < n; ++b) {
       anel_mg_report& r = reps[b];
       r = anel_mg_report{};
       st = spec_report(fin[b], phis[b], rhss[b], s, &r);
       if (st != ANEL_OK && st != ANEL_ERR_NOCONV) return st;
       r.status = st;
-      r.ms = ms;
+      more = more || !r.reserved;
       if (st != ANEL_OK) rc = st;
     }
+    // the batch's device time, V-cycles included
+    if (more) ANEL_CUDA_TRY(cudaEventRecord(ev1_, s));
+    ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
+    float ms = 0.f;
+    ANEL_CUDA_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
+    for (int b = 0; b < n; ++b) reps[b].ms = ms;
     st = check_launch("batched solve");
     if (st == ANEL_OK) st = take_kernel_error("batched solve");
     return st != ANEL_OK ? st : rc;

@@ -43,3 +43,16 @@ def test_corrections_count_towards_the_cycle_limit(n):
         s.close()
     cycle = launches[4] - launches[3]
     assert cycle > 0 and launches[3] - launches[2] < 2 * cycle
+
+
+def test_batch_time_holds_the_cycles():
+    """ms of a batch's reports: 58 V-cycles after the two corrections, so far
+    more than a quarter of a single solve's time."""
+    g, s, rhs = problem(GRIDS[0], 60)
+    for _ in range(2):
+        s.solve(rhs * 0.0, rhs)
+        alone = s.last_report.ms
+        reps = s.solve_batch([rhs * 0.0 for _ in range(3)], [rhs] * 3)
+    s.close()
+    for r in reps:
+        assert r.status == abi.ERR_NOCONV and r.ms == reps[0].ms > 0.25 * alone
