@@ -1724,12 +1724,14 @@ void MGSolver::solve_spec(int n, const SpecDev& D0, const DevLevel<double>& F, c
   }
 }
 
+static bool spec_hands_over(const SpecState& st) { return !st.conv && st.act && std::isfinite(st.rel); }
+
 // The report of a member after its direct corrections; V-cycles go on from
 // there where it needs them.  reserved = 1: the direct solve alone did it.
 int MGSolver::spec_report(const SpecState& st, double* d_phi, const double* d_rhs, cudaStream_t s,
                           anel_mg_report* rep) {
   const int done = st.iter;
-  if (!st.conv && st.act && std::isfinite(st.rel)) {
+  if (spec_hands_over(st)) {
     const int rc = solve_vcycle(d_phi, d_rhs, s, rep);
     if (rc == ANEL_OK) rep->iter += done;
     return rc;
@@ -2055,7 +2057,7 @@ bool MGSolver::batch_capable() const {
   return col_ && prm_.precision == ANEL_PREC_MIXED && gsolve_state_ >= 0;
 }
 
-void MGSolver::batch_free() {
+void MGSolver::batch_free_cycles() {
   if (bgraph_) cudaGraphExecDestroy(bgraph_);
   bgraph_ = nullptr;
   bgraph_n_ = 0;
@@ -2064,32 +2066,61 @@ void MGSolver::batch_free() {
     cudaFree(d_bsrc32_[l]);
     d_bphi32_[l] = d_bsrc32_[l] = nullptr;
   }
-  cudaFree(d_bspec_);
-  d_bspec_ = nullptr;
   cudaFree(d_bdir_);
   cudaFree(d_bpart_);
   cudaFree(d_bnorm_);
+  d_bdir_ = d_bpart_ = d_bnorm_ = nullptr;
+  bcyc_ = 0;
+}
+
+void MGSolver::batch_free() {
+  batch_free_cycles();
+  cudaFree(d_bspec_);
   cudaFree(d_bmt_);
   cudaFree(d_bact_);
   cudaFree(d_bconv_);
   if (h_bmt_) cudaFreeHost(h_bmt_);
   if (h_bconv_) cudaFreeHost(h_bconv_);
-  d_bdir_ = d_bpart_ = d_bnorm_ = nullptr;
+  d_bspec_ = nullptr;
   d_bmt_ = h_bmt_ = nullptr;
   d_bact_ = nullptr;
   d_bconv_ = h_bconv_ = nullptr;
   bcap_ = 0;
 }
 
+// The buffers of n members: their table, flags and states, and those of
+// the direct solve or of the V-cycles; a call that cannot have them all gives back what it got.
 int MGSolver::batch_reserve(int n) {
   if (n <= bcap_) return ANEL_OK;
   ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
   batch_free();
-  if (spec_.ok) {
-    const int st = spec_reserve(spec_, n);
-    if (st != ANEL_OK) return st;
-    ANEL_CUDA_TRY(cudaMalloc(&d_bspec_, (size_t)n * spec_work_doubles(nx_, ny_, nz_) * sizeof(double)));
-  } else {
+  auto reserve = [&]() -> int {
+    if (spec_.ok) {
+      const int st = spec_reserve(spec_, n);
+      if (st != ANEL_OK) return st;
+      ANEL_CUDA_TRY(cudaMalloc(&d_bspec_, (size_t)n * spec_work_doubles(nx_, ny_, nz_) * sizeof(double)));
+    }
+    ANEL_CUDA_TRY(cudaMalloc(&d_bmt_, (size_t)n * sizeof(MemberIO)));
+    ANEL_CUDA_TRY(cudaMalloc(&d_bact_, (size_t)n * sizeof(int)));
+    ANEL_CUDA_TRY(cudaMalloc(&d_bconv_, (size_t)n * sizeof(BatchConv)));
+    ANEL_CUDA_TRY(cudaHostAlloc(&h_bmt_, (size_t)n * sizeof(MemberIO), cudaHostAllocDefault));
+    ANEL_CUDA_TRY(cudaHostAlloc(&h_bconv_, (size_t)n * sizeof(BatchConv), cudaHostAllocDefault));
+    return ANEL_OK;
+  };
+  int st = reserve();
+  if (st == ANEL_OK && !spec_.ok) st = batch_reserve_cycles(n);
+  if (st != ANEL_OK) batch_free();
+  else bcap_ = n;
+  return st;
+}
+
+// The buffers of n members' V-cycles: with the others above, or where a
+// direct batch first hands members over.
+int MGSolver::batch_reserve_cycles(int n) {
+  if (n <= bcyc_) return ANEL_OK;
+  ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
+  batch_free_cycles();
+  auto reserve = [&]() -> int {
     for (int l = 1; l <= ngrid_; ++l) {
       const size_t b = (size_t)fp32_elems(l) * n * sizeof(float);
       ANEL_CUDA_TRY(cudaMalloc(&d_bphi32_[l], b));
@@ -2103,15 +2134,13 @@ int MGSolver::batch_reserve(int n) {
     }
     ANEL_CUDA_TRY(cudaMalloc(&d_bpart_, (size_t)col_resid_part_doubles_members(L64(ngrid_), n) * sizeof(double)));
     ANEL_CUDA_TRY(cudaMalloc(&d_bnorm_, (size_t)2 * n * sizeof(double)));
-  }
-  ANEL_CUDA_TRY(cudaMalloc(&d_bmt_, (size_t)n * sizeof(MemberIO)));
-  ANEL_CUDA_TRY(cudaMalloc(&d_bact_, (size_t)n * sizeof(int)));
-  ANEL_CUDA_TRY(cudaMalloc(&d_bconv_, (size_t)n * sizeof(BatchConv)));
-  ANEL_CUDA_TRY(cudaHostAlloc(&h_bmt_, (size_t)n * sizeof(MemberIO), cudaHostAllocDefault));
-  ANEL_CUDA_TRY(cudaHostAlloc(&h_bconv_, (size_t)n * sizeof(BatchConv), cudaHostAllocDefault));
-  ANEL_CUDA_TRY(setup_wait());
-  bcap_ = n;
-  return ANEL_OK;
+    ANEL_CUDA_TRY(setup_wait());
+    return ANEL_OK;
+  };
+  const int st = reserve();
+  if (st != ANEL_OK) batch_free_cycles();
+  else bcyc_ = n;
+  return st;
 }
 
 int MGSolver::build_batch_graph(int n, cudaStream_t s) {
@@ -2213,61 +2242,87 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
       return ANEL_ERR_ARG;
     }
   int st = batch_reserve(n);
+  if (st == ANEL_OK && !spec_.ok) st = batch_cycles_ready(n, s);
   if (st != ANEL_OK) return st;
-  if (!spec_.ok && bgraph_n_ != n) {
-    st = build_batch_graph(n, s);
-    if (st != ANEL_OK) return st;
-  }
   for (int b = 0; b < n; ++b) h_bmt_[b] = MemberIO{phis[b], rhss[b]};
   ANEL_CUDA_TRY(cudaMemcpyAsync(d_bmt_, h_bmt_, (size_t)n * sizeof(MemberIO), cudaMemcpyHostToDevice, s));
   ANEL_CUDA_TRY(cudaEventRecord(ev0_, s));
-  if (spec_.ok) {
+  for (int b = 0; b < n; ++b) reps[b] = anel_mg_report{};
+  int rc = ANEL_OK;
+  if (!spec_.ok) {
+    std::vector<anel_mg_report*> out(n);
+    for (int b = 0; b < n; ++b) out[b] = reps + b;
+    rc = batch_cycles(n, out.data(), s);
+    if (rc != ANEL_OK && rc != ANEL_ERR_NOCONV) return rc;
+  } else {
     SpecDev D = spec_.d;
     D.mt = d_bmt_;
     D.work = reinterpret_cast<double2*>(d_bspec_);
     solve_spec(n, D, L64(ngrid_), s);
     ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
+    // the members that two corrections leave unconverged go on with V-cycles
+    // together, or one by one where there is no memory for that
     const std::vector<SpecState> fin(spec_.h_st, spec_.h_st + n);
-    int rc = ANEL_OK;
-    bool more = false;
+    std::vector<int> rest;
+    std::vector<anel_mg_report*> out;
+    for (int b = 0; b < n; ++b)
+      if (spec_hands_over(fin[b])) {
+        rest.push_back(b);
+        out.push_back(reps + b);
+      }
+    const int m = (int)rest.size();
+    const bool together = m > 1 && batch_cycles_ready(m, s) == ANEL_OK;
+    if (together) {
+      for (int q = 0; q < m; ++q) h_bmt_[q] = MemberIO{phis[rest[q]], rhss[rest[q]]};
+      ANEL_CUDA_TRY(cudaMemcpyAsync(d_bmt_, h_bmt_, (size_t)m * sizeof(MemberIO), cudaMemcpyHostToDevice, s));
+      rc = batch_cycles(m, out.data(), s);
+      if (rc != ANEL_OK && rc != ANEL_ERR_NOCONV) return rc;
+    }
     for (int b = 0; b < n; ++b) {
       anel_mg_report& r = reps[b];
-      r = anel_mg_report{};
+      if (together && spec_hands_over(fin[b])) {
+        if (r.status == ANEL_OK) r.iter += fin[b].iter;
+        continue;
+      }
       st = spec_report(fin[b], phis[b], rhss[b], s, &r);
       if (st != ANEL_OK && st != ANEL_ERR_NOCONV) return st;
       r.status = st;
-      more = more || !r.reserved;
       if (st != ANEL_OK) rc = st;
     }
     // the batch's device time, V-cycles included
-    if (more) ANEL_CUDA_TRY(cudaEventRecord(ev1_, s));
-    ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
-    float ms = 0.f;
-    ANEL_CUDA_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
-    for (int b = 0; b < n; ++b) reps[b].ms = ms;
-    st = check_launch("batched solve");
-    if (st == ANEL_OK) st = take_kernel_error("batched solve");
-    return st != ANEL_OK ? st : rc;
+    if (m) ANEL_CUDA_TRY(cudaEventRecord(ev1_, s));
   }
+  ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
+  float ms = 0.f;
+  ANEL_CUDA_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
+  for (int b = 0; b < n; ++b) reps[b].ms = ms;
+  st = check_launch("batched solve");
+  if (st == ANEL_OK) st = take_kernel_error("batched solve");
+  return st != ANEL_OK ? st : rc;
+}
+
+// the buffers and the graph of n members' V-cycles
+int MGSolver::batch_cycles_ready(int n, cudaStream_t s) {
+  const int st = batch_reserve_cycles(n);
+  return st != ANEL_OK || bgraph_n_ == n ? st : build_batch_graph(n, s);
+}
+
+// The V-cycles of the first n members of the table, and their reports; ev1_
+// marks the end.
+int MGSolver::batch_cycles(int n, anel_mg_report* const* reps, cudaStream_t s) {
   ANEL_CUDA_TRY(cudaGraphLaunch(bgraph_, s));
   ANEL_CUDA_TRY(cudaEventRecord(ev1_, s));
   ANEL_CUDA_TRY(cudaMemcpyAsync(h_bconv_, d_bconv_, (size_t)n * sizeof(BatchConv), cudaMemcpyDeviceToHost, s));
   ANEL_CUDA_TRY(cudaStreamSynchronize(s));
-  float ms = 0.f;
-  ANEL_CUDA_TRY(cudaEventElapsedTime(&ms, ev0_, ev1_));
-  st = take_kernel_error("batched solve");
-  if (st != ANEL_OK) return st;
   const BatchConv* cv = static_cast<const BatchConv*>(h_bconv_);
   int itmax = 0, rc = ANEL_OK;
   for (int b = 0; b < n; ++b) {
-    anel_mg_report& r = reps[b];
-    r = anel_mg_report{};
+    anel_mg_report& r = *reps[b];
     const bool conv = cv[b].conv != 0;
     r.iter = conv ? cv[b].iter : prm_.maxcy + 1;
     r.relmax = cv[b].rel;
     r.resid = cv[b].rel;
     r.status = conv ? ANEL_OK : ANEL_ERR_NOCONV;
-    r.ms = ms;
     itmax = std::max(itmax, cv[b].iter);
     if (!conv) rc = ANEL_ERR_NOCONV;
   }

@@ -2,13 +2,15 @@
 reach leaves every member unconverged after two corrections."""
 import numpy as np
 import pytest
+import torch
 
 from anelastic_solve_b200 import abi
 from anelastic_solve_b200 import grid as G
+from anelastic_solve_b200._lib import lib
 from anelastic_solve_b200.mg import MGSolver
 
 from .helpers import compatible, field
-from .test_failed_calls import zline
+from .test_failed_calls import memory_left, zline
 from .test_mg_batch import to_dev
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +58,65 @@ def test_batch_time_holds_the_cycles():
     s.close()
     for r in reps:
         assert r.status == abi.ERR_NOCONV and r.ms == reps[0].ms > 0.25 * alone
+
+
+def members(g):
+    """Right-hand sides of a batch: incompatible (the first, third and last),
+    solvable, not finite."""
+    rng = np.random.default_rng(7)
+    good = compatible(field(g, rng), g, abi.MODE_METRIC)
+    bad = [np.asfortranarray(good + 0.1 * field(g, rng) + q) for q in (1, 2, 3)]
+    nan = good.copy(order="F")
+    nan[3, 3, 3] = np.nan
+    return [to_dev(a) for a in (bad[0], good, bad[1], nan, bad[2])]
+
+
+def hand_over_case(n, maxcy):
+    """A context, the members, their solutions and reports alone."""
+    g = G.shear_layer_grid(*n, stretched=True)
+    p = zline(g, 1e-11)
+    p.maxcy = maxcy
+    s, rhs = MGSolver(g, p), members(g)
+    phi, reps = [torch.zeros_like(f) for f in rhs], []
+    for q, f in zip(phi, rhs):
+        s.solve(q, f)
+        reps.append(s.last_report)
+    assert [r.reserved for r in reps] == [0, 1, 0, 1, 0]
+    return s, rhs, phi, reps
+
+
+def assert_batch_equals(s, rhs, phi, reps):
+    got = [torch.zeros_like(f) for f in rhs]
+    for r, w in zip(s.solve_batch(got, rhs), reps):
+        assert (r.status, r.iter, r.reserved) == (w.status, w.iter, w.reserved)
+        np.testing.assert_array_equal([r.resid, r.relmax], [w.resid, w.relmax])
+    for q, w in zip(got, phi):
+        assert torch.equal(q.nan_to_num(), w.nan_to_num())
+
+
+def test_batch_hands_over_together():
+    """Members that need V-cycles get them in one batched loop, with the
+    results of their solves alone, beside members that need none; then in
+    batches of one and two such members."""
+    s, rhs, phi, reps = hand_over_case((16, 8, 64), 12)
+    assert_batch_equals(s, rhs, phi, reps)
+    n0 = lib().anel_kernel_launch_count()
+    assert_batch_equals(s, rhs, phi, reps)
+    assert lib().anel_kernel_launch_count() - n0 < 0.5 * sum(r.launches for r in reps)
+    for pick in (slice(1, 3), slice(1, 5)):
+        assert_batch_equals(s, rhs[pick], phi[pick], reps[pick])
+    s.close()
+
+
+def test_batch_hands_over_one_by_one_without_memory():
+    """Where the batched cycles' levels cannot be had (three members of
+    256x128x128 need 140 MB) the members go on one by one."""
+    s, rhs, phi, reps = hand_over_case((256, 128, 128), 4)
+    s.solve_batch([torch.zeros_like(f) for f in rhs], [rhs[1]] * 5)  # the direct solve's own buffers
+    got = [torch.zeros_like(f) for f in rhs]
+    with memory_left(24 << 20):
+        out = s.solve_batch(got, rhs)
+    assert [(r.status, r.iter) for r in out] == [(r.status, r.iter) for r in reps]
+    for q, w in zip(got, phi):
+        assert torch.equal(q.nan_to_num(), w.nan_to_num())
+    s.close()
