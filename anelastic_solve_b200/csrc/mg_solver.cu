@@ -2057,89 +2057,64 @@ bool MGSolver::batch_capable() const {
   return col_ && prm_.precision == ANEL_PREC_MIXED && gsolve_state_ >= 0;
 }
 
-void MGSolver::batch_free_cycles() {
+void MGSolver::batch_free() {
   if (bgraph_) cudaGraphExecDestroy(bgraph_);
   bgraph_ = nullptr;
   bgraph_n_ = 0;
-  for (int l = 0; l <= ANEL_MAX_LEVELS; ++l) {
-    cudaFree(d_bphi32_[l]);
-    cudaFree(d_bsrc32_[l]);
-    d_bphi32_[l] = d_bsrc32_[l] = nullptr;
-  }
-  cudaFree(d_bdir_);
-  cudaFree(d_bpart_);
-  cudaFree(d_bnorm_);
-  d_bdir_ = d_bpart_ = d_bnorm_ = nullptr;
-  bcyc_ = 0;
-}
-
-void MGSolver::batch_free() {
-  batch_free_cycles();
-  cudaFree(d_bspec_);
-  cudaFree(d_bmt_);
-  cudaFree(d_bact_);
-  cudaFree(d_bconv_);
+  cudaFree(d_batch_);
+  d_batch_ = nullptr;
   if (h_bmt_) cudaFreeHost(h_bmt_);
   if (h_bconv_) cudaFreeHost(h_bconv_);
-  d_bspec_ = nullptr;
-  d_bmt_ = h_bmt_ = nullptr;
-  d_bact_ = nullptr;
-  d_bconv_ = h_bconv_ = nullptr;
+  h_bmt_ = nullptr;
+  h_bconv_ = nullptr;
   bcap_ = 0;
 }
 
-// The buffers of n members: their table, flags and states, and those of
-// the direct solve or of the V-cycles; a call that cannot have them all gives back what it got.
+// All device buffers in one allocation, the FP32 levels first: the fine
+// level's two arrays side by side are the direct solve's spectral work space
+// too, which is over before the members' V-cycles begin.  A call that cannot
+// have all of it gives back what it got.
 int MGSolver::batch_reserve(int n) {
   if (n <= bcap_) return ANEL_OK;
   ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
   batch_free();
-  auto reserve = [&]() -> int {
-    if (spec_.ok) {
-      const int st = spec_reserve(spec_, n);
-      if (st != ANEL_OK) return st;
-      ANEL_CUDA_TRY(cudaMalloc(&d_bspec_, (size_t)n * spec_work_doubles(nx_, ny_, nz_) * sizeof(double)));
+  if (spec_.ok) {
+    const int st = spec_reserve(spec_, n);
+    if (st != ANEL_OK) return st;
+  }
+  size_t at = 0, levels = 0;
+  auto carve = [&](auto** p, size_t count) {
+    const size_t here = at;
+    at = (at + count * sizeof(**p) + 255) / 256 * 256;
+    if (d_batch_) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(d_batch_ + here);
+  };
+  auto layout = [&]() {
+    at = 0;
+    for (int l = ngrid_; l >= 1; --l) {
+      carve(&d_bphi32_[l], (size_t)fp32_elems(l) * n);
+      carve(&d_bsrc32_[l], (size_t)fp32_elems(l) * n);
     }
-    ANEL_CUDA_TRY(cudaMalloc(&d_bmt_, (size_t)n * sizeof(MemberIO)));
-    ANEL_CUDA_TRY(cudaMalloc(&d_bact_, (size_t)n * sizeof(int)));
-    ANEL_CUDA_TRY(cudaMalloc(&d_bconv_, (size_t)n * sizeof(BatchConv)));
+    levels = at;
+    carve(&d_bdir_, dirL_ > 0 ? (size_t)n * dir_.f.nm * dir_.f.nz : 0);
+    carve(&d_bpart_, (size_t)col_resid_part_doubles_members(L64(ngrid_), n));
+    carve(&d_bnorm_, (size_t)2 * n);
+    carve(&d_bmt_, n);
+    carve(&d_bact_, n);
+    carve(reinterpret_cast<BatchConv**>(&d_bconv_), n);
+  };
+  layout();
+  auto reserve = [&]() -> int {
+    ANEL_CUDA_TRY(cudaMalloc(&d_batch_, at));
+    layout();
+    ANEL_CUDA_TRY(cudaMemset(d_batch_, 0, levels));
     ANEL_CUDA_TRY(cudaHostAlloc(&h_bmt_, (size_t)n * sizeof(MemberIO), cudaHostAllocDefault));
     ANEL_CUDA_TRY(cudaHostAlloc(&h_bconv_, (size_t)n * sizeof(BatchConv), cudaHostAllocDefault));
-    return ANEL_OK;
-  };
-  int st = reserve();
-  if (st == ANEL_OK && !spec_.ok) st = batch_reserve_cycles(n);
-  if (st != ANEL_OK) batch_free();
-  else bcap_ = n;
-  return st;
-}
-
-// The buffers of n members' V-cycles: with the others above, or where a
-// direct batch first hands members over.
-int MGSolver::batch_reserve_cycles(int n) {
-  if (n <= bcyc_) return ANEL_OK;
-  ANEL_CUDA_TRY(cudaStreamSynchronize(stream_));
-  batch_free_cycles();
-  auto reserve = [&]() -> int {
-    for (int l = 1; l <= ngrid_; ++l) {
-      const size_t b = (size_t)fp32_elems(l) * n * sizeof(float);
-      ANEL_CUDA_TRY(cudaMalloc(&d_bphi32_[l], b));
-      ANEL_CUDA_TRY(cudaMalloc(&d_bsrc32_[l], b));
-      ANEL_CUDA_TRY(cudaMemset(d_bphi32_[l], 0, b));
-      ANEL_CUDA_TRY(cudaMemset(d_bsrc32_[l], 0, b));
-    }
-    if (dirL_ > 0) {
-      const DirectFac& F = dir_.f;
-      ANEL_CUDA_TRY(cudaMalloc(&d_bdir_, (size_t)n * F.nm * F.nz * sizeof(double)));
-    }
-    ANEL_CUDA_TRY(cudaMalloc(&d_bpart_, (size_t)col_resid_part_doubles_members(L64(ngrid_), n) * sizeof(double)));
-    ANEL_CUDA_TRY(cudaMalloc(&d_bnorm_, (size_t)2 * n * sizeof(double)));
     ANEL_CUDA_TRY(setup_wait());
     return ANEL_OK;
   };
   const int st = reserve();
-  if (st != ANEL_OK) batch_free_cycles();
-  else bcyc_ = n;
+  if (st != ANEL_OK) batch_free();
+  else bcap_ = n;
   return st;
 }
 
@@ -2242,7 +2217,7 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
       return ANEL_ERR_ARG;
     }
   int st = batch_reserve(n);
-  if (st == ANEL_OK && !spec_.ok) st = batch_cycles_ready(n, s);
+  if (st == ANEL_OK && !spec_.ok && bgraph_n_ != n) st = build_batch_graph(n, s);
   if (st != ANEL_OK) return st;
   for (int b = 0; b < n; ++b) h_bmt_[b] = MemberIO{phis[b], rhss[b]};
   ANEL_CUDA_TRY(cudaMemcpyAsync(d_bmt_, h_bmt_, (size_t)n * sizeof(MemberIO), cudaMemcpyHostToDevice, s));
@@ -2257,11 +2232,11 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
   } else {
     SpecDev D = spec_.d;
     D.mt = d_bmt_;
-    D.work = reinterpret_cast<double2*>(d_bspec_);
+    D.work = reinterpret_cast<double2*>(d_bphi32_[ngrid_]);
     solve_spec(n, D, L64(ngrid_), s);
     ANEL_CUDA_TRY(cudaEventSynchronize(ev1_));
     // the members that two corrections leave unconverged go on with V-cycles
-    // together, or one by one where there is no memory for that
+    // together, or one by one on a stream that cannot be captured
     const std::vector<SpecState> fin(spec_.h_st, spec_.h_st + n);
     std::vector<int> rest;
     std::vector<anel_mg_report*> out;
@@ -2271,8 +2246,11 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
         out.push_back(reps + b);
       }
     const int m = (int)rest.size();
-    const bool together = m > 1 && batch_cycles_ready(m, s) == ANEL_OK;
+    const bool together = m > 1 && (bgraph_n_ == m || build_batch_graph(m, s) == ANEL_OK);
     if (together) {
+      // the spectral values out of the fine level's pads and ghosts
+      ANEL_CUDA_TRY(cudaMemsetAsync(d_bphi32_[ngrid_], 0,
+                                    reinterpret_cast<char*>(d_bphi32_[ngrid_ - 1]) - d_batch_, s));
       for (int q = 0; q < m; ++q) h_bmt_[q] = MemberIO{phis[rest[q]], rhss[rest[q]]};
       ANEL_CUDA_TRY(cudaMemcpyAsync(d_bmt_, h_bmt_, (size_t)m * sizeof(MemberIO), cudaMemcpyHostToDevice, s));
       rc = batch_cycles(m, out.data(), s);
@@ -2299,12 +2277,6 @@ int MGSolver::solve_batch(int n, double* const* phis, const double* const* rhss,
   st = check_launch("batched solve");
   if (st == ANEL_OK) st = take_kernel_error("batched solve");
   return st != ANEL_OK ? st : rc;
-}
-
-// the buffers and the graph of n members' V-cycles
-int MGSolver::batch_cycles_ready(int n, cudaStream_t s) {
-  const int st = batch_reserve_cycles(n);
-  return st != ANEL_OK || bgraph_n_ == n ? st : build_batch_graph(n, s);
 }
 
 // The V-cycles of the first n members of the table, and their reports; ev1_

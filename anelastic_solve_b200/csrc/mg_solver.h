@@ -120,7 +120,6 @@ class MGSolver {
   // reach)
   bool spec_want_ = false;
   SpecHost spec_;
-  double* d_bspec_ = nullptr;  // spectral work space of a batch
   int build_spec();
   void solve_spec(int n, const SpecDev& D, const DevLevel<double>& F, cudaStream_t s);
   // a solve's V-cycles: what maxcy leaves after the direct corrections
@@ -135,9 +134,10 @@ class MGSolver {
   void relax_col(int l, int iters, cudaStream_t s, int nb = 0);
   void cycle_col(cudaStream_t s, int nb = 0);
   ColLevel C32b(int l, int nb) const;
-  // batch state (solve_batch): member table, active flags and convergence
-  // states of bcap_ members, FP32 levels, direct-solve work and norms of bcyc_
-  int bcap_ = 0, bcyc_ = 0;
+  // batch state (solve_batch): capacity, FP32 levels and direct-solve work
+  // of bcap_ members, member table, active flags, norms, convergence states
+  int bcap_ = 0;
+  char* d_batch_ = nullptr;    // the allocation that holds the device ones
   float* d_bphi32_[ANEL_MAX_LEVELS + 1] = {nullptr};
   float* d_bsrc32_[ANEL_MAX_LEVELS + 1] = {nullptr};
   double* d_bdir_ = nullptr;
@@ -152,9 +152,6 @@ class MGSolver {
   int bgraph_n_ = 0;
   int64_t bgraph_head_launches_ = 0, bgraph_body_launches_ = 0;
   void batch_free();
-  void batch_free_cycles();
-  int batch_reserve_cycles(int n);
-  int batch_cycles_ready(int n, cudaStream_t s);
   int batch_cycles(int n, anel_mg_report* const* reps, cudaStream_t s);
   int build_batch_graph(int n, cudaStream_t s);
   int solve_fp64(double* d_phi, const double* d_rhs, cudaStream_t s, anel_mg_report* rep);

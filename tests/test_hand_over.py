@@ -108,11 +108,11 @@ def test_batch_hands_over_together():
     s.close()
 
 
-def test_batch_hands_over_one_by_one_without_memory():
-    """Where the batched cycles' levels cannot be had (three members of
-    256x128x128 need 140 MB) the members go on one by one."""
+def test_batch_hands_over_without_further_memory():
+    """What the V-cycles need has been there since the batch was reserved:
+    256x128x128, with less than a member's levels left free."""
     s, rhs, phi, reps = hand_over_case((256, 128, 128), 4)
-    s.solve_batch([torch.zeros_like(f) for f in rhs], [rhs[1]] * 5)  # the direct solve's own buffers
+    assert_batch_equals(s, [rhs[1]] * 5, [phi[1]] * 5, [reps[1]] * 5)
     got = [torch.zeros_like(f) for f in rhs]
     with memory_left(24 << 20):
         out = s.solve_batch(got, rhs)
@@ -120,3 +120,22 @@ def test_batch_hands_over_one_by_one_without_memory():
     for q, w in zip(got, phi):
         assert torch.equal(q.nan_to_num(), w.nan_to_num())
     s.close()
+
+
+def test_batch_within_what_a_serving_bucket_is_charged():
+    """Device memory of a context and a batch of eight that hands over,
+    against the serving engine's estimate for a bucket's batch solver: 24
+    bytes a cell, 16 for each member's and its own FP32 levels, and 64 MB."""
+    g = G.shear_layer_grid(256, 256, 256, stretched=True)
+    p = zline(g, 1e-30)
+    p.maxcy = 4
+    rhs = torch.randn(g.ghosted[::-1], dtype=torch.float64, device="cuda")
+    phi = [torch.zeros_like(rhs) for _ in range(8)]
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    s = MGSolver(g, p)
+    for r in s.solve_batch(phi, [rhs] * 8):
+        assert r.status == abi.ERR_NOCONV and r.reserved == 0
+    used = before - torch.cuda.mem_get_info()[0]
+    s.close()
+    assert used <= np.prod(g.ghosted) * (24 + 16 * 9) + (64 << 20)
