@@ -6,6 +6,7 @@
 #include "ns_solver.h"
 #include "tune.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -270,7 +271,7 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
 // Autotuning of the DNS column solve: every launch variant of launch_cn
 // timed with CUDA events on this context's own u and q (all zero at this
 // point; the factors of a placeholder rkdt are dropped afterwards), the
-// fastest kept per (device, grid) for the process.  The variants compute
+// fastest kept per (device, grid, column solves in a launch) for the process.  The variants compute
 // the same bits.
 int NSSolver::tune_cn() {
   // one kernel's variants: forced by the environment variable (no timing;
@@ -278,7 +279,7 @@ int NSSolver::tune_cn() {
   // context's own u and q (all zero at this point; the factors of a
   // placeholder rkdt are dropped afterwards)
   bool timed = false;
-  auto pick = [&](const char* name, int nvar, const char* env, auto run, int* out) -> int {
+  auto pick = [&](const char* name, int nvar, int solves, const char* env, auto run, int* out) -> int {
     const char* force = std::getenv(env);
     if (force && *force) {
       const int v = std::atoi(force);
@@ -290,7 +291,7 @@ int NSSolver::tune_cn() {
       return ANEL_OK;
     }
     char key[128];
-    std::snprintf(key, sizeof(key), "%s dev%d %dx%dx%d", name, device_, nx_, ny_, nz_);
+    std::snprintf(key, sizeof(key), "%s dev%d %dx%dx%d solves=%d", name, device_, nx_, ny_, nz_, solves);
     int v = tune_lookup(key);
     if (v < 0 && !tune_enabled()) v = 0;
     if (v < 0) {
@@ -321,14 +322,15 @@ int NSSolver::tune_cn() {
     *out = v;
     return ANEL_OK;
   };
-  int st = pick("k_cn_column", kCNVariants, "ANEL_CN_VARIANT", [&](int q) {
-    CNSet set[5];
+  CNSet set[5];
+  const int ns = cn_set(0, set);
+  int st = pick("k_cn_column", kCNVariants, ns, "ANEL_CN_VARIANT", [&](int q) {
     const NSDev* d = &D_;
     const double rkdt = 1e-3;
-    launch_cn(&d, set, cn_set(0, set), &rkdt, 1, 1.0 / 3.0, q, stream_);
+    launch_cn(&d, set, ns, &rkdt, 1, 1.0 / 3.0, q, stream_);
   }, &cnvar_);
   if (st == ANEL_OK && D_.vles)
-    st = pick("k_cn_column_les", kCNLesVariants, "ANEL_CN_LES_VARIANT", [&](int q) {
+    st = pick("k_cn_column_les", kCNLesVariants, std::min(ns, cnb_n_), "ANEL_CN_LES_VARIANT", [&](int q) {
       cn_solve_les(0, 1.0 / 3.0, 1e-3, q, stream_);
     }, &cnlesvar_);
   if (st != ANEL_OK) return st;
