@@ -25,3 +25,13 @@ def test_choices_are_kept_per_number_of_solves_in_a_launch():
     keys = {k.strip() for k in keys if "24x12x64" in k and k.startswith("k_cn")}
     at = "dev0 24x12x64 solves="
     assert keys == {f"k_cn_column {at}4", f"k_cn_column {at}5", f"k_cn_column_les {at}4"}
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(les=True, scal1_on=1)])
+def test_a_tuned_context_is_a_fresh_one(kw):
+    """The fields that the variants are timed on are zero again."""
+    s = context(G.shear_layer_grid(40, 12, 64, stretched=True), **kw)
+    names = ("u", "v", "w", "p", "rho", "scal1", "q_u", "q_v", "q_w", "q_rho", "q_s", "psrc")
+    for k, v in s.get_fields(names).items():
+        assert not v.any(), k
+    s.close()
