@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "fp64_div.h"
 #include "mg_launch.h"
 #include "pdl.cuh"
 
@@ -284,16 +285,13 @@ __global__ void __launch_bounds__(256, 3) k_spec_y(SpecDev D) {
   }
 }
 
-// 1 / x for a normal x: the hardware's approximation (20 bits) and two
-// Newton steps y <- y + y (1 - x y), each doubling its correct bits, so
-// within a unit in the last place.  A division branches to its special
-// cases, which a chain of them waits for.
+// 1 / x for a normal x from the hardware's approximation (its top 20
+// mantissa bits).  A division branches to its special cases, which a chain of
+// them waits for.
 __device__ __forceinline__ double spec_rcp(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-#pragma unroll
-  for (int q = 0; q < 2; ++q) y = fma(y, fma(-x, y, 1.0), y);
-  return y;
+  return rcp_newton(x, y);
 }
 
 // The z-systems of eight modes at a time.  Thread (mode w, segment g) holds

@@ -1,6 +1,7 @@
 // ns_kernels.cu -- sm_100a kernels of the RK3 sub-step.  Compiled with
 // -fmad=false: every sum/product is rounded as the reference's Fortran
 // expressions evaluated left to right (citations per kernel).
+#include "fp64_div.h"
 #include "ns_launch.h"
 #include "pdl.cuh"
 
@@ -602,25 +603,11 @@ struct CNFac {
 // sweeps run in batches of kCNU rows whose global loads are issued before
 // any of the batch's stores, so a column costs n/kCNU memory latencies
 // instead of n.  The arithmetic and its order are those of the
-// row-by-row Thomas algorithm.
+// row-by-row Thomas algorithm.  A row's eliminated diagonal is the same for
+// every column, so its reciprocal is formed once per block, and the back
+// substitution's chain of divisions is half as long (div_by).
 constexpr int kCNU = 8;
 constexpr int kCNThreads = 256;
-
-// a / b, correctly rounded, from y = 1 / b rounded to nearest: two
-// corrections q <- q + (a - b q) y.  The first makes q faithful, and then the
-// second gives the rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990);
-// outside the exponents where no step can over- or underflow (for which y is
-// NaN where |b| is not within 2^-100..2^100), and for zero, infinite and NaN
-// quotients, the division itself.  b is a row's eliminated
-// diagonal, the same for every column, so its reciprocal is formed once per
-// block, and the back substitution's chain of divisions is half as long.
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-  const double q0 = a * y;
-  const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
-  const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
-  const unsigned e = (unsigned)(__double2hiint(q0) >> 20) & 0x7ffu;
-  return e - 200u < 1600u ? q2 : a / b;
-}
 
 // U rows per batch: with the columns per block, the launch variants the
 // autotuner chooses from (launch_cn); the arithmetic does not depend on
@@ -645,8 +632,7 @@ __device__ __forceinline__ void cn_column(const NSDev& D, double* __restrict__ f
     const bool in = r < n;
     s_ap[r] = in ? F.ap[r] : 0.0;
     s_bp[r] = in ? F.bp[r] : 1.0;
-    const unsigned eb = (unsigned)(__double2hiint(s_bp[r]) >> 20) & 0x7ffu;
-    s_y[r] = eb - 923u <= 200u ? 1.0 / s_bp[r] : __longlong_as_double(0x7ff8000000000000LL);
+    s_y[r] = div_reciprocal(s_bp[r]);
     s_c[r] = in ? F.c[r] : 0.0;
     s_t1[r] = in ? F.t1[r] : 0.0;
     s_t2[r] = in ? F.t2[r] : 0.0;
