@@ -1153,7 +1153,7 @@ __global__ void __launch_bounds__(256) k_cfl_max(NSDev D, unsigned long long* ou
 // (w of the cell below kept from the previous row), per-block sums of
 // |div|*vol and vol and maxima on the bit patterns; the member's last block
 // to arrive adds the blocks' sums in block order and writes the results to
-// out and to mapped host memory, so the pass is one launch and needs no
+// mapped host memory, so the pass is one launch and needs no
 // zeroing, fold or copy (seven launches of 4 us each before).
 // With cfl the same pass also takes calcdt's maximum of rdxc |u| + rdzc |w|
 // + rdyc |v| of the cell averages (the expression of k_cfl_max, in its
@@ -1163,8 +1163,7 @@ template <int N>
 struct DivOut {
   double* part[N];       // 4 doubles per block
   unsigned* count[N];
-  double* out[N];        // 4 doubles: sum |div| vol, sum vol, max |div|, CFL maximum
-  double* host[N];       // its mirror in mapped host memory
+  double* host[N];       // 4 doubles: sum |div| vol, sum vol, max |div|, CFL maximum
 };
 
 template <int N>
@@ -1259,11 +1258,11 @@ __global__ void __launch_bounds__(128) k_divergence(const __grid_constant__ NSMa
   reduce();
   if (threadIdx.x == 0) {
     *O.count[m_] = 0;
-    double *o = O.out[m_], *h = O.host[m_];
-    o[0] = h[0] = s1;
-    o[1] = h[1] = s2;
-    o[2] = h[2] = __longlong_as_double(m);
-    o[3] = h[3] = __longlong_as_double(mc);
+    double* h = O.host[m_];
+    h[0] = s1;
+    h[1] = s2;
+    h[2] = __longlong_as_double(m);
+    h[3] = __longlong_as_double(mc);
   }
 }
 
@@ -1836,7 +1835,6 @@ void launch_divergence(const NSDev* const* Ds, const DivSet* set, int n, bool cf
     for (int q = 0; q < m; ++q) {
       O.part[q] = set[b + q].part;
       O.count[q] = set[b + q].count;
-      O.out[q] = set[b + q].out;
       O.host[q] = set[b + q].host;
     }
     dim3 g = divergence_grid(P.d[0]);

@@ -90,12 +90,10 @@ void launch_plane_avg(const NSDev& D, const double* a, const double* wx, const d
 void launch_diag_update(int Z, double dtt, const double* m, double* dg, cudaStream_t s);
 // One member's divergence pass: partial sums (divergence_part_doubles), an
 // arrival counter (zero), and the results sum |div| vol, sum vol, max |div|
-// and, with cfl, calcdt's CFL maximum, on the device and in mapped host
-// memory
+// and, with cfl, calcdt's CFL maximum, in mapped host memory
 struct DivSet {
   double* part;
   unsigned* count;
-  double* out;
   double* host;
 };
 int64_t divergence_part_doubles(const NSDev& D);

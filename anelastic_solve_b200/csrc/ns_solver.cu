@@ -201,10 +201,10 @@ int NSSolver::init(const anel_grid_desc* g, const anel_mg_params* mgp, const ane
   ANEL_CUDA_TRY(cudaMalloc(&d_prof_, 2 * (size_t)Z * sizeof(double)));
   const size_t ncn = 3 * 5 * 9 * (size_t)Z;
   ANEL_CUDA_TRY(cudaMalloc(&d_cn_, ncn * sizeof(double)));
-  // [0] the CFL maximum of k_cfl_max, [1] arrival counter and [4..7] results
-  // of the divergence pass
-  ANEL_CUDA_TRY(cudaMalloc(&d_red_, 8 * sizeof(unsigned long long)));
-  ANEL_CUDA_TRY(cudaMemset(d_red_, 0, 8 * sizeof(unsigned long long)));
+  // device: [0] the CFL maximum of k_cfl_max, [1] arrival counter of the
+  // divergence pass; host: [0] as there, [4..7] results of the divergence pass
+  ANEL_CUDA_TRY(cudaMalloc(&d_red_, 2 * sizeof(unsigned long long)));
+  ANEL_CUDA_TRY(cudaMemset(d_red_, 0, 2 * sizeof(unsigned long long)));
   ANEL_CUDA_TRY(cudaHostAlloc(&h_red_, 8 * sizeof(double), cudaHostAllocMapped));
   // device view
   D_.nx = nx_;
@@ -1286,15 +1286,14 @@ int NSSolver::project(cudaStream_t s, int* iters, double* relmax) {
 }
 
 // divergence (Routines.F90:54-183) of the current fields; with_cfl also the
-// CFL maximum: results in d_red_[4..7] and, once the stream has been waited
-// for, in h_red_[4..7]
+// CFL maximum: results in h_red_[4..7] once the stream has been waited for
 int NSSolver::divergence_prepare() {
   if (!d_part_) ANEL_CUDA_TRY(cudaMalloc(&d_part_, divergence_part_doubles(D_) * sizeof(double)));
   return ANEL_OK;
 }
 
 DivSet NSSolver::divergence_set() const {
-  return DivSet{d_part_, reinterpret_cast<unsigned*>(d_red_ + 1), reinterpret_cast<double*>(d_red_ + 4), h_red_ + 4};
+  return DivSet{d_part_, reinterpret_cast<unsigned*>(d_red_ + 1), h_red_ + 4};
 }
 
 int NSSolver::divergence_pass(cudaStream_t s, bool with_cfl) {
