@@ -264,9 +264,11 @@ int MGSolver::init(const anel_grid_desc* g, const anel_mg_params* p, int device)
   ANEL_CUDA_TRY(cudaHostAlloc(&h_pin_, 4 * sizeof(double) + sizeof(SpecState), cudaHostAllocMapped));
   choose_direct_level();
   {
-    // The direct fine-level solve is the faster correction at every size
-    // and tolerance (512x256x512 cold: 2.7 ms against 17-25 ms of V-cycles;
-    // 64x32x64: 0.07 against 0.7 ms).  The column cycle keeps solves to
+    // The direct fine-level solve was the faster correction at each of
+    // nineteen sizes from 16x16x64 to 1922x62x64, with prime factors up to 31
+    // (cold, to 1e-11: 512x256x512 2.07 against 22.0 ms of V-cycles, 16x16x64
+    // 0.04 against 0.82, 496x232x256 3.9 against 73, 448x224x256 1.29 against
+    // 9.9, the least gain 7.3 times).  The column cycle keeps solves to
     // 1e-10 and looser all the same: there the answer is the iterate the
     // cycle stops at, and the parity of a 64x32x512 run with the FP64 oracle,
     // which stops at 1e-10 too, is within its 1e-8 bound on w with V-cycles

@@ -85,9 +85,10 @@ __device__ __forceinline__ void spec_norm_finish(SpecNorm& N, const SpecDev& D, 
 // The passes wait for DRAM with 16 to 24 warps per SM (the transforms' stages
 // fill the registers), so each block asks L2 for what the block that will
 // take its place reads: the block `resident` further on, in launch order.
-// 512x256x512: forward 539 -> 515 us, y 260 -> 219, update 411 -> 361, check
-// 326 -> 314, the whole solve 2.79 -> 2.58 ms; twice the distance gives
-// nothing.
+// 512x256x512: forward 539 -> 515 us, y 260 -> 219, z 350 -> 365, update
+// 411 -> 361, check 326 -> 314 (ncu, cold); a solve with its caller's gauge
+// (0.46 ms) 2.79 -> 2.58 ms, 2.60 without the z pass's; twice the distance
+// gives nothing.
 __device__ __forceinline__ void spec_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ bool spec_next_block(int resident, int& bx, int& by) {
   const int at = blockIdx.x + gridDim.x * blockIdx.y + resident;

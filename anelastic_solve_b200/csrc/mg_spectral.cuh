@@ -7,8 +7,9 @@
 //   s(p, q) = 4 a1 sin^2(pi p / nx) + 4 a3 sin^2(pi q / ny),
 // with the z-ghost rule folded into the end rows.  So one step of the
 // mixed-precision solve's defect correction, phi += A^-1 (f - A phi), is
-// five passes over memory: residual and x transform, y transform, z-systems,
-// inverse y transform, inverse x transform and update.  All of it is FP64.
+// six passes over memory: residual and x transform, y transform, z-systems,
+// inverse y transform, inverse x transform and update, and the residual norm
+// of the result.  All of it is FP64.
 //
 // Spectral array of one member: [k][j][c] complex, nxh = nx/2 per row, in
 // the space of nx*ny*nz doubles.  nx is even (the level rule), so a real

@@ -107,7 +107,8 @@ typedef struct {
 /* Per-solve report (the reference prints the same numbers,
  * NSsolver.F90:524 and mg_solver.F90:123). */
 typedef struct {
-  int32_t iter;        /* V-cycles (MIXED: defect-correction iterations) */
+  int32_t iter;        /* V-cycles (MIXED: defect-correction iterations, by
+                        * V-cycles or direct, maxcy at most together) */
   int32_t status;      /* ANEL_OK or ANEL_ERR_NOCONV / _TIMEOUT */
   double relmax;       /* reference stop metric of the last cycle */
   double resid;        /* ||f - A phi||_2 / ||f||_2 (fine operator) after the solve */
@@ -177,7 +178,8 @@ int anel_mg_ctx_solve(anel_mg_ctx* ctx, double* phif, const double* rhsf, int32_
  * the defect-correction loop is one CUDA graph per batch size, and each
  * member stops at its own tolerance.  Member b ends bit-identical to
  * anel_mg_ctx_solve of it alone; reports[b] is its report (ms: the whole
- * batch).  Needs a mixed-precision ZLINE context on the column layout
+ * batch).  Members that the direct solve does not converge go on with
+ * V-cycles together.  Needs a mixed-precision ZLINE context on the column layout
  * (x/y semi-coarsened levels, nz = 32*M), else ANEL_ERR_UNSUPPORTED.
  * Returns ANEL_ERR_NOCONV if any member did not converge. */
 int anel_mg_ctx_solve_batch(anel_mg_ctx* ctx, int32_t n, double* const* d_phis, const double* const* d_rhss,
