@@ -183,8 +183,8 @@ __global__ void __launch_bounds__(128) k_dir_solve(DirectFac F) {
 #pragma unroll
   for (int q = 0; q < M - 1; ++q) y[q] = y[q] + FL[q * 32 + lane] * xprev + FR[q * 32 + lane] * xs;
   y[M - 1] = xs;
-  if (m == 0) {
-    // the constant mode's profile is fixed only up to a constant (the
+  if (m == 0 && f[NF] == 0.0) {
+    // a pinned mode's profile is fixed only up to a constant (the
     // pinned row picks one): return it with zero mean, so that successive
     // coarse corrections add no drifting constant to the solution
     double sum = 0.0;
