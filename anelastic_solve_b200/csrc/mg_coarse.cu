@@ -69,6 +69,32 @@ int direct_build(DirectHost& D, int nx, int ny, int nz, double a1, double a2, do
   if (zZ == 2) dia0[nz - 1] += sup[nz - 1];
   double scale = 0.0;
   for (int r = 0; r < nz; ++r) scale = std::fmax(scale, std::fabs(dia0[r]));
+  // Mode (0, 0) is singular under Neumann walls.  Its null vector, to a mean
+  // of 1, is the constant where the rows sum to zero (r(z) constant), else
+  // r(z), which the rows' recurrence gives where the last pivot vanishes.
+  std::vector<double> nul(nz, 0.0);
+  bool pin = false;
+  {
+    const double shift = 2.0 * a1 + 2.0 * a3;
+    double worst = 0.0, piv = 1.0;
+    for (int r = 0; r < nz; ++r) {
+      const double d = dia0[r] + shift;
+      worst = std::fmax(worst, std::fabs(d + (r > 0 ? sub[r] : 0.0) + (r < nz - 1 ? sup[r] : 0.0)));
+      piv = r > 0 ? d - sub[r] * sup[r - 1] / piv : d;
+    }
+    if (worst <= 1e-12 * scale) {
+      pin = true;
+      nul.assign(nz, 1.0);
+    } else if (std::fabs(piv) <= 1e-10 * std::fabs(dia0[nz - 1] + shift)) {
+      pin = true;
+      double sum = nul[0] = 1.0;
+      for (int r = 0; r + 1 < nz; ++r) {
+        nul[r + 1] = -((dia0[r] + shift) * nul[r] + (r > 0 ? sub[r] * nul[r - 1] : 0.0)) / sup[r];
+        sum += nul[r + 1];
+      }
+      for (double& v : nul) v *= nz / sum;
+    }
+  }
   for (int q = 0; q < ny; ++q)
     for (int p = 0; p < nx; ++p) {
       const int m = p + nx * q;
@@ -76,17 +102,11 @@ int direct_build(DirectHost& D, int nx, int ny, int nz, double a1, double a2, do
       for (int r = 0; r < nz; ++r) dia[r] = dia0[r] + shift;
       sb = sub;
       double rhs_scale = 1.0;
-      if (m == 0) {
-        // singular under Neumann walls (rows sum to zero): pin the gauge by
-        // replacing the last row with phi = 0
-        double worst = 0.0;
-        for (int r = 0; r < nz; ++r)
-          worst = std::fmax(worst, std::fabs(dia[r] + (r > 0 ? sub[r] : 0.0) + (r < nz - 1 ? sup[r] : 0.0)));
-        if (worst <= 1e-12 * scale) {
-          sb[nz - 1] = 0.0;
-          dia[nz - 1] = 1.0;
-          rhs_scale = 0.0;
-        }
+      if (m == 0 && pin) {
+        // pin the gauge by replacing the last row with phi = 0
+        sb[nz - 1] = 0.0;
+        dia[nz - 1] = 1.0;
+        rhs_scale = 0.0;
       }
       const int st = col_sweep_factors_d(nz, M, sb, dia, sup, mf);
       if (st != ANEL_OK) {
@@ -98,7 +118,7 @@ int direct_build(DirectHost& D, int nx, int ny, int nz, double a1, double a2, do
       o[col_fac_floats(M)] = rhs_scale;
     }
   direct_free(D);
-  const size_t nd = Bx.size() + By.size() + fac.size() + (size_t)nz * nm;
+  const size_t nd = Bx.size() + By.size() + fac.size() + nul.size() + (size_t)nz * nm;
   ANEL_CUDA_TRY(cudaMalloc(&D.d_buf, nd * sizeof(double)));
   D.bytes = nd * sizeof(double);
   double* p = D.d_buf;
@@ -116,6 +136,7 @@ int direct_build(DirectHost& D, int nx, int ny, int nz, double a1, double a2, do
   D.f.Bx = put(Bx);
   D.f.By = put(By);
   D.f.fac = put(fac);
+  D.f.nul = put(nul);
   D.f.work = p;
   // launch attributes set here, outside any stream capture
   const int sm = (int)dir_smem_bytes(nx, ny);
@@ -184,16 +205,16 @@ __global__ void __launch_bounds__(128) k_dir_solve(DirectFac F) {
   for (int q = 0; q < M - 1; ++q) y[q] = y[q] + FL[q * 32 + lane] * xprev + FR[q * 32 + lane] * xs;
   y[M - 1] = xs;
   if (m == 0 && f[NF] == 0.0) {
-    // a pinned mode's profile is fixed only up to a constant (the
+    // a pinned mode's profile is fixed only up to its null vector (the
     // pinned row picks one): return it with zero mean, so that successive
-    // coarse corrections add no drifting constant to the solution
+    // coarse corrections add no drifting multiple to the solution
     double sum = 0.0;
 #pragma unroll
     for (int q = 0; q < M; ++q) sum += y[q];
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const double mean = sum / (double)(32 * M);
 #pragma unroll
-    for (int q = 0; q < M; ++q) y[q] -= mean;
+    for (int q = 0; q < M; ++q) y[q] -= mean * F.nul[lane * M + q];
   }
 #pragma unroll
   for (int q = 0; q < M; ++q) w[lane * M + q] = y[q];

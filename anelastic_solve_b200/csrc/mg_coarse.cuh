@@ -13,8 +13,8 @@
 // column sweep (lane s owns rows s*M .. s*M+M-1; inner rows by Thomas
 // elimination, the 32 separators by cyclic reduction over the lanes), in
 // FP64 with per-mode factors precomputed on the host.  The mode that is
-// constant in x and y is singular under Neumann z walls (constant null
-// vector): its last row is replaced by phi = 0, which pins the gauge.
+// constant in x and y is singular under Neumann z walls (null vector r(z)):
+// its last row is replaced by phi = 0, which pins the gauge.
 //
 // In the mixed-precision cycle this replaces the relaxation of the chosen
 // level and of every level below it: the FP32 residual restricted to the
@@ -39,6 +39,7 @@ struct DirectFac {
   const double* Bx;    // nx x nx, row p = basis function p over i
   const double* By;    // ny x ny
   const double* fac;   // [nm][dir_fac_per_mode(M)]
+  const double* nul;   // [nz] null vector of mode (0, 0), mean 1 (0: none)
   double* work;        // [nmem][nm][nz] modal right-hand side, then solution
   // members of a batch (the same level of independent problems): member b
   // has its own work block; act[b] == 0 skips it (null: all active)

@@ -50,3 +50,10 @@ def check(n, tbc, vbc, rate):
 def test_dirichlet_walls(n, tbc, rate):
     """No null vector: nothing is taken from the solution of mode (0, 0)."""
     check(n, tbc, (0, 0.2, 0, -0.1, 0, 0), rate)
+
+
+@pytest.mark.parametrize("rate", [0.0, 1e-3, 0.05])
+@pytest.mark.parametrize("n", [(32, 16, 64), (64, 32, 128), (16, 8, 512)])
+def test_density_under_neumann_walls(n, rate):
+    """The null vector is r(z) = exp(-rate z)."""
+    check(n, (0, 1, 0, 1, 0, 0), (0.0,) * 6, rate)
