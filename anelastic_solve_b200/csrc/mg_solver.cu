@@ -361,7 +361,7 @@ int MGSolver::tune_col() {
 
 MGSolver::~MGSolver() {
   if (device_ >= 0) cudaSetDevice(device_);
-  if (g32x_) cudaGraphExecDestroy(g32x_);
+  graphs_free();
   for (int l = 0; l <= ANEL_MAX_LEVELS; ++l) {
     cudaFree(d_phi64_[l]);
     cudaFree(d_src64_[l]);
@@ -386,7 +386,6 @@ MGSolver::~MGSolver() {
   spec_free(spec_);
   batch_free();
   if (h_err_) cudaFreeHost(h_err_);
-  if (gsolve_) cudaGraphExecDestroy(gsolve_);
   if (side_) cudaStreamDestroy(side_);
   cudaFree(d_conv_);
   cudaFree(d_max_);
@@ -724,11 +723,22 @@ int MGSolver::build_direct(int l, DirectHost& D) {
                       zcode_[l][0], zcode_[l][1]);
 }
 
+// The captured cycle and the solve graphs, made again when next needed.
+void MGSolver::graphs_free() {
+  for (cudaGraphExec_t* g : {&g32x_, &gsolve_, &bgraph_}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+  bgraph_n_ = 0;
+}
+
 int MGSolver::build_zline_factors() {
   const bool lj = prm_.smoother == ANEL_SMOOTHER_LJ;
   if (dirL_ > 0) {
     // coefficients changed (density): rebuild the direct solve; a level
-    // that does not qualify keeps the relaxation
+    // that does not qualify keeps the relaxation.  The graphs made so far
+    // hold the old one's buffer.
+    graphs_free();
     const int st = build_direct(dirL_, dir_);
     if (st == ANEL_ERR_UNSUPPORTED) {
       direct_free(dir_);

@@ -113,6 +113,7 @@ class MGSolver {
   DirectHost dirfine_;
   int build_direct(int l, DirectHost& D);
   void choose_direct_level();
+  void graphs_free();
   // FP64 direct solve of the fine level (mg_spectral.cuh): the mixed solve's
   // correction where x and y are periodic and uniform and the extents are
   // transformable; V-cycles take over if two corrections do not reach the
